@@ -219,7 +219,7 @@ int topk_merge_lists(int device, const void *d_lists, uint32_t nlists, uint64_t 
  * the query (host weights indexed by attribute id, host attr), and device outputs
  * for min(k, n) ids / scores (d_threshold may be NULL); work is enqueued on
  * `stream` (a cudaStream_t, NULL = the legacy default stream).  The scan's scratch
- * is a fixed array compiled into the library (about 8.4 MB on each GPU that loads
+ * is a fixed array compiled into the library (about 9.7 MB on each GPU that loads
  * it, held until the process exits): k is limited to 1024 (TOPK_ERR_UNSUPPORTED
  * above), and calls whose work overlaps on the GPU share that array and race, so
  * serialise them.  The first call on each device performs a one-time set-up on

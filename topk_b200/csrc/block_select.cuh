@@ -28,10 +28,6 @@ struct SmemSrc {
   const uint2 *p;
   __device__ uint2 operator()(uint32_t j) const { return p[j]; }
 };
-struct KeySrc {  // bare keys (no ids), as a source of (key, 0) entries
-  const uint32_t *p;
-  __device__ uint2 operator()(uint32_t j) const { return make_uint2(p[j], 0u); }
-};
 
 // Block-wide radix select over `count` entries of `src` with key >= min_key: finds
 // (prefix, mask) such that exactly `need` valid entries satisfy
@@ -190,93 +186,236 @@ __device__ uint32_t block_reduce(const uint2 *src, uint32_t count, uint2 *dst, u
   return kept;
 }
 
-// The k-th largest key among the entries src(0..count) with key >= min_key (keys only:
-// equal keys count once each, no ids): the key v with fewer than k entries above v and
-// at least k at or above it; 0 when fewer than k entries qualify.  Four 8-bit digit
-// passes from the top.  `count` must be the same in every thread; `hist` holds 256 bins.
-// The source may live in global memory: each thread loads kKthBatch entries before it
-// uses any, so a pass waits for one load latency per NT * kKthBatch entries.
-constexpr int kKthBatch = 8;
-template <int NT, class Src>
-__device__ uint32_t block_kth_key(const Src &src, uint32_t count, uint32_t min_key, uint32_t k, uint32_t *hist,
-                                  SelShared *sh) {
+// Drop the entries with key < min_key from buf[0..n), in place; returns how many are left
+// (the same in every thread).  sh->wcount must be 0.  1024 entries at a time: read into
+// registers, then written at the front, which never passes the entries still to be read.
+template <int NT>
+__device__ uint32_t block_compact(uint2 *buf, uint32_t n, uint32_t min_key, SelShared *sh) {
+  constexpr int kPer = 4;
   const int t = threadIdx.x;
-  const int lane = t & 31;
-  uint32_t v = 0;
-  for (uint32_t base = 0; base < count; base += NT * kKthBatch) {
-    uint32_t key[kKthBatch];
+#pragma unroll 1
+  for (uint32_t base = 0; base < n; base += NT * kPer) {
+    uint2 e[kPer];
 #pragma unroll
-    for (int u = 0; u < kKthBatch; ++u) {
+    for (int u = 0; u < kPer; ++u) {
       const uint32_t j = base + (uint32_t)u * NT + t;
-      key[u] = j < count ? src(j).x : 0u;
+      e[u] = j < n ? buf[j] : make_uint2(0u, 0u);
     }
+    __syncthreads();
 #pragma unroll
-    for (int u = 0; u < kKthBatch; ++u) v += (base + (uint32_t)u * NT + t < count && key[u] >= min_key);
+    for (int u = 0; u < kPer; ++u) {
+      const bool keep = base + (uint32_t)u * NT + t < n && e[u].x >= min_key;
+      const unsigned bal = __ballot_sync(0xFFFFFFFFu, keep);
+      uint32_t pos = 0;
+      if ((t & 31) == 0 && bal) pos = atomicAdd(&sh->wcount, (uint32_t)__popc(bal));
+      pos = __shfl_sync(0xFFFFFFFFu, pos, 0);
+      if (keep) buf[pos + __popc(bal & ((1u << (t & 31)) - 1u))] = e[u];
+    }
   }
-  v = warp_sum_u32(v);
-  if (t == 0) sh->valid = 0;
   __syncthreads();
-  if (lane == 0) atomicAdd(&sh->valid, v);
-  __syncthreads();
-  if (sh->valid < k) return 0u;  // uniform
-  uint32_t prefix = 0, need = k;
-  for (int shift = 24; shift >= 0; shift -= 8) {
-    for (int b = t; b < 256; b += NT) hist[b] = 0;
-    __syncthreads();
-    for (uint32_t base = 0; base < count; base += NT * kKthBatch) {  // uniform trip count
-      uint32_t key[kKthBatch];
+  const uint32_t left = sh->wcount;
+  __syncthreads();  // every thread has its copy before thread 0 may reset wcount
+  return left;
+}
+
+// The 32 words of a warp, descending across its lanes (bitonic).
+__device__ __forceinline__ uint32_t warp_sort_desc(uint32_t v, int lane) {
 #pragma unroll
-      for (int u = 0; u < kKthBatch; ++u) {
-        const uint32_t j = base + (uint32_t)u * NT + t;
-        key[u] = j < count ? src(j).x : 0u;
-      }
+  for (int size = 2; size <= 32; size <<= 1)
 #pragma unroll
-      for (int u = 0; u < kKthBatch; ++u) {
-        if (base + (uint32_t)u * NT >= count) break;  // uniform: no entry of this slot in range
-        uint32_t bin = 0xFFFFFFFFu;
-        if (base + (uint32_t)u * NT + t < count && key[u] >= min_key &&
-            (shift == 24 || (key[u] >> (shift + 8)) == (prefix >> (shift + 8))))
-          bin = (key[u] >> shift) & 255u;
-        if (!__any_sync(0xFFFFFFFFu, bin != 0xFFFFFFFFu)) continue;  // warp-uniform: nothing to count
-        const unsigned peers = __match_any_sync(0xFFFFFFFFu, bin);
-        if (bin != 0xFFFFFFFFu && lane == __ffs(peers) - 1) atomicAdd(&hist[bin], (uint32_t)__popc(peers));
-      }
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, v, stride);
+      v = ((lane & size) == 0) == ((lane & stride) == 0) ? max(v, o) : min(v, o);
     }
-    __syncthreads();
-    if (t < 32) {  // lane l owns bins [255-8l-7, 255-8l], visited from high to low
-      const int top = 255 - 8 * t;
-      uint32_t local[8], sum = 0;
+  return v;
+}
+
+// Bins of the linear histograms below, and what one level costs: about five block
+// barriers, whatever the number of keys -- a digit-wise select pays those per 8 bits, and
+// a barrier phase of a nearly idle SM takes 0.2-0.4 us.
+constexpr uint32_t kLinBins = 2048;
+
+// Of the bins [0, kLinBins), highest first: the bin in which the running count (from
+// `above`) reaches k.  hist[11] = the bin, hist[12] = the count above it, hist[13] = its
+// own.  With `scan` each bin is left holding the count above it instead of its own.
+template <int NT>
+__device__ __forceinline__ void bins_find(uint32_t *bins, uint32_t above, uint32_t k, uint32_t *hist, bool scan) {
+  static_assert(kLinBins == 8 * NT, "eight bins per thread");
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  uint32_t *mine = bins + (kLinBins - 8u - 8u * (uint32_t)t);  // thread 0 owns the highest eight
+  uint32_t c[8], sum = 0;
 #pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        local[b] = hist[top - b];
-        sum += local[b];
-      }
-      uint32_t incl = sum;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (t >= o) incl += y;
-      }
-      const uint32_t excl = incl - sum;
-      if (excl < need && need <= incl) {
-        uint32_t run = excl;
-#pragma unroll
-        for (int b = 0; b < 8; ++b) {
-          if (run + local[b] >= need) {
-            sh->digit = (uint32_t)(top - b);
-            sh->above = run;
-            break;
-          }
-          run += local[b];
-        }
-      }
-    }
-    __syncthreads();
-    need -= sh->above;
-    prefix |= sh->digit << shift;
-    __syncthreads();  // everyone has read the result before the next pass rewrites it
+  for (int i = 0; i < 8; ++i) {
+    c[i] = mine[i];
+    sum += c[i];
   }
-  return prefix;
+  uint32_t incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) hist[warp] = incl;
+  __syncthreads();
+  uint32_t run = above + incl - sum;
+  for (int w = 0; w < warp; ++w) run += hist[w];
+#pragma unroll
+  for (int i = 7; i >= 0; --i) {
+    if (run < k && k <= run + c[i]) {
+      hist[11] = (uint32_t)(mine - bins) + (uint32_t)i;
+      hist[12] = run;
+      hist[13] = c[i];
+    }
+    if (scan) mine[i] = run;
+    run += c[i];
+  }
+  __syncthreads();
+}
+
+// A lower bound of the k-th largest of the keys src[j * STRIDE], j < np (key 0: not an
+// entry), in global memory, with at most k + k / 4 + 32 keys at or above it (more only
+// where keys are equal); 0 when fewer than k keys were read.  count = keys at or above it;
+// covered = every key was read (past NT * 16 + stage_cap of them the rest is left out,
+// which only lowers the bound).  Linear bins between the smallest and the largest key, and
+// again inside the bin of the k-th when that is too full.  Keys sit in registers (16 per
+// thread) and, past those, in `stage`.
+struct KthBound {
+  uint32_t key, count;
+  bool covered;
+};
+constexpr int kKthRegs = 16;  // keys per thread in registers
+template <int NT, int STRIDE>
+__device__ __noinline__ KthBound block_kth_bound(const uint32_t *src, uint32_t np, uint32_t k, uint32_t *stage,
+                                                 uint32_t stage_cap, uint32_t *bins, uint32_t *hist) {
+  constexpr int kR = kKthRegs;
+  const int t = threadIdx.x, lane = t & 31;
+  KthBound b{0u, 0u, np <= (uint32_t)(NT * kR) + stage_cap};
+  const uint32_t nr = min(np, (uint32_t)(NT * kR));
+  const uint32_t ns = min(np - nr, stage_cap);
+  uint32_t key[kR];
+#pragma unroll
+  for (int u = 0; u < kR; ++u) {
+    const uint32_t j = (uint32_t)u * NT + t;
+    key[u] = j < nr ? __ldcg(src + (size_t)j * STRIDE) : 0u;
+  }
+  for (uint32_t j = t; j < ns; j += NT) stage[j] = __ldcg(src + (size_t)(nr + j) * STRIDE);  // read back by this thread
+  // hist[8..10]: the smallest key - 1, the largest key, the number of keys
+  if (t == 0) {
+    hist[8] = 0xFFFFFFFFu;
+    hist[9] = 0;
+    hist[10] = 0;
+  }
+  uint32_t lo = 0xFFFFFFFFu, hi = 0, v = 0;
+  auto see = [&](uint32_t x) {
+    hi = max(hi, x);
+    lo = min(lo, x - 1u);  // 0 wraps to the top: left out
+    v += x != 0u;
+  };
+#pragma unroll
+  for (int u = 0; u < kR; ++u) {
+    if ((uint32_t)u * NT >= nr) break;  // uniform
+    see(key[u]);
+  }
+  for (uint32_t j = t; j < ns; j += NT) see(stage[j]);
+  lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+  hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+  v = __reduce_add_sync(0xFFFFFFFFu, v);
+  __syncthreads();
+  if (lane == 0) {
+    atomicMin(&hist[8], lo);
+    atomicMax(&hist[9], hi);
+    atomicAdd(&hist[10], v);
+  }
+  __syncthreads();
+  lo = hist[8] + 1u;
+  hi = hist[9];
+  const uint32_t valid = hist[10];
+  if (valid >= k) {
+    uint32_t above = 0;
+#pragma unroll 1
+    for (;;) {
+      const uint32_t width = hi - lo;  // bins of 2^s keys each
+      const int s = max(0, 21 - __clz((int)width));
+      for (uint32_t i = t; i < kLinBins; i += NT) bins[i] = 0;
+      __syncthreads();
+      auto count = [&](uint32_t x) {
+        if (x - lo <= width) atomicAdd(&bins[(x - lo) >> s], 1u);
+      };
+#pragma unroll
+      for (int u = 0; u < kR; ++u) {
+        if ((uint32_t)u * NT >= nr) break;  // uniform
+        count(key[u]);
+      }
+      for (uint32_t j = t; j < ns; j += NT) count(stage[j]);
+      __syncthreads();
+      bins_find<NT>(bins, above, k, hist, false);
+      b.key = lo + (hist[11] << s);
+      above = hist[12];
+      b.count = above + hist[13];
+      if (s == 0 || b.count <= k + k / 4u + 32u) break;  // uniform
+      lo = b.key;
+      hi = min(hi, b.key + ((1u << s) - 1u));
+      __syncthreads();  // hist has been read
+    }
+  }
+  __syncthreads();  // hist and bins are free again
+  return b;
+}
+
+// The rank of every entry buf[0..n) among them, best first: entries fall into linear bins
+// over their keys, and an entry counts the better ones of its own bin.  emit(rank, entry)
+// runs once per entry.  order: n words.  False, with nothing emitted, when a bin holds so
+// many entries (equal keys, mostly) that a sort is cheaper.
+template <int NT, class Emit>
+__device__ __forceinline__ bool block_rank_bins(const uint2 *buf, uint32_t n, uint32_t *order, uint32_t *bins,
+                                                uint32_t *hist, Emit emit) {
+  const int t = threadIdx.x;
+  constexpr uint32_t kMostPerBin = 48;
+  if (t == 0) {
+    hist[8] = 0xFFFFFFFFu;
+    hist[9] = 0;
+    hist[10] = 0;
+  }
+  uint32_t lo = 0xFFFFFFFFu, hi = 0, most = 0;
+  for (uint32_t j = t; j < n; j += NT) {
+    lo = min(lo, buf[j].x);
+    hi = max(hi, buf[j].x);
+  }
+  lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+  hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+  for (uint32_t i = t; i < kLinBins; i += NT) bins[i] = 0;
+  __syncthreads();
+  if ((t & 31) == 0) {
+    atomicMin(&hist[8], lo);
+    atomicMax(&hist[9], hi);
+  }
+  __syncthreads();
+  lo = hist[8];
+  hi = hist[9];
+  const int s = max(0, 21 - __clz((int)(hi - lo)));
+  for (uint32_t j = t; j < n; j += NT) most = max(most, atomicAdd(&bins[(buf[j].x - lo) >> s], 1u));
+  most = __reduce_max_sync(0xFFFFFFFFu, most);
+  if ((t & 31) == 0) atomicMax(&hist[10], most);
+  __syncthreads();
+  if (hist[10] >= kMostPerBin) return false;  // uniform
+  bins_find<NT>(bins, 0u, 0xFFFFFFFFu, hist, true);  // each bin: the entries above it
+  // the bins' members, bin by bin; afterwards a bin holds the end of its members
+  for (uint32_t j = t; j < n; j += NT) order[atomicAdd(&bins[(buf[j].x - lo) >> s], 1u)] = j;
+  __syncthreads();
+  for (uint32_t j = t; j < n; j += NT) {
+    const uint2 e = buf[j];
+    const uint32_t bin = (e.x - lo) >> s;
+    const uint64_t c = composite(e.x, e.y);
+    // the members start where the bin above ends
+    const uint32_t first = bin + 1u < kLinBins ? bins[bin + 1u] : 0u, end = bins[bin];
+    uint32_t r = first;
+    for (uint32_t i = first; i < end; ++i) {
+      const uint2 o = buf[order[i]];
+      r += composite(o.x, o.y) > c;
+    }
+    emit(r, e);
+  }
+  return true;
 }
 
 // Barrier after one stage of a bitonic network whose comparator i (thread i % NT, whole

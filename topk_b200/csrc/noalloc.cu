@@ -12,7 +12,7 @@
 // Limits and sharing:
 //   * k <= kNoAllocMaxK (1024); the launch uses at most kNoAllocMaxGrid CTAs, and for
 //     k above 256 fewer CTAs per SM than topk_query may use (the slots are fixed).
-//   * The array takes kNoAllocScratchBytes (about 8.4 MB) of device memory on every
+//   * The array takes kNoAllocScratchBytes (about 9.7 MB) of device memory on every
 //     GPU that loads this library, for as long as the process lives.
 //   * Every call on a device uses the same array.  Calls whose kernels overlap on
 //     the GPU (different streams, or different host threads without ordering)
@@ -46,13 +46,16 @@ constexpr uint32_t kNoAllocMaxGrid = 8 * 148;
 constexpr uint32_t kNoAllocSlotEntries = 1u << 20;  // 8 MiB
 constexpr uint32_t kNoAllocMaxSlots = 2 * kNoAllocMaxGrid + kMaxLevels;
 constexpr uint32_t kNoAllocMaxGroups = kNoAllocMaxGrid + kMaxLevels;
-// published best keys before the merge: at most 8 * kPubMaxPerWarp per CTA
-constexpr uint32_t kNoAllocPubEntries = 8 * kPubMaxPerWarp * kNoAllocMaxGrid;
-// layout: ScanScratch | done[groups] | slot_count[slots] | pad | slots[entries] | pub[entries]
+// published best entries, and their keys per threshold epoch
+constexpr uint32_t kNoAllocPubEntries = kPubMaxEntries * kNoAllocMaxGrid;
+constexpr uint32_t kNoAllocPubKeys = kPubMaxKeys * kNoAllocMaxGrid;
+// layout: ScanScratch | done[groups] | slot_count[slots] | pad | slots[entries] |
+//         pub[entries] | epub[epochs][keys]
 constexpr size_t kMetaBytes = sizeof(ScanScratch) + (size_t)kNoAllocMaxGroups * 4;
 constexpr size_t kSlotsOff = (kMetaBytes + (size_t)kNoAllocMaxSlots * 4 + 255) / 256 * 256;
 constexpr size_t kPubOff = kSlotsOff + (size_t)kNoAllocSlotEntries * sizeof(uint2);
-constexpr size_t kNoAllocScratchBytes = kPubOff + (size_t)kNoAllocPubEntries * sizeof(uint2);
+constexpr size_t kEpubOff = kPubOff + (size_t)kNoAllocPubEntries * sizeof(uint2);
+constexpr size_t kNoAllocScratchBytes = kEpubOff + (size_t)kMaxEpochs * kNoAllocPubKeys * sizeof(uint32_t);
 
 // The scratch.  In host code this name is only a stand-in for the symbol: its
 // device address comes from cudaGetSymbolAddress below, once per device.
@@ -166,10 +169,16 @@ extern "C" int topk_query_noalloc(const float *d_table, uint64_t n, uint64_t ld,
   // and the threshold; a failure shows as a CUDA error on the stream.
   p.wait_limit = 1ull << 26;
   p.fault_mode = 0;
-  if (kk >= kPubMinK && (uint32_t)pl.grid >= kPubMinGrid) {
+  if (const uint32_t m = pub_entries((uint32_t)kk, (uint32_t)pl.grid)) {
     p.pub = reinterpret_cast<uint2 *>(blk + kPubOff);
-    p.pub_m = pub_keys_per_cta((uint32_t)kk, (uint32_t)pl.grid);
+    p.pub_m = m;
     p.pub_wait = kPubWaitPolls;
+    p.epub = reinterpret_cast<uint32_t *>(blk + kEpubOff);
+    p.epub_stride = kNoAllocPubKeys;
+    p.epoch_shift = kEpochShift;
+    p.epochs = scan_epochs(tiles, (uint32_t)pl.grid, kEpochShift);
+    p.epoch_keys = epoch_keys((uint32_t)kk, (uint32_t)pl.grid);
+    p.epoch_wait = kEpochWaitPolls;
   }
   p.scratch = reinterpret_cast<ScanScratch *>(blk);
   p.done = reinterpret_cast<uint32_t *>(blk + sizeof(ScanScratch));
@@ -188,28 +197,6 @@ extern "C" int topk_query_noalloc(const float *d_table, uint64_t n, uint64_t ld,
   // arrival counters (the scan expects them at zero when it starts).
   if ((e = cudaMemsetAsync(blk, 0, kMetaBytes, s)) != cudaSuccess)
     return fail(TOPK_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
-  // Large k over a large table: the threshold pass over every kSampleStride-th tile
-  // first, as topk_query runs it; its bound goes to a spare word of the array's header
-  // (zeroed above) and seeds the scan.
-  if (p.pub && kk >= sample_min_k(qq) && tiles >= kSampleMinTiles) {
-    uint32_t *seed_word = &p.scratch->pad[0];
-    ScanParams q = p;
-    q.num_tiles = (uint32_t)((tiles + kSampleStride - 1) / kSampleStride);
-    q.tile_step = (uint64_t)pl.tile * kSampleStride;
-    q.kth_only = 1;
-    q.out_kth_key = seed_word;
-    q.out_ids = nullptr;
-    q.out_scores = nullptr;
-    q.out_threshold = nullptr;
-    ScanPlan qp = pl;
-    qp.grid = (int)std::min<uint64_t>((uint64_t)pl.grid, q.num_tiles);
-    if ((uint32_t)qp.grid >= kPubMinGrid) {
-      q.pub_m = pub_keys_per_cta((uint32_t)kk, (uint32_t)qp.grid);
-      if ((e = launch_scan(qp, q, s)) != cudaSuccess)
-        return fail(TOPK_ERR_CUDA, "threshold pass launch: %s", cudaGetErrorString(e));
-      p.thr_seed_dev = seed_word;
-    }
-  }
   if ((e = launch_scan(pl, p, s)) != cudaSuccess)
     return fail(TOPK_ERR_CUDA, "scan launch: %s", cudaGetErrorString(e));
   return TOPK_OK;

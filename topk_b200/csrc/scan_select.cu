@@ -19,15 +19,29 @@
 //     3.6 TB/s; q = 4: 4.5 -> 5.5 TB/s, same-box A/B).
 //   * An object passes if its score is >= the running threshold; passing objects
 //     go to a shared candidate buffer (warp-aggregated append).  When the buffer
-//     nears capacity (a barrier vote, so every thread decides alike) the CTA keeps
-//     its top-k by an 8-bit radix select on the 64-bit (key, ~id) word, raises its
-//     own threshold and publishes its k-th key with atomicMax to a global word that
-//     every CTA folds into its filter.  Any CTA's k-th best lower-bounds the global
-//     k-th best, so nothing that can win is dropped.
-//   * End: a merge tree with fan-in G.  Each CTA writes its survivors to a slot; the
-//     last CTA of each group of G slots (per-group arrival counter) merges them to k
-//     entries in shared memory and moves up; the root sorts (bitonic) and writes the
-//     result.  Counters are put back to zero for the next query.
+//     nears capacity (a barrier vote, so every thread decides alike) the CTA drops
+//     what lies below the threshold by now, in place; only when that leaves too much
+//     (equal scores, or no bound yet) does it keep its top-k by an 8-bit radix select
+//     on the 64-bit (key, ~id) word.
+//   * The threshold comes from the grid as a whole: after tiles 1, 4, 16, ... every CTA
+//     publishes the largest keys it holds, and block 0, which scans nothing, takes the
+//     k-th largest of them -- k real objects score at least that -- as the threshold of
+//     all (epoch_publish, coordinate).  A CTA's own k-th best is the k-th of its share
+//     only: with k = 1024 of 739 CTAs it let ~700 times too much through, and every CTA
+//     ran selects and passed k entries up a merge tree.
+//   * End: each CTA publishes what it still holds above the threshold, about k entries in
+//     all, and the coordinator ranks them and writes the result.  Where the published
+//     entries cannot hold it (many equal scores, the best rows side by side in one CTA)
+//     a merge tree with fan-in G answers: each CTA writes its best k to a slot; the last
+//     CTA of each group of G slots (per-group arrival counter) merges them to k entries
+//     in shared memory and moves up; the root sorts (bitonic) and writes the result.
+//     Counters are put back to zero for the next query.
+//   Measured (us a query on a stream, independent rows, before -> after): 2^20 rows q = 4
+//   k = 16 35.4 -> 21.3, k = 100 about 55 -> 22; 2^24 rows q = 2 k = 16 70 -> 52, k = 1024
+//   205 -> 81 (two launches before: a threshold pass over every 64th tile first), q = 8
+//   k = 1024 201 -> 119; 2^27 rows q = 4 k = 1024 397 -> 351; q = 2 k = 16 230 -> 228.
+//   A launch's fixed cost is what is left: the first tiles' latency (~5 us), the first
+//   epoch (~8 us, hidden from q = 8 on), the end (~8 us).
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -56,12 +70,20 @@ struct SmemCtl {
   uint32_t reductions;
   uint32_t is_last;
   uint32_t red_g;      // threshold snapshot shared by the block
+  uint32_t state;      // the end of the scan as this CTA goes on: kEndDone, kEndTree
+  uint32_t gen0;       // the decision word as the scan started (it changes only after every
+                       // CTA has arrived)
+  uint32_t epoch0_seen;  // epoch 0's bound has been waited for
+  uint32_t keep_min;   // no entry of this CTA below it can belong to the result (inclusive,
+                       // unlike thr_g: entries that tie a bound may have come before it)
+  uint32_t my_tiles;   // tiles of this CTA (read where it is rare: it holds no register)
+  uint32_t epoch;      // next threshold epoch
   SelShared sel;       // state of the block-wide selects
 };
 
 // shared layout
-constexpr int kOffCtl = 0;        // SmemCtl (80 B)
-constexpr int kOffNever = 96;     // test barrier (u64)
+constexpr int kOffCtl = 0;        // SmemCtl (104 B)
+constexpr int kOffNever = 112;    // test barrier (u64)
 constexpr int kOffHist = 128;     // 256-bin radix histogram
 constexpr int kOffWsm = 1152;     // weights of the runtime-q path (kMaxQ floats)
 constexpr int kOffScnt = 1408;    // entry counts of a merge group's slots (kMaxFanin words)
@@ -180,7 +202,7 @@ __device__ __forceinline__ float4 score_cols(const ScanParams &p, const float4 *
 // thread too few bytes in flight otherwise).
 constexpr int kPrefetchQ = 4;
 
-// Tiles between two select votes of the scan (see scan_select_kernel).
+// Tiles between two votes on the buffer's fill (see scan_select_kernel).
 __host__ __device__ constexpr uint32_t scan_vote_tiles(int qq, bool part) {
   return (qq >= 1 && qq <= 2 && !part) ? 2u : 1u;
 }
@@ -191,6 +213,408 @@ __host__ __device__ constexpr uint32_t scan_vote_tiles(int qq, bool part) {
 template <int QQ>
 constexpr int scan_min_blocks() {
   return (QQ >= 1 && QQ <= 2) ? 6 : (QQ >= 3 && QQ <= 8) ? 5 : 4;
+}
+
+// ---------------------------------------------------------------- results
+// Put the scratch back to zero for the next scan (one thread, after everything else).
+__device__ __forceinline__ void reset_scratch(ScanScratch *s) {
+  s->acc_reductions = 0;
+  s->acc_tiles = 0;
+  s->pub_arrived = 0;
+  s->pub_n = 0;
+  s->hid_key = 0;
+  s->finishers = 0;
+  s->epoch0_ready = 0;
+  for (uint32_t e = 0; e < kMaxEpochs; ++e) s->epoch_arrived[e] = 0;
+  s->g_thr = 0;
+  s->g_app = 0;
+  __threadfence();
+}
+
+// The scan's statistics (thread 0 of the CTA that answers).
+__device__ __forceinline__ void write_stats(const ScanParams &p, uint32_t merged, uint32_t res_n, uint32_t kth_key) {
+  ScanScratch *s = p.scratch;
+  if (p.out_count) *p.out_count = res_n;
+  if (p.out_kth_key) *p.out_kth_key = res_n == p.k ? kth_key : 0u;
+  const uint32_t reds = ld_volatile_u32(&s->acc_reductions);
+  const uint32_t tiles = ld_volatile_u32(&s->acc_tiles);
+  s->last_cands = merged;
+  s->last_reductions = reds;
+  if (p.out_stats) {
+    p.out_stats[0] = merged;
+    p.out_stats[1] = reds;
+    p.out_stats[2] = tiles;
+  }
+}
+
+// res[0..res_n) descending -> the result, ascending (whole CTA).
+__device__ __forceinline__ void write_sorted(const ScanParams &p, const uint2 *res, uint32_t res_n, uint32_t merged) {
+  const int t = threadIdx.x;
+  if (p.out_ids) {  // (a round that only wants the k-th key has no result arrays)
+    for (uint32_t r = t; r < res_n; r += kScanThreads) {
+      const uint2 e = res[r];
+      const uint32_t pos = res_n - 1 - r;  // ascending output
+      p.out_ids[pos] = (uint64_t)e.y;
+      p.out_scores[pos] = key2f(e.x);
+    }
+  }
+  if (t == 0) {
+    if (p.out_threshold) *p.out_threshold = res_n ? key2f(res[res_n - 1].x) : 0.0f;
+    write_stats(p, merged, res_n, res_n ? res[res_n - 1].x : 0u);
+  }
+}
+
+// ---------------------------------------------------------------- publishing
+constexpr uint32_t kEndDone = 0, kEndTree = 1;
+// Entries ranked by counting alone, one per thread.
+constexpr uint32_t kRankMax = kScanThreads;
+// Up to this k a CTA bounds its own k-th best from 32 of its threads' largest keys.
+constexpr uint32_t kLocalBoundK = 32;
+
+// The r <= 4 largest of a warp's 32 keys, one per lane, to dst[0..r) (0: no key).
+__device__ __forceinline__ void warp_top_keys(uint32_t m, uint32_t r, uint32_t *dst, int lane) {
+#pragma unroll 1
+  for (uint32_t x = 0; x < r; ++x) {
+    const uint32_t w = __reduce_max_sync(0xFFFFFFFFu, m);
+    if (lane == 0) dst[x] = w;
+    if (lane == __ffs(__ballot_sync(0xFFFFFFFFu, m == w)) - 1) m = 0;
+  }
+}
+
+// The next threshold epoch, after every append of the segment: this CTA publishes the
+// largest key it holds (epoch_keys == 1), or each warp the epoch_keys / 8 largest of its
+// threads' largest keys -- keys of distinct objects -- for the coordinator; nothing here
+// waits for it.  In epoch 0 with k <= kLocalBoundK the CTA also takes the k-th largest of
+// 32 of those as a first bound of its own, so its buffer does not fill before epoch 0's.
+__device__ __forceinline__ void epoch_publish(const ScanParams &p, const uint2 *cand, SmemCtl *ctl, uint32_t *hist) {
+  const int t = threadIdx.x;
+  const int lane = t & 31, warp = t >> 5;
+  const uint32_t epoch = ctl->epoch;
+  uint32_t *mine = p.epub + (size_t)epoch * p.epub_stride + (size_t)(blockIdx.x - 1u) * p.epoch_keys;
+  bsync();
+  const uint32_t n = ctl->count;
+  uint32_t m = 0;  // this thread's largest key; a short buffer is dealt over the warps entry by entry
+  if (n <= (uint32_t)kScanThreads) {
+    const uint32_t j = (uint32_t)lane * (kScanThreads / 32) + (uint32_t)warp;
+    if (j < n) m = cand[j].x;
+  } else {
+#pragma unroll 4
+    for (uint32_t j = t; j < n; j += kScanThreads) m = max(m, cand[j].x);
+  }
+  if (p.epoch_keys == 1u) {
+    warp_top_keys(m, 4u, hist + 4 * warp, lane);
+    bsync();
+    if (warp == 0) {
+      const uint32_t v = warp_sort_desc(hist[lane], lane);
+      const uint32_t kth = __shfl_sync(0xFFFFFFFFu, v, (int)min(p.k, 32u) - 1);
+      if (lane == 0) {
+        *mine = v;
+        // rows in id order lose a tie with the k-th; rows with ids of their own may win it
+        if (epoch == 0 && p.k <= kLocalBoundK && kth) {
+          ctl->keep_min = kth;
+          ctl->thr_local = max(ctl->thr_local, kth + (p.row_ids ? 0u : 1u));
+        }
+        __threadfence();
+        atomicAdd(&p.scratch->epoch_arrived[epoch], 8u);
+        ctl->epoch = epoch + 1u;
+      }
+    }
+  } else {
+    const uint32_t r = p.epoch_keys / 8u;
+    warp_top_keys(m, r, mine + (uint32_t)warp * r, lane);
+    bsync();  // (every thread has read the epoch)
+    if (lane == 0) {
+      __threadfence();
+      atomicAdd(&p.scratch->epoch_arrived[epoch], 1u);
+      if (warp == 0) ctl->epoch = epoch + 1u;
+    }
+  }
+  bsync();  // the buffer and the control block have been read and written
+}
+
+// The end of a CTA's scan (p.pub set): it publishes its entries at or above its running
+// threshold when they are at most kPubMaxEntries, else those at or above the pub_m-th
+// largest of its threads' largest keys, and keeps the largest such limit of any CTA in
+// hid_key: no unpublished entry that could belong to the result reaches it.  Then it
+// waits for the coordinator's decision; true: the merge tree answers.
+__device__ __forceinline__ bool publish_entries(const ScanParams &p, const uint2 *cand, SmemCtl *ctl, uint32_t *hist) {
+  const int t = threadIdx.x;
+  const int lane = t & 31, warp = t >> 5;
+  ScanScratch *sc = p.scratch;
+  const uint32_t n = ctl->count;
+  uint32_t *wk = hist;                                 // 4 keys per warp
+  uint2 *list = reinterpret_cast<uint2 *>(hist + 32);  // kPubMaxEntries entries
+  if (t == 0) {
+    ctl->sel.valid = 0;
+    ctl->sel.wcount = 0;
+  }
+  bsync();
+  // (an append threshold in id order may be one above an inclusive bound)
+  const uint32_t a = max(ctl->thr_g[0], ctl->thr_g[1]);
+  const uint32_t g = max(ctl->keep_min, a - (a && !p.row_ids ? 1u : 0u));
+  uint32_t m = 0, v = 0;
+#pragma unroll 4
+  for (uint32_t j = t; j < n; j += kScanThreads) {
+    const uint32_t x = cand[j].x;
+    m = max(m, x);
+    v += x >= g;
+  }
+  v = __reduce_add_sync(0xFFFFFFFFu, v);
+  if (lane == 0) atomicAdd(&ctl->sel.valid, v);
+  if (n > kPubMaxEntries) warp_top_keys(m, 4u, wk + 4 * warp, lane);
+  bsync();
+  uint32_t limit = g, hid = 0;  // entries below the limit stay unpublished
+  if (ctl->sel.valid > kPubMaxEntries) {
+    const uint32_t x = warp_sort_desc(wk[lane], lane);
+    limit = max(g, __shfl_sync(0xFFFFFFFFu, x, (int)p.pub_m - 1));
+    hid = limit > g ? limit : 0u;  // (no entry below g belongs to the result)
+  }
+#pragma unroll 4
+  for (uint32_t j = t; j < n; j += kScanThreads) {
+    const uint2 e = cand[j];
+    if (e.x >= limit) {
+      const uint32_t at = atomicAdd(&ctl->sel.wcount, 1u);
+      if (at < kPubMaxEntries) list[at] = e;
+    }
+  }
+  bsync();
+  if (warp == 0) {
+    const uint32_t c = min(ctl->sel.wcount, kPubMaxEntries);
+    if (ctl->sel.wcount > kPubMaxEntries) hid = 0xFFFFFFFFu;  // (ties at the limit)
+    uint32_t base = 0;
+    if (lane == 0) {
+      if (c) base = atomicAdd(&sc->pub_n, c);
+      if (hid) atomicMax(&sc->hid_key, hid);
+    }
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    for (uint32_t j = lane; j < c; j += 32) p.pub[base + j] = list[j];
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) {
+      atomicAdd(&sc->pub_arrived, 1u);
+      const uint32_t gen0 = ctl->gen0;
+      uint32_t gen = gen0;
+      for (uint32_t it = 0; it < p.pub_wait && gen == gen0; ++it) {
+        __nanosleep(kPubWaitNs);
+        gen = ld_volatile_u32(&sc->gen);
+      }
+      if (gen == gen0) gen = atomicCAS(&sc->gen, gen0, gen0 | 1u);  // waited out: through the tree
+      ctl->state = (gen == gen0 || gen == (gen0 | 1u)) ? kEndTree : kEndDone;
+      __threadfence();  // a raised g_thr is read after the decision
+    }
+  }
+  bsync();
+  return ctl->state == kEndTree;
+}
+
+// The entries of comp[0..n) above `mine` (shared memory).
+__device__ __forceinline__ uint32_t rank_of(const unsigned long long *comp, uint32_t n, unsigned long long mine) {
+  uint32_t r = 0;
+#pragma unroll 8
+  for (uint32_t j = 0; j < n; ++j) r += comp[j] > mine;
+  return r;
+}
+
+// The coordinator (block 0 of a launch with p.pub): scans nothing.  Per epoch, once every
+// scanning CTA has published, it raises the global threshold to the k-th largest of the
+// epoch's keys (k real objects score at least that).  At the end it takes the k-th
+// largest published key T: when hid_key <= T the published entries at or above T hold the
+// result and it answers the query; else T becomes the global threshold and the merge
+// tree answers.  A block of its own, because the CTA that arrives last -- the slowest --
+// would be held up by this work in every epoch, and its code stays in the instruction
+// cache from epoch to epoch.  Its waits are bounded; given up, the tree answers.
+__device__ __noinline__ void coordinate(const ScanParams &p, SmemCtl *ctl, uint2 *buf, uint32_t *hist) {
+  const int t = threadIdx.x;
+  ScanScratch *sc = p.scratch;
+  const uint32_t gen0 = ctl->gen0, ncta = gridDim.x - 1u;
+  // its shared memory: keys or entries, then the linear bins
+  uint32_t *stage = reinterpret_cast<uint32_t *>(buf);
+  const uint32_t stage_cap = 2u * p.mcap - kLinBins;
+  uint32_t *bins = stage + stage_cap;
+  uint32_t epoch = 0;
+#pragma unroll 1
+  for (;;) {
+    // wait for the epoch (8 arrivals per CTA) or the end, whichever is first
+    if (t == 0) {
+      uint32_t st = 2;  // given up, or decided by a CTA that waited out
+      for (uint64_t it = 0; it < p.wait_limit; ++it) {
+        const uint32_t ended = ld_volatile_u32(&sc->pub_arrived);
+        const uint32_t ep = epoch < p.epochs ? ld_volatile_u32(&sc->epoch_arrived[epoch]) : 0u;
+        if (ended == ncta) {
+          st = 1;
+          break;
+        }
+        if (ep == 8u * ncta) {
+          st = 0;
+          break;
+        }
+        if ((it & 15u) == 15u && ld_volatile_u32(&sc->gen) != gen0) break;
+        __nanosleep(100);
+      }
+      ctl->state = st;
+    }
+    bsync();
+    const uint32_t st = ctl->state;
+    bsync();
+    if (st == 2) {
+      if (t == 0) atomicCAS(&sc->gen, gen0, gen0 | 1u);
+      break;
+    }
+    __threadfence();
+    if (st == 0) {
+      const KthBound b = block_kth_bound<kScanThreads, 1>(p.epub + (size_t)epoch * p.epub_stride,
+                                                          ncta * p.epoch_keys, p.k, stage, stage_cap, bins, hist);
+      if (t == 0) {
+        if (b.key) {
+          atomicMax(&sc->g_thr, b.key);
+          // in id order the rows that a CTA still has to scan when it sees this bound come
+          // after every published one: they lose a tie with it
+          atomicMax(&sc->g_app, b.key + (p.row_ids ? 0u : 1u));
+        }
+        if (epoch == 0) atomicExch(&sc->epoch0_ready, b.key + 1u);
+      }
+      ++epoch;
+      continue;
+    }
+    const uint32_t np = ld_volatile_u32(&sc->pub_n), hid_key = ld_volatile_u32(&sc->hid_key);
+    unsigned long long *comp = reinterpret_cast<unsigned long long *>(buf);
+    const bool few = np <= kRankMax;  // ranked at once, no bound needed first
+    KthBound b{0u, np, true};
+    // more equal scores than a CTA or this block can hold: the tree takes them as they are
+    if (hid_key == 0xFFFFFFFFu || np > kScanThreads * kKthRegs + stage_cap) {
+      b.covered = false;
+    } else if (few) {
+      unsigned long long mine = 0ull;
+      if (t < (int)np) {
+        const uint2 e = __ldcg(p.pub + t);
+        mine = composite(e.x, e.y);
+        comp[t] = mine;
+      }
+      if (t == 0) ctl->red_g = 0;
+      bsync();
+      uint32_t r = rank_of(comp, np, mine);
+      if (t < (int)np && r == p.k - 1u) ctl->red_g = (uint32_t)(mine >> 32);  // the k-th key
+      bsync();
+      b.key = ctl->red_g;
+      if (np < p.k) b.key = 0;
+    } else {
+      b = block_kth_bound<kScanThreads, 2>(reinterpret_cast<const uint32_t *>(p.pub), np, p.k, stage, stage_cap, bins,
+                                           hist);
+    }
+    // (no bound: fewer than k keys above 0 were published, and all count)
+    const uint32_t cnt = few || !b.key ? np : b.count;
+    const bool complete = b.covered && (b.key ? hid_key <= b.key : hid_key == 0u);
+    if (t == 0) {
+      if (b.key) atomicMax(&sc->g_thr, b.key);
+      __threadfence();
+      const bool want = complete && cnt <= stage_cap / 3u;  // (an entry and its place in the order: 3 words)
+      const uint32_t old = atomicCAS(&sc->gen, gen0, want ? gen0 + 2u : gen0 | 1u);
+      ctl->state = want && old == gen0 ? kEndDone : kEndTree;  // (a CTA that waited out takes the tree)
+      ctl->sel.wcount = 0;
+      ctl->red_g = 0;
+    }
+    bsync();
+    if (ctl->state == kEndTree) break;
+    // rank every entry at or above the bound; the best k are the result, ascending
+    const uint32_t res_n = min(cnt, p.k);
+    auto emit = [&](uint32_t r, uint32_t key, uint32_t id) {
+      if (r >= res_n) return;
+      const uint32_t pos = res_n - 1u - r;
+      if (p.out_ids) {
+        p.out_ids[pos] = (uint64_t)id;
+        p.out_scores[pos] = key2f(key);
+      }
+      if (pos == 0) {
+        if (p.out_threshold) *p.out_threshold = key2f(key);
+        ctl->red_g = key;
+      }
+    };
+    if (!few) {
+#pragma unroll 4
+      for (uint32_t j = t; j < np; j += kScanThreads) {
+        const uint2 e = __ldcg(p.pub + j);
+        if (e.x >= b.key) {
+          const uint32_t at = atomicAdd(&ctl->sel.wcount, 1u);  // < cnt
+          if (cnt <= kRankMax) comp[at] = composite(e.x, e.y);
+          else buf[at] = e;
+        }
+      }
+      bsync();
+    }
+    if (cnt <= kRankMax) {
+      if (t < (int)cnt) {
+        const unsigned long long mine = comp[t];
+        emit(rank_of(comp, cnt, mine), (uint32_t)(mine >> 32), 0xFFFFFFFFu - (uint32_t)mine);
+      }
+    } else if (!block_rank_bins<kScanThreads>(buf, cnt, stage + 2u * cnt, bins, hist,
+                                              [&](uint32_t r, uint2 e) { emit(r, e.x, e.y); })) {
+      uint2 *res = buf, *selb = buf + p.cap;  // many equal keys
+      if (cnt > p.k) {
+        block_reduce<kScanThreads>(buf, cnt, selb, p.k, 0u, hist, &ctl->sel);
+        res = selb;
+      }
+      block_sort_desc<kScanThreads>(res, res_n);
+      for (uint32_t r = t; r < res_n; r += kScanThreads) emit(r, res[r].x, res[r].y);
+    }
+    bsync();
+    if (t == 0) {
+      if (!res_n && p.out_threshold) *p.out_threshold = 0.0f;
+      write_stats(p, cnt, res_n, ctl->red_g);
+    }
+    if (t == 0) reset_scratch(sc);
+    return;
+  }
+  // through the tree: the later of this block and the tree's root resets the scratch
+  if (t == 0) {
+    __threadfence();
+    if (atomicAdd(&sc->finishers, 1u) == 1u) {
+      reset_scratch(sc);
+      sc->gen = gen0 + 2u;
+    }
+  }
+}
+
+// A threshold pass ends here (KTH): each warp publishes the best pub_m / 8 of its
+// threads' words, the last CTA writes the k-th largest published key (0 when fewer than
+// k were published).
+template <int NB>
+__device__ __forceinline__ void kth_pass_end(const ScanParams &p, uint64_t (&best)[NB], uint2 *cand0, SmemCtl *ctl,
+                                          uint32_t *hist) {
+  const int t = threadIdx.x;
+  const int lane = t & 31;
+  const uint32_t r = p.pub_m / 8u;
+  uint2 *mine = p.pub + (size_t)blockIdx.x * p.pub_m + (size_t)(t >> 5) * r;
+  for (uint32_t i = 0; i < r; ++i) {
+    uint64_t m = best[0];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const uint64_t y = __shfl_xor_sync(0xFFFFFFFFu, m, o);
+      m = y > m ? y : m;
+    }
+    if (m != 0ull && best[0] == m) {  // the one lane that holds it pops it
+#pragma unroll
+      for (int x = 0; x + 1 < NB; ++x) best[x] = best[x + 1];
+      best[NB - 1] = 0ull;
+    }
+    if (lane == 0) mine[i] = make_uint2((uint32_t)(m >> 32), 0u);
+  }
+  __threadfence();
+  bsync();
+  if (t == 0) ctl->is_last = atomicAdd(&p.scratch->pub_arrived, 1u) == gridDim.x - 1u ? 1u : 0u;
+  bsync();
+  if (!ctl->is_last) return;
+  __threadfence();
+  const KthBound b = block_kth_bound<kScanThreads, 2>(reinterpret_cast<const uint32_t *>(p.pub), gridDim.x * p.pub_m,
+                                                      p.k, reinterpret_cast<uint32_t *>(cand0), 2u * p.mcap - kLinBins,
+                                                      reinterpret_cast<uint32_t *>(cand0 + p.mcap) - kLinBins, hist);
+  if (t == 0) {
+    *p.out_kth_key = b.key;
+    p.scratch->g_thr = 0;
+    p.scratch->acc_reductions = 0;
+    p.scratch->acc_tiles = 0;
+    p.scratch->pub_arrived = 0;
+    __threadfence();
+  }
 }
 
 // QQ: compile-time attribute count (0 = runtime, any qq <= kMaxQ).  PART: partition
@@ -217,8 +641,8 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
   const int lane = t & 31;
   const uint32_t qq = QQ > 0 ? (uint32_t)QQ : p.qq;
   const uint32_t cap = p.cap;
-  const uint32_t my_tiles =
-      blockIdx.x < p.num_tiles ? (p.num_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+  // scanning CTAs: all blocks, or all but block 0, the coordinator (p.pub)
+  const uint32_t ncta = p.ncta, cta = blockIdx.x - (!KTH && p.pub ? 1u : 0u);
 
   if (QQ == 0 && t < (int)kMaxQ && t < (int)qq) wsm[t] = p.w[t];
   if (t == 0) {
@@ -232,6 +656,12 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
     // can read the second slot before thread 0's first copy into it
     ctl->thr_g[0] = ctl->thr_g[1] = max(ld_volatile_u32(&p.scratch->g_thr), seed);
     ctl->reductions = 0;
+    // (without the tree's flag: a CTA may start after another one has waited out)
+    ctl->gen0 = ld_volatile_u32(&p.scratch->gen) & ~1u;
+    ctl->epoch0_seen = 0;
+    ctl->keep_min = 0;
+    ctl->epoch = 0;
+    ctl->my_tiles = cta < p.num_tiles ? (p.num_tiles - cta + ncta - 1) / ncta : 0;
   }
   bsync();
 
@@ -245,6 +675,11 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
     }
   }
 
+  if (!KTH && p.pub && blockIdx.x == 0) {
+    coordinate(p, ctl, cand0, hist);
+    return;
+  }
+
   uint32_t g_pending = 0;  // thread 0's in-flight copy of the global threshold
   // next-tile prefetch: the loads of tile i + 1 are in flight while tile i is scored
   constexpr int kPQ = (QQ >= 1 && QQ <= kPrefetchQ) ? QQ : 1;
@@ -256,16 +691,16 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
   const uint32_t pmask = (1u << p.part_shift) - 1u;
   uint32_t part_cur = 0, key_cur = 0xFFFFFFFFu, part_nx = 0, key_nx = 0xFFFFFFFFu;
   auto part_of = [&](uint32_t j, uint32_t &part, uint32_t &key) {
-    const uint64_t x = ((uint64_t)blockIdx.x + (uint64_t)j * gridDim.x) >> p.part_shift;
+    const uint64_t x = ((uint64_t)cta + (uint64_t)j * ncta) >> p.part_shift;
     part = __ldg(p.part_list + x);
     if (p.part_key) key = __ldg(p.part_key + x);
   };
   if (PART) {
-    if (my_tiles > 0) part_of(0, part_cur, key_cur);
-    if (my_tiles > 1) part_of(1, part_nx, key_nx);
+    if (ctl->my_tiles > 0) part_of(0, part_cur, key_cur);
+    if (ctl->my_tiles > 1) part_of(1, part_nx, key_nx);
   }
   auto tile_row = [&](uint32_t j, uint32_t part) -> uint64_t {  // first row of tile j of this CTA
-    const uint64_t tix = blockIdx.x + (uint64_t)j * gridDim.x;
+    const uint64_t tix = cta + (uint64_t)j * ncta;
     if constexpr (PART) return ((uint64_t)part << p.part_rows_log2) + (tix & pmask) * kTile;
     return p.tile_begin + tix * p.tile_step;
   };
@@ -277,296 +712,239 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
   };
   // id order with prefetch: first row and index of the tile whose loads went out last;
   // tile j lies wholly inside [row_begin, row_end) iff j - int_lo < int_n (unsigned)
-  uint64_t next_row = p.tile_begin + (uint64_t)blockIdx.x * p.tile_step;
-  uint32_t next_tix = blockIdx.x;
+  uint64_t next_row = p.tile_begin + (uint64_t)cta * p.tile_step;
+  uint32_t next_tix = cta;
   auto load_next = [&](float4 *dst) {
     const uint64_t r = next_row + (uint64_t)t * kVec;
     const bool inner = next_tix - p.int_lo < p.int_n;
     load_cols<kPQ>(p, p.colp, r, !inner, dst);
   };
   float4 xn[kPQ];
-  if (prefetch && my_tiles) {
-    if constexpr (PART) load_rows(tile_row(0, part_cur), xn);
-    else load_next(xn);
-  }
   // tiles between two select votes: 2 for q <= 2 in id order (a thread's work per tile
   // is small there and the vote's barrier was the top stall), 1 elsewhere; the buffer
   // has room for that many tiles above its select mark (plan_scan)
   constexpr uint32_t kVoteTiles = scan_vote_tiles(QQ, PART);
   uint32_t after = 0;  // fill after this thread's warp last appended, since the last vote
+  // the tiles run in segments, each ended by a threshold epoch (the last by the end)
+  uint32_t seg = 0, seg_len = p.epochs ? 1u : ctl->my_tiles;  // the segment's first tile and length
   uint64_t kbest[KTH ? kPubMaxPerWarp : 1];  // KTH: this thread's best words, descending
 #pragma unroll
   for (int b = 0; b < (KTH ? (int)kPubMaxPerWarp : 1); ++b) kbest[b] = 0ull;
-  uint32_t i = 0;  // after the loop: the tiles this CTA scanned
   // q <= 2 in id order: two tiles per loop pass, so the prefetched registers swap roles
   // instead of being copied (q = 2 on 2^28 rows: 0.420 -> 0.406 ms)
   constexpr int kUnroll = kVoteTiles == 2 ? 2 : 1;
-#pragma unroll(kUnroll)
-  for (; i < my_tiles; ++i) {
-    // every thread reads the same thresholds in tile i (see SmemCtl::thr_g); in id
-    // order they are read after the scores, so they hold no register across the loads
-    uint32_t thr = 0;
-    if constexpr (PART && !KTH) {
-      thr = max(ctl->thr_local, ctl->thr_g[i & 1u]);
-      // nothing in this partition (nor in any later one of this CTA) can reach thr
-      if (key_cur < thr) break;
+  bool stopped = false;
+  for (;;) {
+    // the segment's first loads; its last tile prefetches nothing, so the epoch's code
+    // holds no loads in flight in registers
+    if (prefetch && seg_len) {
+      if constexpr (PART) {
+        load_rows(tile_row(seg, part_cur), xn);
+      } else {
+        next_row = p.tile_begin + ((uint64_t)cta + (uint64_t)seg * ncta) * p.tile_step;
+        next_tix = cta + seg * ncta;
+        load_next(xn);
+      }
     }
-    const uint64_t tile0 = (prefetch && !PART) ? next_row : tile_row(i, part_cur);
-    const uint64_t row0 = tile0 + (uint64_t)t * kVec;
-    const bool interior = (prefetch && !PART) ? next_tix - p.int_lo < p.int_n
-                                              : tile0 >= p.row_begin && tile0 + kTile <= p.row_end;  // uniform
-    float4 s;
-    if (prefetch) {
-      float4 x[kPQ];
-#pragma unroll
-      for (int m = 0; m < kPQ; ++m) x[m] = xn[m];
-      if (i + 1 < my_tiles) {
-        if constexpr (PART) {
-          load_rows(tile_row(i + 1, part_nx), xn);
-        } else {
-          next_row += p.grid_rows;
-          next_tix += gridDim.x;
-          load_next(xn);
+    uint32_t i = 0;  // tiles of the segment so far
+    // two tiles per vote: after every odd one, and in the second segment, which starts at
+    // tile 1, after every even one -- no more than two tiles ever meet an unvoted buffer
+    const uint32_t vote_at = seg == 1u ? 0u : 1u;
+#pragma unroll(kUnroll)
+    for (; i < seg_len; ++i) {
+      // every thread reads the same thresholds in tile i (see SmemCtl::thr_g); in id
+      // order they are read after the scores, so they hold no register across the loads
+      uint32_t thr = 0;
+      if constexpr (PART && !KTH) {
+        thr = max(ctl->thr_local, ctl->thr_g[i & 1u]);
+        // nothing in this partition (nor in any later one of this CTA) can reach thr
+        if (key_cur < thr) {
+          stopped = true;
+          break;
         }
       }
-      s = score_cols<kPQ>(p, x);
-    } else {
-      s = score4<QQ>(p, wsm, qq, row0, !interior);
-    }
-    if constexpr (PART) {
-      part_cur = part_nx;
-      key_cur = key_nx;
-      if (i + 2 < my_tiles) part_of(i + 2, part_nx, key_nx);
-    }
+      const uint64_t tile0 = (prefetch && !PART) ? next_row : tile_row(seg + i, part_cur);
+      const uint64_t row0 = tile0 + (uint64_t)t * kVec;
+      const bool interior = (prefetch && !PART) ? next_tix - p.int_lo < p.int_n
+                                                : tile0 >= p.row_begin && tile0 + kTile <= p.row_end;  // uniform
+      float4 s;
+      if (prefetch) {
+        float4 x[kPQ];
+#pragma unroll
+        for (int m = 0; m < kPQ; ++m) x[m] = xn[m];
+        if (i + 1 < seg_len) {
+          if constexpr (PART) {
+            load_rows(tile_row(seg + i + 1, part_nx), xn);
+          } else {
+            next_row += p.grid_rows;
+            next_tix += ncta;
+            load_next(xn);
+          }
+        }
+        s = score_cols<kPQ>(p, x);
+      } else {
+        s = score4<QQ>(p, wsm, qq, row0, !interior);
+      }
+      if constexpr (PART) {
+        part_cur = part_nx;
+        key_cur = key_nx;
+        if (seg + i + 2 < ctl->my_tiles) part_of(seg + i + 2, part_nx, key_nx);
+      }
 
-    if constexpr (KTH) {
-      // a threshold pass: every object of the tile against this thread's best words
-      const float sk[4] = {s.x, s.y, s.z, s.w};
+      if constexpr (KTH) {
+        // a threshold pass: every object of the tile against this thread's best words
+        const float sk[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const bool ok = interior || (row0 + v >= p.row_begin && row0 + v < p.row_end);
+          uint64_t c = ok ? composite(f2key(sk[v]), (uint32_t)(row0 + v)) : 0ull;
+#pragma unroll
+          for (int b = 0; b < (int)kPubMaxPerWarp; ++b)
+            if (c > kbest[b]) {
+              const uint64_t x = kbest[b];
+              kbest[b] = c;
+              c = x;
+            }
+        }
+        continue;
+      }
+      if constexpr (!PART) thr = max(ctl->thr_local, ctl->thr_g[i & 1u]);
+      // key(score) >= thr  <=>  thr == 0 (everything, NaN included) or score >= thr_float(thr)
+      const bool take_all = thr == 0u;
+      const float thr_f = thr_float(thr);
+      const float sv[4] = {s.x, s.y, s.z, s.w};
+      unsigned pass_mask = 0;
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
-        const bool ok = interior || (row0 + v >= p.row_begin && row0 + v < p.row_end);
-        uint64_t c = ok ? composite(f2key(sk[v]), (uint32_t)(row0 + v)) : 0ull;
+        bool pv = take_all || sv[v] >= thr_f;
+        if (!interior) pv = pv && row0 + v >= p.row_begin && row0 + v < p.row_end;
+        pass_mask |= (unsigned)pv << v;
+      }
+      // `after` = fill after this warp's append.  The warp that appends last before a
+      // vote sees the final count, so OR-voting "after > cap - kVoteTiles * TILE" at the
+      // barrier gives every thread the same reduce decision.  (Reading ctl->count after
+      // a barrier would not: a fast warp may already be appending the next tile.)
+      if (__ballot_sync(0xFFFFFFFFu, pass_mask != 0u)) {  // warp-uniform: some lane passed
+        uint2 *cand = cand0;
+        const uint32_t npass = __popc(pass_mask);
+        uint32_t incl = npass;
 #pragma unroll
-        for (int b = 0; b < (int)kPubMaxPerWarp; ++b)
-          if (c > kbest[b]) {
-            const uint64_t x = kbest[b];
-            kbest[b] = c;
-            c = x;
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+          if (lane >= o) incl += y;
+        }
+        const uint32_t wtotal = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        uint32_t base = 0;
+        if (lane == 31) base = atomicAdd(&ctl->count, wtotal);
+        base = __shfl_sync(0xFFFFFFFFu, base, 31);
+        after = base + wtotal;
+        base += incl - npass;
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          if (pass_mask & (1u << v)) {
+            if (TOPK_CHECK(base < cap, kDiagAppend, i, base, cap))
+              cand[base] = make_uint2(f2key(sv[v]), p.row_ids ? __ldg(p.row_ids + row0 + v) : (uint32_t)(row0 + v));
+            ++base;
           }
       }
-      continue;
-    }
-    if constexpr (!PART) thr = max(ctl->thr_local, ctl->thr_g[i & 1u]);
-    // key(score) >= thr  <=>  thr == 0 (everything, NaN included) or score >= thr_float(thr)
-    const bool take_all = thr == 0u;
-    const float thr_f = thr_float(thr);
-    const float sv[4] = {s.x, s.y, s.z, s.w};
-    unsigned pass_mask = 0;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      bool pv = take_all || sv[v] >= thr_f;
-      if (!interior) pv = pv && row0 + v >= p.row_begin && row0 + v < p.row_end;
-      pass_mask |= (unsigned)pv << v;
-    }
-    // `after` = fill after this warp's append.  The warp that appends last before a
-    // vote sees the final count, so OR-voting "after > cap - kVoteTiles * TILE" at the
-    // barrier gives every thread the same reduce decision.  (Reading ctl->count after
-    // a barrier would not: a fast warp may already be appending the next tile.)
-    if (__ballot_sync(0xFFFFFFFFu, pass_mask != 0u)) {  // warp-uniform: some lane passed
-      uint2 *cand = cand0;
-      const uint32_t npass = __popc(pass_mask);
-      uint32_t incl = npass;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= o) incl += y;
-      }
-      const uint32_t wtotal = __shfl_sync(0xFFFFFFFFu, incl, 31);
-      uint32_t base = 0;
-      if (lane == 31) base = atomicAdd(&ctl->count, wtotal);
-      base = __shfl_sync(0xFFFFFFFFu, base, 31);
-      after = base + wtotal;
-      base += incl - npass;
-#pragma unroll
-      for (int v = 0; v < 4; ++v)
-        if (pass_mask & (1u << v)) {
-          if (TOPK_CHECK(base < cap, kDiagAppend, i, base, cap))
-            cand[base] = make_uint2(f2key(sv[v]), p.row_ids ? __ldg(p.row_ids + row0 + v) : (uint32_t)(row0 + v));
-          ++base;
-        }
-    }
-    // thread 0 hands the CTA its copy of the global threshold (see SmemCtl::thr_g): it
-    // loads the global word every 8 tiles and applies it 7 tiles later, so the L2 round
-    // trip is never waited on.  The new value goes to the slot the next tile reads, and
-    // on the tile after into the other slot too; between updates both slots agree.
-    if (t == 0) {
-      if ((i & 7u) == 7u) ctl->thr_g[(i + 1u) & 1u] = max(ctl->thr_g[i & 1u], g_pending);
-      if ((i & 7u) == 0u) {
-        ctl->thr_g[(i + 1u) & 1u] = ctl->thr_g[i & 1u];
-        g_pending = ld_volatile_u32(&p.scratch->g_thr);
-      }
-    }
-    // (uniform: every thread takes the same votes)
-    if (kVoteTiles > 1 && (i % kVoteTiles) != kVoteTiles - 1 && i + 1 < my_tiles) continue;
-    const bool full = __syncthreads_or(after > cap - kVoteTiles * kTile);
-    after = 0;
-    if (full) {
-      if (t == 0) ctl->red_g = ld_volatile_u32(&p.scratch->g_thr);
-      bsync();
-      // the best k into the output area, then back to the front of the buffer
-      const uint32_t kept = block_reduce<kScanThreads>(cand0, ctl->count, selb, p.k, ctl->red_g, hist, &ctl->sel);
-      for (uint32_t j = t; j < kept; j += kScanThreads) cand0[j] = selb[j];
+      // thread 0 hands the CTA its copy of the global threshold (see SmemCtl::thr_g): it
+      // loads the global word every 4 tiles and applies it 3 tiles later, so the L2 round
+      // trip is never waited on.  The new value goes to the slot the next tile reads, and
+      // on the tile after into the other slot too; between updates both slots agree.
       if (t == 0) {
-        ctl->count = kept;
-        ctl->reductions++;
-        if (kept == p.k) {  // the CTA knows a k-th key
-          // Rows in id order: a later row has a larger id and loses a tie with the
-          // k-th, so it must beat it strictly.  Rows carrying their own ids (a
-          // reordered copy) may win the tie: the threshold stays inclusive.
-          ctl->thr_local = ctl->sel.kept_min + (p.row_ids ? 0u : 1u);
-          atomicMax(&p.scratch->g_thr, ctl->sel.kept_min);
+        if ((i & 3u) == 3u) ctl->thr_g[(i + 1u) & 1u] = max(ctl->thr_g[i & 1u], g_pending);
+        if ((i & 3u) == 0u) {
+          ctl->thr_g[(i + 1u) & 1u] = ctl->thr_g[i & 1u];
+          g_pending = max(ld_volatile_u32(&p.scratch->g_thr), ld_volatile_u32(&p.scratch->g_app));
         }
       }
-      bsync();
+      // (uniform: every thread takes the same votes; the scan's end needs no room)
+      if (kVoteTiles > 1 && (i & 1u) != vote_at) continue;
+      const bool full = __syncthreads_or(after > cap - kVoteTiles * kTile);
+      after = 0;
+      if (full && seg + i + 1 < ctl->my_tiles) {
+        if (t == 0) {
+          uint32_t g = ctl->keep_min;  // (k entries of this CTA or k published objects reach it)
+          // the first fill may come before any bound: epoch 0's is on its way, and dropping
+          // what lies below it costs one pass over the buffer instead of a select
+          if (p.epochs && !ctl->epoch0_seen) {
+            uint32_t w = ld_volatile_u32(&p.scratch->epoch0_ready);
+            for (uint32_t it = 0; it < p.epoch_wait && !w && !g; ++it) {
+              __nanosleep(kEpochWaitNs);
+              w = ld_volatile_u32(&p.scratch->epoch0_ready);
+            }
+            ctl->epoch0_seen = (w || !g) ? 1u : 0u;
+            if (w) g = max(g, w - 1u);
+          }
+          g = max(g, ld_volatile_u32(&p.scratch->g_thr));
+          ctl->red_g = ctl->keep_min = g;
+          ctl->thr_g[0] = ctl->thr_g[1] =
+              max(max(ctl->thr_g[0], ctl->thr_g[1]), max(g, ld_volatile_u32(&p.scratch->g_app)));
+          ctl->sel.wcount = 0;
+        }
+        bsync();
+        // what lies below the bound out of the buffer, in place; a select when much is left
+        const uint32_t left = block_compact<kScanThreads>(cand0, ctl->count, ctl->red_g, &ctl->sel);
+        if (left <= (cap - kVoteTiles * kTile) / 2u) {
+          if (t == 0) ctl->count = left;
+          bsync();
+          continue;
+        }
+        // the best k into the output area, then back to the front of the buffer
+        const uint32_t kept = block_reduce<kScanThreads>(cand0, left, selb, p.k, 0u, hist, &ctl->sel);
+        for (uint32_t j = t; j < kept; j += kScanThreads) cand0[j] = selb[j];
+        if (t == 0) {
+          ctl->count = kept;
+          ctl->reductions++;
+          if (kept == p.k) {  // the CTA knows a k-th key
+            // Rows in id order: a later row has a larger id and loses a tie with the
+            // k-th, so it must beat it strictly.  Rows carrying their own ids (a
+            // reordered copy) may win the tie: the threshold stays inclusive.
+            ctl->thr_local = ctl->sel.kept_min + (p.row_ids ? 0u : 1u);
+            atomicMax(&p.scratch->g_thr, ctl->sel.kept_min);
+          }
+        }
+        bsync();
+      }
     }
+    seg += i;
+    if (stopped || ctl->epoch >= p.epochs) break;
+    epoch_publish(p, cand0, ctl, hist);
+    seg_len = (ctl->epoch < p.epochs ? seg << p.epoch_shift : ctl->my_tiles) - seg;
   }
 
-  // ---- end of scan: reduce to <= k (a threshold pass publishes from its buffer as is) ----
+  // ---- end of scan ----
   bsync();
-  if (t == 0) ctl->red_g = ld_volatile_u32(&p.scratch->g_thr);
+  if (t == 0 && ctl->reductions) atomicAdd(&p.scratch->acc_reductions, ctl->reductions);
+  if (PART && t == 0) atomicAdd(&p.scratch->acc_tiles, seg);
+
+  if constexpr (KTH) {
+    kth_pass_end(p, kbest, cand0, ctl, hist);
+    return;
+  }
+  if (p.pub && !publish_entries(p, cand0, ctl, hist)) return;
+
+  // ---- merge tree: this CTA's best k first ----
+  if (t == 0) {
+    ctl->red_g = ld_volatile_u32(&p.scratch->g_thr);
+    ctl->reductions = 0;
+  }
   bsync();
-  if (!KTH && ctl->count > p.k && !p.kth_only) {
+  if (ctl->count > p.k) {
     const uint32_t kept = block_reduce<kScanThreads>(cand0, ctl->count, selb, p.k, ctl->red_g, hist, &ctl->sel);
     for (uint32_t j = t; j < kept; j += kScanThreads) cand0[j] = selb[j];
     if (t == 0) {
       ctl->count = kept;
-      ctl->reductions++;
+      atomicAdd(&p.scratch->acc_reductions, 1u);
       if (kept == p.k) atomicMax(&p.scratch->g_thr, ctl->sel.kept_min);
     }
     bsync();
   }
-  if (t == 0 && ctl->reductions) atomicAdd(&p.scratch->acc_reductions, ctl->reductions);
-  if (PART && t == 0) atomicAdd(&p.scratch->acc_tiles, i);
 
-  // ---- a tight bound before the merge (p.pub set: large k) ----
-  // Each CTA's own k-th key is a weak bound of the global k-th (the best of one CTA's
-  // share), so without more every CTA would pass ~k entries up the merge tree.  Each
-  // CTA publishes the keys of its best M = pub_m entries; the last to arrive takes the
-  // k-th largest of all published keys -- k real objects score at least that, so it is
-  // a lower bound of the global k-th, close to it when the best objects are spread over
-  // the CTAs -- and raises the global threshold to it; the others wait for that (a
-  // bounded wait: if it runs out they go on with the threshold they have, which is
-  // still exact, only slower) and the merge tree then carries about k entries in all.
-  if (KTH || p.pub) {
-    const uint2 *res0 = cand0;
-    // Each warp publishes the best r = pub_m / 8 entries of its share of the buffer
-    // (entries j = t, t + 256, ...): every thread keeps its own best r, then r rounds of
-    // a warp maximum, each taken from the lane that holds it.  The CTA's pub_m keys are
-    // the best of 8 disjoint shares -- keys of distinct real objects, which is all the
-    // bound needs.  Unused places publish key 0.
-    {
-      constexpr int kR = kPubMaxPerWarp;
-      const uint32_t r = p.pub_m / 8u;
-      const uint32_t n = ctl->count;
-      uint64_t best[kR];
-#pragma unroll
-      for (int i = 0; i < kR; ++i) best[i] = KTH ? kbest[i] : 0ull;
-      for (uint32_t j = t; !KTH && j < n; j += kScanThreads) {
-        const uint2 e = res0[j];
-        uint64_t c = composite(e.x, e.y);
-#pragma unroll
-        for (int i = 0; i < kR; ++i)  // insertion into the descending list
-          if (c > best[i]) {
-            const uint64_t x = best[i];
-            best[i] = c;
-            c = x;
-          }
-      }
-      uint2 *mine = p.pub + (size_t)blockIdx.x * p.pub_m + (size_t)(t >> 5) * r;
-      for (uint32_t i = 0; i < r; ++i) {
-        uint64_t m = best[0];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const uint64_t y = __shfl_xor_sync(0xFFFFFFFFu, m, o);
-          m = y > m ? y : m;
-        }
-        if (m != 0ull && best[0] == m) {  // the one lane that holds it pops it
-#pragma unroll
-          for (int x = 0; x + 1 < kR; ++x) best[x] = best[x + 1];
-          best[kR - 1] = 0ull;
-        }
-        // (key, place): distinct entries even for padding
-        if (lane == 0) mine[i] = make_uint2((uint32_t)(m >> 32), blockIdx.x * p.pub_m + (t >> 5) * r + i);
-      }
-    }
-    __threadfence();
-    bsync();
-    if (t == 0) ctl->is_last = atomicAdd(&p.scratch->pub_arrived, 1u) == gridDim.x - 1u ? 1u : 0u;
-    bsync();
-    if ((KTH || p.kth_only) && !ctl->is_last) return;  // a threshold pass: only the last CTA goes on
-    if (ctl->is_last) {
-      __threadfence();
-      // the k-th largest published key; entries of key 0 are padding (or NaN scores,
-      // the lowest anyway): left out.  The keys go to this CTA's free candidate space
-      // first (independent loads, kStageBatch in flight per thread), so the select's
-      // five passes read shared memory, not L2.
-      const uint32_t np = gridDim.x * p.pub_m;
-      // (a threshold pass has no candidates; a scan's <= k sit at the buffer's front)
-      uint32_t *stage = reinterpret_cast<uint32_t *>(KTH ? cand0 : cand0 + p.k);
-      const uint32_t stage_cap = KTH ? 2u * p.mcap : 2u * (p.mcap - p.k);
-      uint32_t kth;
-      if (np <= stage_cap) {
-        constexpr int kStageBatch = 8;
-        for (uint32_t base = 0; base < np; base += kScanThreads * kStageBatch) {
-          uint32_t v[kStageBatch];
-#pragma unroll
-          for (int u = 0; u < kStageBatch; ++u) {
-            const uint32_t j = base + (uint32_t)u * kScanThreads + t;
-            v[u] = j < np ? __ldcg(&p.pub[j].x) : 0u;
-          }
-#pragma unroll
-          for (int u = 0; u < kStageBatch; ++u) {
-            const uint32_t j = base + (uint32_t)u * kScanThreads + t;
-            if (j < np) stage[j] = v[u];
-          }
-        }
-        bsync();
-        kth = block_kth_key<kScanThreads>(KeySrc{stage}, np, 1u, p.k, hist, &ctl->sel);
-      } else {
-        kth = block_kth_key<kScanThreads>(SmemSrc{p.pub}, np, 1u, p.k, hist, &ctl->sel);
-      }
-      if (KTH || p.kth_only) {
-        // the bound is the pass's result; every other CTA has left: put the counters back
-        if (t == 0) {
-          *p.out_kth_key = kth;
-          p.scratch->g_thr = 0;
-          p.scratch->acc_reductions = 0;
-          p.scratch->acc_tiles = 0;
-          p.scratch->pub_arrived = 0;
-          p.scratch->pub_ready = 0;
-          __threadfence();
-        }
-        return;
-      }
-      if (t == 0) {
-        if (kth) atomicMax(&p.scratch->g_thr, kth);
-        __threadfence();
-        atomicExch(&p.scratch->pub_ready, 1u);
-      }
-    } else if (t == 0) {
-      for (uint32_t it = 0; it < p.pub_wait && !ld_volatile_u32(&p.scratch->pub_ready); ++it) __nanosleep(64);
-      __threadfence();  // the raised g_thr is read after the flag
-    }
-    bsync();
-  }
-
-  if constexpr (KTH) return;  // (the last CTA has returned above)
-
-  // ---- merge tree ----
   const uint32_t k = p.k;
   uint2 *res = cand0;
   uint32_t res_n = ctl->count;
-  uint32_t level = 0, slot = blockIdx.x, merged = res_n;
+  uint32_t level = 0, slot = cta, merged = res_n;
   uint32_t kpad = 1;  // k rounded up to a power of two: the kept entries and the sort's padding
   while (kpad < k) kpad <<= 1;
   uint2 *outb = mbuf + (p.mcap - kpad);
@@ -656,33 +1034,15 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
 
   // ---- root: sort and write the result (res has room for the padding) ----
   block_sort_desc<kScanThreads>(res, res_n);
-  if (p.out_ids) {  // (a round that only wants the k-th key has no result arrays)
-    for (uint32_t r = t; r < res_n; r += kScanThreads) {
-      const uint2 e = res[r];
-      const uint32_t pos = res_n - 1 - r;  // ascending output
-      p.out_ids[pos] = (uint64_t)e.y;
-      p.out_scores[pos] = key2f(e.x);
-    }
-  }
+  write_sorted(p, res, res_n, merged);
   if (t == 0) {
-    if (p.out_threshold) *p.out_threshold = res_n ? key2f(res[res_n - 1].x) : 0.0f;
-    if (p.out_count) *p.out_count = res_n;
-    if (p.out_kth_key) *p.out_kth_key = res_n == k ? res[res_n - 1].x : 0u;
-    const uint32_t reds = ld_volatile_u32(&p.scratch->acc_reductions);
-    const uint32_t tiles = ld_volatile_u32(&p.scratch->acc_tiles);
-    p.scratch->last_cands = merged;
-    p.scratch->last_reductions = reds;
-    if (p.out_stats) {
-      p.out_stats[0] = merged;
-      p.out_stats[1] = reds;
-      p.out_stats[2] = tiles;
-    }
-    p.scratch->acc_reductions = 0;
-    p.scratch->acc_tiles = 0;
-    p.scratch->pub_arrived = 0;  // every CTA has left its wait: it published a slot above
-    p.scratch->pub_ready = 0;
-    p.scratch->g_thr = 0;
+    // with a coordinator, the later of it and this CTA resets the scratch (no CTA waits for
+    // the decision any more: each has published a slot)
     __threadfence();
+    if (!p.pub || atomicAdd(&p.scratch->finishers, 1u) == 1u) {
+      reset_scratch(p.scratch);
+      if (p.pub) p.scratch->gen = ctl->gen0 + 2u;
+    }
   }
 }
 
@@ -770,7 +1130,7 @@ ScanPlan plan_scan(uint32_t qq, uint32_t k, uint64_t rows, int num_sms, size_t s
   const void *fn_kth = reinterpret_cast<const void *>(kernel_for(qq, part, true));
   const uint64_t tiles = (rows + 3 + kTile) / kTile;
   auto finish = [&](ScanPlan pl) {
-    uint64_t grid = (uint64_t)num_sms * (uint64_t)pl.ctas_per_sm;
+    uint64_t grid = (uint64_t)num_sms * (uint64_t)pl.ctas_per_sm - 1u;  // one place for the coordinator
     if (grid > tiles) grid = tiles;
     if (grid < 1) grid = 1;
     pl.grid = (int)grid;
@@ -877,6 +1237,7 @@ cudaError_t launch_scan(const ScanPlan &pl, const ScanParams &p, cudaStream_t st
     return cudaErrorInvalidValue;
   ScanParams q = p;
   for (uint32_t m = 0; m < 4; ++m) q.colp[m] = m < p.qq ? p.table + (uint64_t)p.attr[m] * p.ld : p.table;
+  q.ncta = (uint32_t)pl.grid;
   q.grid_rows = (uint64_t)pl.grid * p.tile_step;
   // id order: tiles [int_lo, int_lo + int_n) lie wholly inside [row_begin, row_end)
   q.int_lo = p.tile_begin < p.row_begin ? 1u : 0u;
@@ -884,7 +1245,8 @@ cudaError_t launch_scan(const ScanPlan &pl, const ScanParams &p, cudaStream_t st
   if (p.row_end >= p.tile_begin + kTile) hi = (p.row_end - p.tile_begin - kTile) / p.tile_step + 1;
   if (hi > p.num_tiles) hi = p.num_tiles;
   q.int_n = hi > q.int_lo ? (uint32_t)(hi - q.int_lo) : 0u;
-  kernel_for(p.qq, p.part_list != nullptr, p.kth_only != 0)<<<pl.grid, kScanThreads, pl.smem, stream>>>(q);
+  const int grid = pl.grid + (p.pub && !p.kth_only ? 1 : 0);  // and the coordinator
+  kernel_for(p.qq, p.part_list != nullptr, p.kth_only != 0)<<<grid, kScanThreads, pl.smem, stream>>>(q);
   return cudaGetLastError();
 }
 

@@ -89,8 +89,11 @@ struct Ctx {
   uint32_t *done = nullptr;
   uint32_t *slot_count = nullptr;
   uint2 *slots = nullptr;
-  uint2 *pub = nullptr;  // published best keys before the merge (8 * kPubMaxPerWarp per CTA of the largest grid)
-  uint32_t *d_seed_word = nullptr;  // a threshold pass's bound, read by the scan after it
+  // published best entries (kPubMaxEntries per CTA of the largest grid), one allocation:
+  // pub[max_grid * kPubMaxEntries] | epub[kMaxEpochs][max_grid * kPubMaxKeys]
+  uint2 *pub = nullptr;
+  uint32_t *epub = nullptr;
+  uint32_t epub_stride = 0;
   uint32_t max_slots = 0, max_groups = 0;
   size_t slot_entries = 0;  // capacity of `slots`
   size_t meta_bytes = 0;    // bytes that must be zero between queries (header + done)
@@ -212,7 +215,6 @@ int ctx_create(topk_table_t h, Ctx **out) {
     if (c->stream) cudaStreamDestroy(c->stream);
     cudaFree(c->scratch);
     cudaFree(c->pub);
-    cudaFree(c->d_seed_word);
     cudaFree(c->d_res);
     cudaFree(c->d_count2);
     if (c->h_res) cudaFreeHost(c->h_res);
@@ -240,9 +242,12 @@ int ctx_create(topk_table_t h, Ctx **out) {
   c->slot_count = reinterpret_cast<uint32_t *>(blk + c->meta_bytes);
   c->slots = reinterpret_cast<uint2 *>(blk + slots_off);
   if ((e = cudaMemset(blk, 0, slots_off)) != cudaSuccess) return bail(e, "scratch memset");
-  if ((e = cudaMalloc(&c->pub, (size_t)8 * kPubMaxPerWarp * max_grid * sizeof(uint2))) != cudaSuccess)
+  c->epub_stride = kPubMaxKeys * max_grid;
+  const size_t pub_entries_max = (size_t)kPubMaxEntries * max_grid;
+  if ((e = cudaMalloc(&c->pub, pub_entries_max * sizeof(uint2) +
+                                   (size_t)kMaxEpochs * c->epub_stride * sizeof(uint32_t))) != cudaSuccess)
     return bail(e, "publish area");
-  if ((e = cudaMalloc(&c->d_seed_word, 256)) != cudaSuccess) return bail(e, "seed word");
+  c->epub = reinterpret_cast<uint32_t *>(c->pub + pub_entries_max);
   if ((e = cudaMalloc(&c->d_res, result_bytes(kMaxK))) != cudaSuccess) return bail(e, "result block");
   if ((e = cudaMalloc(&c->d_count2, 2 * sizeof(unsigned long long))) != cudaSuccess) return bail(e, "count");
   if ((e = cudaHostAlloc(&c->h_res, result_bytes(kMaxK) + kStageBytes, cudaHostAllocDefault)) != cudaSuccess)
@@ -261,7 +266,6 @@ void ctx_free(Ctx *c) {
   if (c->stream) cudaStreamDestroy(c->stream);
   cudaFree(c->scratch);
   cudaFree(c->pub);
-  cudaFree(c->d_seed_word);
   cudaFree(c->d_res);
   cudaFree(c->d_count2);
   cudaFree(c->d_ids_scratch);
@@ -400,10 +404,18 @@ int enqueue_scan(topk_table_t h, Ctx *c, cudaStream_t stream, uint64_t r0, uint6
     return fail(TOPK_ERR_UNSUPPORTED, "merge tree of %d CTAs does not fit the scratch", pl.grid);
   p.wait_limit = h->wait_limit;
   p.fault_mode = (uint32_t)h->fault_mode;
-  if (k >= kPubMinK && (uint32_t)pl.grid >= kPubMinGrid) {
+  if (const uint32_t m = pub_entries((uint32_t)k, (uint32_t)pl.grid)) {
     p.pub = c->pub;
-    p.pub_m = pub_keys_per_cta((uint32_t)k, (uint32_t)pl.grid);
+    p.pub_m = m;
     p.pub_wait = kPubWaitPolls;
+    if (!ps) {
+      p.epub = c->epub;
+      p.epub_stride = c->epub_stride;
+      p.epoch_shift = kEpochShift;
+      p.epochs = scan_epochs(tiles, (uint32_t)pl.grid, kEpochShift);
+      p.epoch_keys = epoch_keys((uint32_t)k, (uint32_t)pl.grid);
+      p.epoch_wait = kEpochWaitPolls;
+    }
   }
   p.scratch = c->scratch;
   p.slots = c->slots;
@@ -437,28 +449,6 @@ int enqueue_scan(topk_table_t h, Ctx *c, cudaStream_t stream, uint64_t r0, uint6
     p.out_threshold = nullptr;
     p.out_count = nullptr;
     p.out_stats = nullptr;
-  }
-  // Large k over a large table in id order: a threshold pass over every
-  // kSampleStride-th tile first (its own launch, same kernel, no merge), whose bound
-  // seeds this scan, so its CTAs rarely need a select.
-  if (!ps && p.pub && k >= sample_min_k(qq) && tiles >= kSampleMinTiles) {
-    ScanParams q = p;
-    q.num_tiles = (uint32_t)((tiles + kSampleStride - 1) / kSampleStride);
-    q.tile_step = (uint64_t)pl.tile * kSampleStride;
-    q.kth_only = 1;
-    q.out_kth_key = c->d_seed_word;
-    q.out_ids = nullptr;
-    q.out_scores = nullptr;
-    q.out_threshold = nullptr;
-    q.out_count = nullptr;
-    q.out_stats = nullptr;
-    ScanPlan qp = pl;
-    qp.grid = (int)std::min<uint64_t>((uint64_t)pl.grid, q.num_tiles);
-    if ((uint32_t)qp.grid >= kPubMinGrid) {
-      q.pub_m = pub_keys_per_cta((uint32_t)k, (uint32_t)qp.grid);
-      CK(launch_scan(qp, q, stream));
-      p.thr_seed_dev = c->d_seed_word;
-    }
   }
   CK(launch_scan(pl, p, stream));
   return TOPK_OK;

@@ -15,10 +15,16 @@ constexpr uint32_t kLdAlign = 64;     // device column stride alignment (rows)
 constexpr int kMaxLevels = 12;        // merge-tree levels (fan-in >= 2, <= 4096 CTAs)
 constexpr int kScanSmemFixed = 1536;  // barriers, control block, radix histogram, weights
 
-// Device-side per-context scratch of the fused scan.  Zero between queries:
-// the kernel puts every counter back before it ends.
+// Threshold epochs of a scan (ScanParams::epochs): at most kMaxEpochs; in id order after
+// tiles 1, 4, 16, ... of every CTA.
+constexpr uint32_t kMaxEpochs = 6;
+constexpr uint32_t kEpochShift = 2;
+
+// Device-side per-context scratch of the fused scan.  Zero between queries (but for
+// `gen`): the kernel puts every counter back before it ends.
 struct ScanScratch {
   uint32_t g_thr;           // running global threshold key (objects below it cannot win)
+  uint32_t g_app;           // the same for rows still to be scanned (ScanParams::epub)
   uint32_t error;           // nonzero after a device wait gave up (bit 0: stage wait)
   uint32_t acc_reductions;  // CTA block-selects during this scan
   uint32_t last_cands;      // entries merged at the root of the last scan
@@ -27,10 +33,25 @@ struct ScanScratch {
   // tile, two values); the access it guarded was skipped.
   uint32_t diag[5];
   uint32_t acc_tiles;       // tiles scanned during this scan (partition mode)
-  uint32_t pub_arrived;     // CTAs that published their best keys (ScanParams::pub)
-  uint32_t pub_ready;       // 1 once the bound from the published keys is in g_thr
-  uint32_t pad[3];
+  uint32_t pad0[20];
+  // The words that CTAs count on or poll sit in lines of their own: hundreds of polls a
+  // microsecond on one line hold up every other access to it.
+  uint32_t pub_arrived;     // CTAs that published their best entries (ScanParams::pub)
+  uint32_t pub_n;           // entries published
+  uint32_t hid_key;         // no CTA holds an unpublished entry with a key at or above it
+  uint32_t epoch_arrived[kMaxEpochs];  // eight per CTA
+  uint32_t finishers;       // merge tree: its root and the coordinator, the later resets
+  uint32_t pad1[22];
+  // How the scan in flight ends: twice the number of scans finished on this scratch,
+  // plus one while the current scan ends through its merge tree.  It moves on by two
+  // when a scan is answered, so a CTA that waits for the decision sees it however
+  // late it looks.
+  uint32_t gen;
+  uint32_t pad2[31];
+  uint32_t epoch0_ready;    // 1 once epoch 0's bound is in g_thr
+  uint32_t pad3[31];
 };
+static_assert(sizeof(ScanScratch) == 512, "four 128-byte lines");
 
 // TOPK_BOUNDS_CHECK codes
 enum : uint32_t {
@@ -67,12 +88,28 @@ struct ScanParams {
   uint32_t fault_mode;  // 1: wait on a barrier nothing completes (timeout test)
   ScanScratch *scratch;
   uint2 *slots;         // merge-tree slots, k entries each (key, id)
-  // May be null.  Before the merge each CTA publishes the keys of its best pub_m
-  // entries here (grid * pub_m entries) and the k-th largest of them raises the global
-  // threshold; non-last CTAs wait at most pub_wait polls for it.
+  // May be null (then the merge tree answers).  Else block 0 of the launch coordinates and
+  // scans nothing (launch_scan adds it to the plan's grid).  At its end each scanning CTA
+  // publishes its best entries here (at most kPubMaxEntries per CTA, about pub_m when it
+  // holds more); the coordinator answers the query from the published entries when none
+  // of the unpublished ones can belong to the result, else raises the global threshold
+  // to the k-th largest published key and starts the merge tree.  The CTAs wait for that
+  // decision, at most pub_wait polls; one whose wait runs out takes the decision for
+  // the tree.
   uint2 *pub;
   uint32_t pub_m;
   uint32_t pub_wait;
+  // Threshold epochs (needs pub): after its tile 1, then 2^epoch_shift times as many,
+  // and so on (`epochs` of them) each CTA publishes the largest keys it holds (epoch_keys
+  // of them, 1 or a multiple of 8) in epub[epoch] (epub_stride keys each); the coordinator
+  // raises the global threshold to the k-th largest of them.  A CTA whose
+  // buffer fills before epoch 0's bound is there waits for it, at most epoch_wait polls.
+  uint32_t *epub;
+  uint32_t epub_stride;
+  uint32_t epochs;
+  uint32_t epoch_shift;
+  uint32_t epoch_keys;
+  uint32_t epoch_wait;
   // Threshold pass (needs pub and out_kth_key): the published keys' k-th largest goes
   // to *out_kth_key (0 when fewer than k were published) and the scan ends there, no
   // merge and no result.  Run over a sample of the tiles (tile_step) it seeds the full
@@ -109,36 +146,57 @@ struct ScanParams {
   // rows from one tile of a CTA to its next in id order (grid * tile_step), and the
   // tiles [int_lo, int_lo + int_n) that lie wholly inside [row_begin, row_end).
   const float *colp[4];
+  uint32_t ncta;        // scanning CTAs: the plan's grid
   uint64_t grid_rows;
   uint32_t int_lo;
   uint32_t int_n;
 };
 
-// The published-keys bound before the merge (ScanParams::pub): used for k >= this and
-// grids of at least kPubMinGrid CTAs; pub_keys_per_cta(k, grid) keys per CTA, so the
-// array needs grid * 8 * kPubMaxPerWarp entries.  (From k = 128: at k = 64 the bound
-// cost more than it saved, 0.447 against 0.439 ms at q = 2 on 2^28 rows.)
-constexpr uint32_t kPubMinK = 128;
-constexpr uint32_t kPubMinGrid = 16;
-constexpr uint32_t kPubWaitPolls = 4096;  // ~64 ns each
-// Keys published per CTA: a multiple of its 8 warps, at least ceil(k / grid) + 1, at
-// most 8 * kPubMaxPerWarp.
+// Publishing (ScanParams::pub): grids of at least kPubMinGrid CTAs; the arrays need
+// grid * kPubMaxEntries entries and grid * kPubMaxKeys keys per epoch.
+constexpr uint32_t kPubMinGrid = 2;
+// Polls of the two waits, about 1 us and 0.25 us apart (a decision wait hides behind the
+// answering CTA's last microseconds; waiting longer for epoch 0 costs more than a select).
+constexpr uint32_t kPubWaitPolls = 256, kPubWaitNs = 1000;
+constexpr uint32_t kEpochWaitPolls = 64, kEpochWaitNs = 250;
 constexpr uint32_t kPubMaxPerWarp = 4;
+constexpr uint32_t kPubMaxKeys = 8 * kPubMaxPerWarp;  // of an epoch
+constexpr uint32_t kPubMaxEntries = 96;               // at the end
+// Entries a CTA that holds more than kPubMaxEntries aims to publish.  With the k best
+// spread over the CTAs it holds lambda = k / grid of them; lambda + 3 sqrt(lambda) + 2
+// leaves one out in under 1-2 % of queries (then the merge tree answers).  0: no
+// publishing, too few CTAs for k entries.
+inline uint32_t pub_entries(uint32_t k, uint32_t grid) {
+  if (grid < kPubMinGrid || (uint64_t)grid * kPubMaxEntries < k) return 0;
+  const double l = (double)k / grid;
+  const uint32_t r = (uint32_t)__builtin_ceil(l + 3.0 * __builtin_sqrt(l) + 2.0);
+  return r < 24u ? r : 24u;
+}
+// Epochs of a scan over `tiles` tiles, after 1, m, m^2, ... tiles (m = 2^shift): each ends
+// before the scan does, with every CTA still taking part; none when no CTA has a third
+// tile (its buffer holds two without a select).
+inline uint32_t scan_epochs(uint64_t tiles, uint32_t grid, uint32_t shift) {
+  uint32_t e = 0;
+  if ((tiles + grid - 1) / grid >= 3)
+    for (uint64_t at = 1; at * grid < tiles && e < kMaxEpochs; at <<= shift) ++e;
+  return e;
+}
+// Keys a CTA publishes per epoch: its largest while that is at least 4k keys in all, else
+// 1, 2 or 4 per warp (at least 2k in all, when the grid has them): the k-th largest of
+// them then lies close to the k-th largest key seen so far.
+inline uint32_t epoch_keys(uint32_t k, uint32_t grid) {
+  if ((uint64_t)grid >= 4ull * k) return 1;
+  uint32_t r = 1;
+  while (r < kPubMaxPerWarp && 8ull * r * grid < 2ull * k) r *= 2;
+  return 8 * r;
+}
+// Keys a threshold pass (kth_only) publishes per CTA: a multiple of its 8 warps, at
+// least ceil(k / grid) + 1, at most 8 * kPubMaxPerWarp.
 inline uint32_t pub_keys_per_cta(uint32_t k, uint32_t grid) {
   const uint32_t want = (k + grid - 1) / grid + 1;
   const uint32_t r = (want + 7) / 8;
   return 8 * (r < kPubMaxPerWarp ? r : kPubMaxPerWarp);
 }
-// A full-table scan with k >= sample_min_k(qq) first runs a threshold pass over every
-// kSampleStride-th tile (kth_only), when the table has at least kSampleMinTiles tiles,
-// and starts from its bound: few candidates ever reach the select.  The pass pays where
-// the selects it saves are a large part of a short scan: from k = 128 at q <= 2, from
-// k = 512 up to q = 8, never above (measured per q and k on 2^28 rows; at q = 16 it
-// cost 1-3 %, at q = 2, k = 1024 it saved 60 %).
-constexpr uint32_t kSampleMinK = 128;
-inline uint32_t sample_min_k(uint32_t qq) { return qq <= 2 ? kSampleMinK : qq <= 8 ? 512u : 0xFFFFFFFFu; }
-constexpr uint32_t kSampleStride = 64;
-constexpr uint64_t kSampleMinTiles = 1u << 16;
 
 struct ScanPlan {
   uint32_t tile;     // objects per tile
