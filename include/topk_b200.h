@@ -219,7 +219,7 @@ int topk_merge_lists(int device, const void *d_lists, uint32_t nlists, uint64_t 
  * the query (host weights indexed by attribute id, host attr), and device outputs
  * for min(k, n) ids / scores (d_threshold may be NULL); work is enqueued on
  * `stream` (a cudaStream_t, NULL = the legacy default stream).  The scan's scratch
- * is a fixed array compiled into the library (about 9.7 MB on each GPU that loads
+ * is a fixed array compiled into the library (about 11.8 MB on each GPU that loads
  * it, held until the process exits): k is limited to 1024 (TOPK_ERR_UNSUPPORTED
  * above), and calls whose work overlaps on the GPU share that array and race, so
  * serialise them.  The first call on each device performs a one-time set-up on
@@ -315,9 +315,10 @@ int topk_partition_info(topk_table_t h, uint32_t *num_parts, uint32_t *part_rows
  * cut: a predicted lower bound of the k-th score (e.g. from the learned model),
  * or NaN for none.  With a cut, one scan of the partitions reaching it; the
  * answer is accepted only if at least min(k, n) objects score >= cut, else the
- * plain two-round pruned method runs.  Results identical to topk_query.
+ * scan runs again without it.  Results identical to topk_query.
  * stats (may be NULL): [0] partitions scanned, [1] partitions, [2] 1 if the cut
- * was accepted, [3] scans launched. */
+ * was accepted, [3] rounds: one for a scan from a cut, two for a scan that finds
+ * its threshold on the way. */
 int topk_query_pruned(topk_table_t h, uint64_t k, uint32_t qq, const float *weights, const uint8_t *attr, float cut,
                       uint64_t *ids, float *scores, uint64_t *count, float *threshold, uint64_t *stats);
 

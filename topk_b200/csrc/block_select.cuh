@@ -186,11 +186,11 @@ __device__ uint32_t block_reduce(const uint2 *src, uint32_t count, uint2 *dst, u
   return kept;
 }
 
-// Drop the entries with key < min_key from buf[0..n), in place; returns how many are left
+// Drop the entries below the composite `least` from buf[0..n), in place; returns how many are left
 // (the same in every thread).  sh->wcount must be 0.  1024 entries at a time: read into
 // registers, then written at the front, which never passes the entries still to be read.
 template <int NT>
-__device__ uint32_t block_compact(uint2 *buf, uint32_t n, uint32_t min_key, SelShared *sh) {
+__device__ uint32_t block_compact(uint2 *buf, uint32_t n, uint64_t least, SelShared *sh) {
   constexpr int kPer = 4;
   const int t = threadIdx.x;
 #pragma unroll 1
@@ -204,7 +204,7 @@ __device__ uint32_t block_compact(uint2 *buf, uint32_t n, uint32_t min_key, SelS
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < kPer; ++u) {
-      const bool keep = base + (uint32_t)u * NT + t < n && e[u].x >= min_key;
+      const bool keep = base + (uint32_t)u * NT + t < n && composite(e[u].x, e[u].y) >= least;
       const unsigned bal = __ballot_sync(0xFFFFFFFFu, keep);
       uint32_t pos = 0;
       if ((t & 31) == 0 && bal) pos = atomicAdd(&sh->wcount, (uint32_t)__popc(bal));
@@ -219,13 +219,14 @@ __device__ uint32_t block_compact(uint2 *buf, uint32_t n, uint32_t min_key, SelS
 }
 
 // The 32 words of a warp, descending across its lanes (bitonic).
-__device__ __forceinline__ uint32_t warp_sort_desc(uint32_t v, int lane) {
+template <class W>
+__device__ __forceinline__ W warp_sort_desc(W v, int lane) {
 #pragma unroll
   for (int size = 2; size <= 32; size <<= 1)
 #pragma unroll
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, v, stride);
-      v = ((lane & size) == 0) == ((lane & stride) == 0) ? max(v, o) : min(v, o);
+      const W o = __shfl_xor_sync(0xFFFFFFFFu, v, stride);
+      v = (((lane & size) == 0) == ((lane & stride) == 0)) == (o > v) ? o : v;
     }
   return v;
 }
@@ -272,69 +273,78 @@ __device__ __forceinline__ void bins_find(uint32_t *bins, uint32_t above, uint32
   __syncthreads();
 }
 
-// A lower bound of the k-th largest of the keys src[j * STRIDE], j < np (key 0: not an
-// entry), in global memory, with at most k + k / 4 + 32 keys at or above it (more only
-// where keys are equal); 0 when fewer than k keys were read.  count = keys at or above it;
-// covered = every key was read (past NT * 16 + stage_cap of them the rest is left out,
-// which only lowers the bound).  Linear bins between the smallest and the largest key, and
-// again inside the bin of the k-th when that is too full.  Keys sit in registers (16 per
-// thread) and, past those, in `stage`.
+// A lower bound of the k-th best of the entries src[j] = (key, id), j < np, in global
+// memory (key 0: not an entry), with at most k + k / 4 + 32 entries at or above it: a key
+// and, where too many entries share that key, a lower bound of ~id among them (else 0).
+// key 0 when fewer than k entries were read (past NT * kKthRegs + stage_cap of them the
+// rest is left out, which only lowers the bound; count = those read at or above it).  Linear bins between the smallest and the largest value, and
+// again inside the bin of the k-th when that is too full, over the keys and then over the
+// ~ids.  Values sit in registers (kKthRegs per thread) and, past those, in `stage`.
 struct KthBound {
-  uint32_t key, count;
-  bool covered;
+  uint32_t key, low, count;
+  __device__ uint64_t word() const { return ((uint64_t)key << 32) | low; }
 };
-constexpr int kKthRegs = 16;  // keys per thread in registers
-template <int NT, int STRIDE>
-__device__ __noinline__ KthBound block_kth_bound(const uint32_t *src, uint32_t np, uint32_t k, uint32_t *stage,
+constexpr int kKthRegs = 16;
+template <int NT>
+__device__ __noinline__ KthBound block_kth_bound(const uint2 *src, uint32_t np, uint32_t k, uint32_t *stage,
                                                  uint32_t stage_cap, uint32_t *bins, uint32_t *hist) {
   constexpr int kR = kKthRegs;
   const int t = threadIdx.x, lane = t & 31;
-  KthBound b{0u, 0u, np <= (uint32_t)(NT * kR) + stage_cap};
+  KthBound b{0u, 0u, 0u};
   const uint32_t nr = min(np, (uint32_t)(NT * kR));
   const uint32_t ns = min(np - nr, stage_cap);
-  uint32_t key[kR];
+  uint32_t above = 0;  // entries above the range in hand
+#pragma unroll 1
+  for (int part = 0; part < 2; ++part) {  // the keys, then (ties) the ~ids of the entries with key b.key
+    // values: 0 = not one
+    uint32_t val[kR];
+    auto value = [&](uint32_t j) {
+      if (part == 0) return __ldcg(&src[j].x);
+      const uint2 e = __ldcg(src + j);
+      return e.x == b.key ? 0xFFFFFFFFu - e.y : 0u;
+    };
 #pragma unroll
-  for (int u = 0; u < kR; ++u) {
-    const uint32_t j = (uint32_t)u * NT + t;
-    key[u] = j < nr ? __ldcg(src + (size_t)j * STRIDE) : 0u;
-  }
-  for (uint32_t j = t; j < ns; j += NT) stage[j] = __ldcg(src + (size_t)(nr + j) * STRIDE);  // read back by this thread
-  // hist[8..10]: the smallest key - 1, the largest key, the number of keys
-  if (t == 0) {
-    hist[8] = 0xFFFFFFFFu;
-    hist[9] = 0;
-    hist[10] = 0;
-  }
-  uint32_t lo = 0xFFFFFFFFu, hi = 0, v = 0;
-  auto see = [&](uint32_t x) {
-    hi = max(hi, x);
-    lo = min(lo, x - 1u);  // 0 wraps to the top: left out
-    v += x != 0u;
-  };
+    for (int u = 0; u < kR; ++u) {
+      const uint32_t j = (uint32_t)u * NT + t;
+      val[u] = j < nr ? value(j) : 0u;
+    }
+#pragma unroll 8
+    for (uint32_t j = t; j < ns; j += NT) stage[j] = value(nr + j);  // read back by this thread
+    // hist[8..10]: the smallest value - 1, the largest, their number
+    if (t == 0) {
+      hist[8] = 0xFFFFFFFFu;
+      hist[9] = 0;
+      hist[10] = 0;
+    }
+    uint32_t lo = 0xFFFFFFFFu, hi = 0, v = 0;
+    auto see = [&](uint32_t x) {
+      hi = max(hi, x);
+      lo = min(lo, x - 1u);  // 0 wraps to the top: left out
+      v += x != 0u;
+    };
 #pragma unroll
-  for (int u = 0; u < kR; ++u) {
-    if ((uint32_t)u * NT >= nr) break;  // uniform
-    see(key[u]);
-  }
-  for (uint32_t j = t; j < ns; j += NT) see(stage[j]);
-  lo = __reduce_min_sync(0xFFFFFFFFu, lo);
-  hi = __reduce_max_sync(0xFFFFFFFFu, hi);
-  v = __reduce_add_sync(0xFFFFFFFFu, v);
-  __syncthreads();
-  if (lane == 0) {
-    atomicMin(&hist[8], lo);
-    atomicMax(&hist[9], hi);
-    atomicAdd(&hist[10], v);
-  }
-  __syncthreads();
-  lo = hist[8] + 1u;
-  hi = hist[9];
-  const uint32_t valid = hist[10];
-  if (valid >= k) {
-    uint32_t above = 0;
+    for (int u = 0; u < kR; ++u) {
+      if ((uint32_t)u * NT >= nr) break;  // uniform
+      see(val[u]);
+    }
+    for (uint32_t j = t; j < ns; j += NT) see(stage[j]);
+    lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+    hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+    v = __reduce_add_sync(0xFFFFFFFFu, v);
+    __syncthreads();
+    if (lane == 0) {
+      atomicMin(&hist[8], lo);
+      atomicMax(&hist[9], hi);
+      atomicAdd(&hist[10], v);
+    }
+    __syncthreads();
+    lo = hist[8] + 1u;
+    hi = hist[9];
+    if (above + hist[10] < k) break;  // (keys only: the ids are those of enough entries)
+    uint32_t bound;
 #pragma unroll 1
     for (;;) {
-      const uint32_t width = hi - lo;  // bins of 2^s keys each
+      const uint32_t width = hi - lo;  // bins of 2^s values each
       const int s = max(0, 21 - __clz((int)width));
       for (uint32_t i = t; i < kLinBins; i += NT) bins[i] = 0;
       __syncthreads();
@@ -344,19 +354,23 @@ __device__ __noinline__ KthBound block_kth_bound(const uint32_t *src, uint32_t n
 #pragma unroll
       for (int u = 0; u < kR; ++u) {
         if ((uint32_t)u * NT >= nr) break;  // uniform
-        count(key[u]);
+        count(val[u]);
       }
       for (uint32_t j = t; j < ns; j += NT) count(stage[j]);
       __syncthreads();
       bins_find<NT>(bins, above, k, hist, false);
-      b.key = lo + (hist[11] << s);
+      bound = lo + (hist[11] << s);
       above = hist[12];
       b.count = above + hist[13];
       if (s == 0 || b.count <= k + k / 4u + 32u) break;  // uniform
-      lo = b.key;
-      hi = min(hi, b.key + ((1u << s) - 1u));
+      lo = bound;
+      hi = min(hi, bound + ((1u << s) - 1u));
       __syncthreads();  // hist has been read
     }
+    if (part == 0) b.key = bound;
+    else b.low = bound;
+    __syncthreads();  // hist has been read
+    if (b.count <= k + k / 4u + 32u) break;
   }
   __syncthreads();  // hist and bins are free again
   return b;

@@ -128,6 +128,10 @@ __device__ __forceinline__ uint32_t ld_volatile_u32(const uint32_t *p) {
   return *reinterpret_cast<const volatile uint32_t *>(p);
 }
 
+__device__ __forceinline__ unsigned long long ld_volatile_u64(const unsigned long long *p) {
+  return *reinterpret_cast<const volatile unsigned long long *>(p);
+}
+
 __device__ __forceinline__ uint32_t warp_min_u32(uint32_t v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));

@@ -12,7 +12,7 @@
 // Limits and sharing:
 //   * k <= kNoAllocMaxK (1024); the launch uses at most kNoAllocMaxGrid CTAs, and for
 //     k above 256 fewer CTAs per SM than topk_query may use (the slots are fixed).
-//   * The array takes kNoAllocScratchBytes (about 9.7 MB) of device memory on every
+//   * The array takes kNoAllocScratchBytes (about 11.8 MB) of device memory on every
 //     GPU that loads this library, for as long as the process lives.
 //   * Every call on a device uses the same array.  Calls whose kernels overlap on
 //     the GPU (different streams, or different host threads without ordering)
@@ -55,7 +55,7 @@ constexpr size_t kMetaBytes = sizeof(ScanScratch) + (size_t)kNoAllocMaxGroups * 
 constexpr size_t kSlotsOff = (kMetaBytes + (size_t)kNoAllocMaxSlots * 4 + 255) / 256 * 256;
 constexpr size_t kPubOff = kSlotsOff + (size_t)kNoAllocSlotEntries * sizeof(uint2);
 constexpr size_t kEpubOff = kPubOff + (size_t)kNoAllocPubEntries * sizeof(uint2);
-constexpr size_t kNoAllocScratchBytes = kEpubOff + (size_t)kMaxEpochs * kNoAllocPubKeys * sizeof(uint32_t);
+constexpr size_t kNoAllocScratchBytes = kEpubOff + (size_t)kMaxEpochs * kNoAllocPubKeys * sizeof(uint2);
 
 // The scratch.  In host code this name is only a stand-in for the symbol: its
 // device address comes from cudaGetSymbolAddress below, once per device.
@@ -169,15 +169,16 @@ extern "C" int topk_query_noalloc(const float *d_table, uint64_t n, uint64_t ld,
   // and the threshold; a failure shows as a CUDA error on the stream.
   p.wait_limit = 1ull << 26;
   p.fault_mode = 0;
-  if (const uint32_t m = pub_entries((uint32_t)kk, (uint32_t)pl.grid)) {
+  const uint32_t epochs = scan_epochs(tiles, (uint32_t)pl.grid, kEpochShift);
+  if (const uint32_t m = pub_entries((uint32_t)kk, (uint32_t)pl.grid, epochs)) {
     p.pub = reinterpret_cast<uint2 *>(blk + kPubOff);
     p.pub_m = m;
     p.pub_wait = kPubWaitPolls;
-    p.epub = reinterpret_cast<uint32_t *>(blk + kEpubOff);
+    p.epub = reinterpret_cast<uint2 *>(blk + kEpubOff);
     p.epub_stride = kNoAllocPubKeys;
     p.epoch_shift = kEpochShift;
-    p.epochs = scan_epochs(tiles, (uint32_t)pl.grid, kEpochShift);
-    p.epoch_keys = epoch_keys((uint32_t)kk, (uint32_t)pl.grid);
+    p.epochs = epochs;
+    p.epoch_keys = epoch_keys((uint32_t)kk, (uint32_t)pl.grid, false);
     p.epoch_wait = kEpochWaitPolls;
   }
   p.scratch = reinterpret_cast<ScanScratch *>(blk);

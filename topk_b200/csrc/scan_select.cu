@@ -29,19 +29,24 @@
 //     all (epoch_publish, coordinate).  A CTA's own k-th best is the k-th of its share
 //     only: with k = 1024 of 739 CTAs it let ~700 times too much through, and every CTA
 //     ran selects and passed k entries up a merge tree.
+//   * Bounds are (key, ~id) composites, so equal scores at the k-th are cut by id as well:
+//     on tables with many equal rows (values clipped at 1) every CTA used to pass its k
+//     ties up the merge tree.  Appending compares keys only, in id order strictly: the rows
+//     a CTA still has to scan come after every published one and lose a tie.
 //   * End: each CTA publishes what it still holds above the threshold, about k entries in
 //     all, and the coordinator ranks them and writes the result.  Where the published
-//     entries cannot hold it (many equal scores, the best rows side by side in one CTA)
-//     a merge tree with fan-in G answers: each CTA writes its best k to a slot; the last
-//     CTA of each group of G slots (per-group arrival counter) merges them to k entries
-//     in shared memory and moves up; the root sorts (bitonic) and writes the result.
-//     Counters are put back to zero for the next query.
+//     entries cannot hold it (the best rows side by side in one CTA, a large k over few
+//     tiles) a merge tree with fan-in G answers: each CTA writes its best k to a slot; the
+//     last CTA of each group of G slots (per-group arrival counter) merges them to k
+//     entries in shared memory and moves up; the root sorts (bitonic) and writes the
+//     result.  Counters are put back to zero for the next query.
 //   Measured (us a query on a stream, independent rows, before -> after): 2^20 rows q = 4
-//   k = 16 35.4 -> 21.3, k = 100 about 55 -> 22; 2^24 rows q = 2 k = 16 70 -> 52, k = 1024
-//   205 -> 81 (two launches before: a threshold pass over every 64th tile first), q = 8
-//   k = 1024 201 -> 119; 2^27 rows q = 4 k = 1024 397 -> 351; q = 2 k = 16 230 -> 228.
+//   k = 16 35.4 -> 23.6, k = 256 64 -> 28; 2^24 rows q = 2 k = 16 70 -> 57, k = 1024 205 ->
+//   79 (two launches before: a threshold pass over every 64th tile first), q = 8 k = 1024
+//   201 -> 116; 2^27 rows q = 4 k = 1024 397 -> 351; q = 2 k = 16 230 -> 230.  Correlated
+//   rows, many equal: 2^24 rows q = 2 k = 1024 272 -> 91.
 //   A launch's fixed cost is what is left: the first tiles' latency (~5 us), the first
-//   epoch (~8 us, hidden from q = 8 on), the end (~8 us).
+//   epoch (~8 us, hidden from q = 8 on), the end (~10 us).
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -74,15 +79,16 @@ struct SmemCtl {
   uint32_t gen0;       // the decision word as the scan started (it changes only after every
                        // CTA has arrived)
   uint32_t epoch0_seen;  // epoch 0's bound has been waited for
-  uint32_t keep_min;   // no entry of this CTA below it can belong to the result (inclusive,
-                       // unlike thr_g: entries that tie a bound may have come before it)
   uint32_t my_tiles;   // tiles of this CTA (read where it is rare: it holds no register)
   uint32_t epoch;      // next threshold epoch
+  unsigned long long keep;  // no entry of this CTA below this composite can belong to the
+                            // result (inclusive, unlike thr_g: entries that tie a bound's
+                            // key may have come before it)
   SelShared sel;       // state of the block-wide selects
 };
 
 // shared layout
-constexpr int kOffCtl = 0;        // SmemCtl (104 B)
+constexpr int kOffCtl = 0;        // SmemCtl (112 B)
 constexpr int kOffNever = 112;    // test barrier (u64)
 constexpr int kOffHist = 128;     // 256-bin radix histogram
 constexpr int kOffWsm = 1152;     // weights of the runtime-q path (kMaxQ floats)
@@ -210,9 +216,10 @@ __host__ __device__ constexpr uint32_t scan_vote_tiles(int qq, bool part) {
 // CTAs per SM the register budget is sized for: few queried columns need little data
 // in flight and gain from more CTAs (6: 42 registers); more columns need their loads
 // in flight without spills (5: 51 registers up to 8 columns, 4: 64 above).
-template <int QQ>
+// Partition mode runs at most 4 CTAs per SM, so it has their registers.
+template <int QQ, bool PART>
 constexpr int scan_min_blocks() {
-  return (QQ >= 1 && QQ <= 2) ? 6 : (QQ >= 3 && QQ <= 8) ? 5 : 4;
+  return PART ? 4 : (QQ >= 1 && QQ <= 2) ? 6 : (QQ >= 3 && QQ <= 8) ? 5 : 4;
 }
 
 // ---------------------------------------------------------------- results
@@ -222,7 +229,8 @@ __device__ __forceinline__ void reset_scratch(ScanScratch *s) {
   s->acc_tiles = 0;
   s->pub_arrived = 0;
   s->pub_n = 0;
-  s->hid_key = 0;
+  s->g_hid = 0;
+  s->g_keep = 0;
   s->finishers = 0;
   s->epoch0_ready = 0;
   for (uint32_t e = 0; e < kMaxEpochs; ++e) s->epoch_arrived[e] = 0;
@@ -232,10 +240,9 @@ __device__ __forceinline__ void reset_scratch(ScanScratch *s) {
 }
 
 // The scan's statistics (thread 0 of the CTA that answers).
-__device__ __forceinline__ void write_stats(const ScanParams &p, uint32_t merged, uint32_t res_n, uint32_t kth_key) {
+__device__ __forceinline__ void write_stats(const ScanParams &p, uint32_t merged, uint32_t res_n) {
   ScanScratch *s = p.scratch;
   if (p.out_count) *p.out_count = res_n;
-  if (p.out_kth_key) *p.out_kth_key = res_n == p.k ? kth_key : 0u;
   const uint32_t reds = ld_volatile_u32(&s->acc_reductions);
   const uint32_t tiles = ld_volatile_u32(&s->acc_tiles);
   s->last_cands = merged;
@@ -250,17 +257,15 @@ __device__ __forceinline__ void write_stats(const ScanParams &p, uint32_t merged
 // res[0..res_n) descending -> the result, ascending (whole CTA).
 __device__ __forceinline__ void write_sorted(const ScanParams &p, const uint2 *res, uint32_t res_n, uint32_t merged) {
   const int t = threadIdx.x;
-  if (p.out_ids) {  // (a round that only wants the k-th key has no result arrays)
-    for (uint32_t r = t; r < res_n; r += kScanThreads) {
-      const uint2 e = res[r];
-      const uint32_t pos = res_n - 1 - r;  // ascending output
-      p.out_ids[pos] = (uint64_t)e.y;
-      p.out_scores[pos] = key2f(e.x);
-    }
+  for (uint32_t r = t; r < res_n; r += kScanThreads) {
+    const uint2 e = res[r];
+    const uint32_t pos = res_n - 1 - r;  // ascending output
+    p.out_ids[pos] = (uint64_t)e.y;
+    p.out_scores[pos] = key2f(e.x);
   }
   if (t == 0) {
     if (p.out_threshold) *p.out_threshold = res_n ? key2f(res[res_n - 1].x) : 0.0f;
-    write_stats(p, merged, res_n, res_n ? res[res_n - 1].x : 0u);
+    write_stats(p, merged, res_n);
   }
 }
 
@@ -271,108 +276,136 @@ constexpr uint32_t kRankMax = kScanThreads;
 // Up to this k a CTA bounds its own k-th best from 32 of its threads' largest keys.
 constexpr uint32_t kLocalBoundK = 32;
 
-// The r <= 4 largest of a warp's 32 keys, one per lane, to dst[0..r) (0: no key).
-__device__ __forceinline__ void warp_top_keys(uint32_t m, uint32_t r, uint32_t *dst, int lane) {
+// The r <= 4 largest of a warp's 32 keys, one per lane, each handed to put(0..r, key, id)
+// on the lane that holds it (key 0: none left).
+template <class Put>
+__device__ __forceinline__ void warp_top(uint32_t key, uint32_t id, uint32_t r, int lane, Put put) {
 #pragma unroll 1
   for (uint32_t x = 0; x < r; ++x) {
-    const uint32_t w = __reduce_max_sync(0xFFFFFFFFu, m);
-    if (lane == 0) dst[x] = w;
-    if (lane == __ffs(__ballot_sync(0xFFFFFFFFu, m == w)) - 1) m = 0;
+    const uint32_t w = __reduce_max_sync(0xFFFFFFFFu, key);
+    if (lane == __ffs(__ballot_sync(0xFFFFFFFFu, key == w)) - 1) {
+      put(x, w, id);
+      key = 0;
+    }
   }
 }
 
 // The next threshold epoch, after every append of the segment: this CTA publishes the
-// largest key it holds (epoch_keys == 1), or each warp the epoch_keys / 8 largest of its
-// threads' largest keys -- keys of distinct objects -- for the coordinator; nothing here
-// waits for it.  In epoch 0 with k <= kLocalBoundK the CTA also takes the k-th largest of
-// 32 of those as a first bound of its own, so its buffer does not fill before epoch 0's.
+// best of its threads' best entries, epoch_keys of them, for the coordinator; nothing
+// here waits for it.  In epoch 0 with k <= kLocalBoundK the CTA also takes the k-th best
+// of 32 of those as a first bound of its own, so its buffer does not fill before epoch
+// 0's bound is there.
 __device__ __forceinline__ void epoch_publish(const ScanParams &p, const uint2 *cand, SmemCtl *ctl, uint32_t *hist) {
   const int t = threadIdx.x;
   const int lane = t & 31, warp = t >> 5;
   const uint32_t epoch = ctl->epoch;
-  uint32_t *mine = p.epub + (size_t)epoch * p.epub_stride + (size_t)(blockIdx.x - 1u) * p.epoch_keys;
+  unsigned long long *words = reinterpret_cast<unsigned long long *>(hist);  // 4 per warp
+  uint2 *mine = p.epub + (size_t)epoch * p.epub_stride + (size_t)(blockIdx.x - 1u) * p.epoch_keys;
   bsync();
   const uint32_t n = ctl->count;
-  uint32_t m = 0;  // this thread's largest key; a short buffer is dealt over the warps entry by entry
+  // this thread's best (of equal keys any); a short buffer is dealt over the warps entry by
+  // entry
+  uint2 m = make_uint2(0u, 0u);
   if (n <= (uint32_t)kScanThreads) {
     const uint32_t j = (uint32_t)lane * (kScanThreads / 32) + (uint32_t)warp;
-    if (j < n) m = cand[j].x;
+    if (j < n) m = cand[j];
   } else {
 #pragma unroll 4
-    for (uint32_t j = t; j < n; j += kScanThreads) m = max(m, cand[j].x);
-  }
-  if (p.epoch_keys == 1u) {
-    warp_top_keys(m, 4u, hist + 4 * warp, lane);
-    bsync();
-    if (warp == 0) {
-      const uint32_t v = warp_sort_desc(hist[lane], lane);
-      const uint32_t kth = __shfl_sync(0xFFFFFFFFu, v, (int)min(p.k, 32u) - 1);
-      if (lane == 0) {
-        *mine = v;
-        // rows in id order lose a tie with the k-th; rows with ids of their own may win it
-        if (epoch == 0 && p.k <= kLocalBoundK && kth) {
-          ctl->keep_min = kth;
-          ctl->thr_local = max(ctl->thr_local, kth + (p.row_ids ? 0u : 1u));
-        }
-        __threadfence();
-        atomicAdd(&p.scratch->epoch_arrived[epoch], 8u);
-        ctl->epoch = epoch + 1u;
-      }
+    for (uint32_t j = t; j < n; j += kScanThreads) {
+      const uint2 e = cand[j];
+      if (e.x > m.x) m = e;
     }
-  } else {
-    const uint32_t r = p.epoch_keys / 8u;
-    warp_top_keys(m, r, mine + (uint32_t)warp * r, lane);
-    bsync();  // (every thread has read the epoch)
+  }
+  // the best of each warp's lanes: enough for r of the block, or for a bound of its own
+  const uint32_t r = p.epoch_keys;
+  const bool local = epoch == 0 && p.k <= kLocalBoundK;
+  if (lane < 4) words[4 * warp + lane] = 0ull;
+  __syncwarp();
+  warp_top(m.x, m.y, local || r > 8u ? 4u : r > 2u ? 2u : 1u, lane,
+           [&](uint32_t x, uint32_t key, uint32_t id) { words[4 * warp + x] = key ? composite(key, id) : 0ull; });
+  bsync();
+  if (warp == 0) {
+    const uint64_t v = warp_sort_desc<uint64_t>(words[lane], lane);
+    if ((uint32_t)lane < r) mine[lane] = make_uint2((uint32_t)(v >> 32), 0xFFFFFFFFu - (uint32_t)v);
+    // rows in id order lose a tie with the k-th; rows with ids of their own may win it
+    if (local && lane == (int)p.k - 1 && v) {
+      ctl->keep = v;
+      ctl->thr_local = max(ctl->thr_local, (uint32_t)(v >> 32) + (p.row_ids ? 0u : 1u));
+    }
+    __threadfence();
+    __syncwarp();
     if (lane == 0) {
-      __threadfence();
       atomicAdd(&p.scratch->epoch_arrived[epoch], 1u);
-      if (warp == 0) ctl->epoch = epoch + 1u;
+      ctl->epoch = epoch + 1u;
     }
   }
   bsync();  // the buffer and the control block have been read and written
 }
 
+// The bounds known by now into the CTA's thresholds (thread 0; barriers around it).  With
+// `wait`, epoch 0's is waited for when it is still on its way.
+__device__ __forceinline__ void take_bound(const ScanParams &p, SmemCtl *ctl, bool wait) {
+  ScanScratch *sc = p.scratch;
+  if (p.epochs && !ctl->epoch0_seen) {
+    uint32_t ready = ld_volatile_u32(&sc->epoch0_ready);
+    for (uint32_t it = 0; it < p.epoch_wait && !ready && wait; ++it) {
+      __nanosleep(kEpochWaitNs);
+      ready = ld_volatile_u32(&sc->epoch0_ready);
+    }
+    ctl->epoch0_seen = (ready || wait) ? 1u : 0u;
+  }
+  const uint64_t g = max((uint64_t)ld_volatile_u64(&sc->g_keep), (uint64_t)ld_volatile_u32(&sc->g_thr) << 32);
+  if (g > ctl->keep) ctl->keep = g;
+  ctl->thr_g[0] = ctl->thr_g[1] =
+      max(max(ctl->thr_g[0], ctl->thr_g[1]), max((uint32_t)(ctl->keep >> 32), ld_volatile_u32(&sc->g_app)));
+}
+
 // The end of a CTA's scan (p.pub set): it publishes its entries at or above its running
-// threshold when they are at most kPubMaxEntries, else those at or above the pub_m-th
-// largest of its threads' largest keys, and keeps the largest such limit of any CTA in
-// hid_key: no unpublished entry that could belong to the result reaches it.  Then it
-// waits for the coordinator's decision; true: the merge tree answers.
+// bound when they are at most kPubMaxEntries, else those at or above the pub_m-th best of
+// its threads' best, and keeps the largest such limit of any CTA in g_hid: no unpublished
+// entry that could belong to the result reaches it.  Then it waits for the coordinator's
+// decision; true: the merge tree answers.
 __device__ __forceinline__ bool publish_entries(const ScanParams &p, const uint2 *cand, SmemCtl *ctl, uint32_t *hist) {
   const int t = threadIdx.x;
   const int lane = t & 31, warp = t >> 5;
   ScanScratch *sc = p.scratch;
   const uint32_t n = ctl->count;
-  uint32_t *wk = hist;                                 // 4 keys per warp
-  uint2 *list = reinterpret_cast<uint2 *>(hist + 32);  // kPubMaxEntries entries
+  uint32_t *keys = hist;                               // 4 per warp, before the list
+  uint2 *list = reinterpret_cast<uint2 *>(hist + 64);  // kPubMaxEntries entries
   if (t == 0) {
     ctl->sel.valid = 0;
     ctl->sel.wcount = 0;
+    // the last epoch's bound (a CTA of two or three tiles may be here before epoch 0's: with
+    // it about k entries are published in all, without it tens of thousands)
+    if (p.epochs) take_bound(p, ctl, true);
   }
   bsync();
-  // (an append threshold in id order may be one above an inclusive bound)
-  const uint32_t a = max(ctl->thr_g[0], ctl->thr_g[1]);
-  const uint32_t g = max(ctl->keep_min, a - (a && !p.row_ids ? 1u : 0u));
+  const uint64_t g = ctl->keep;
+  const uint32_t gkey = (uint32_t)(g >> 32), glow = (uint32_t)g;
   uint32_t m = 0, v = 0;
 #pragma unroll 4
   for (uint32_t j = t; j < n; j += kScanThreads) {
-    const uint32_t x = cand[j].x;
-    m = max(m, x);
-    v += x >= g;
+    const uint2 e = cand[j];
+    m = max(m, e.x);
+    v += e.x > gkey || (e.x == gkey && 0xFFFFFFFFu - e.y >= glow);
   }
   v = __reduce_add_sync(0xFFFFFFFFu, v);
   if (lane == 0) atomicAdd(&ctl->sel.valid, v);
-  if (n > kPubMaxEntries) warp_top_keys(m, 4u, wk + 4 * warp, lane);
+  if (n > kPubMaxEntries) {
+    if (lane < 4) keys[4 * warp + lane] = 0;
+    __syncwarp();
+    warp_top(m, 0u, 4u, lane, [&](uint32_t x, uint32_t key, uint32_t) { keys[4 * warp + x] = key; });
+  }
   bsync();
-  uint32_t limit = g, hid = 0;  // entries below the limit stay unpublished
+  uint64_t limit = g, hid = 0;  // entries below the limit stay unpublished
   if (ctl->sel.valid > kPubMaxEntries) {
-    const uint32_t x = warp_sort_desc(wk[lane], lane);
-    limit = max(g, __shfl_sync(0xFFFFFFFFu, x, (int)p.pub_m - 1));
-    hid = limit > g ? limit : 0u;  // (no entry below g belongs to the result)
+    const uint32_t x = __shfl_sync(0xFFFFFFFFu, warp_sort_desc<uint32_t>(keys[lane], lane), (int)p.pub_m - 1);
+    if (x > gkey) limit = hid = (uint64_t)x << 32;  // (no entry below g belongs to the result)
   }
 #pragma unroll 4
   for (uint32_t j = t; j < n; j += kScanThreads) {
     const uint2 e = cand[j];
-    if (e.x >= limit) {
+    if (composite(e.x, e.y) >= limit) {
       const uint32_t at = atomicAdd(&ctl->sel.wcount, 1u);
       if (at < kPubMaxEntries) list[at] = e;
     }
@@ -380,11 +413,11 @@ __device__ __forceinline__ bool publish_entries(const ScanParams &p, const uint2
   bsync();
   if (warp == 0) {
     const uint32_t c = min(ctl->sel.wcount, kPubMaxEntries);
-    if (ctl->sel.wcount > kPubMaxEntries) hid = 0xFFFFFFFFu;  // (ties at the limit)
+    if (ctl->sel.wcount > kPubMaxEntries) hid = ~0ull;  // (equal keys at the limit)
     uint32_t base = 0;
     if (lane == 0) {
       if (c) base = atomicAdd(&sc->pub_n, c);
-      if (hid) atomicMax(&sc->hid_key, hid);
+      if (hid) atomicMax(&sc->g_hid, (unsigned long long)hid);
     }
     base = __shfl_sync(0xFFFFFFFFu, base, 0);
     for (uint32_t j = lane; j < c; j += 32) p.pub[base + j] = list[j];
@@ -417,10 +450,10 @@ __device__ __forceinline__ uint32_t rank_of(const unsigned long long *comp, uint
 
 // The coordinator (block 0 of a launch with p.pub): scans nothing.  Per epoch, once every
 // scanning CTA has published, it raises the global threshold to the k-th largest of the
-// epoch's keys (k real objects score at least that).  At the end it takes the k-th
-// largest published key T: when hid_key <= T the published entries at or above T hold the
-// result and it answers the query; else T becomes the global threshold and the merge
-// tree answers.  A block of its own, because the CTA that arrives last -- the slowest --
+// epoch's entries (k real objects reach that).  At the end it takes the k-th best
+// published entry T: when g_hid <= T the published entries at or above T hold the result
+// and it answers the query; else T's key becomes the global threshold and the merge tree
+// answers.  A block of its own, because the CTA that arrives last -- the slowest --
 // would be held up by this work in every epoch, and its code stays in the instruction
 // cache from epoch to epoch.  Its waits are bounded; given up, the tree answers.
 __device__ __noinline__ void coordinate(const ScanParams &p, SmemCtl *ctl, uint2 *buf, uint32_t *hist) {
@@ -432,9 +465,10 @@ __device__ __noinline__ void coordinate(const ScanParams &p, SmemCtl *ctl, uint2
   const uint32_t stage_cap = 2u * p.mcap - kLinBins;
   uint32_t *bins = stage + stage_cap;
   uint32_t epoch = 0;
+  bool owner = false;  // thread 0: this block answered
 #pragma unroll 1
   for (;;) {
-    // wait for the epoch (8 arrivals per CTA) or the end, whichever is first
+    // wait for the epoch or the end, whichever is first
     if (t == 0) {
       uint32_t st = 2;  // given up, or decided by a CTA that waited out
       for (uint64_t it = 0; it < p.wait_limit; ++it) {
@@ -444,7 +478,7 @@ __device__ __noinline__ void coordinate(const ScanParams &p, SmemCtl *ctl, uint2
           st = 1;
           break;
         }
-        if (ep == 8u * ncta) {
+        if (ep == ncta) {
           st = 0;
           break;
         }
@@ -462,86 +496,100 @@ __device__ __noinline__ void coordinate(const ScanParams &p, SmemCtl *ctl, uint2
     }
     __threadfence();
     if (st == 0) {
-      const KthBound b = block_kth_bound<kScanThreads, 1>(p.epub + (size_t)epoch * p.epub_stride,
-                                                          ncta * p.epoch_keys, p.k, stage, stage_cap, bins, hist);
+      const KthBound b = block_kth_bound<kScanThreads>(p.epub + (size_t)epoch * p.epub_stride, ncta * p.epoch_keys,
+                                                       p.k, stage, stage_cap, bins, hist);
       if (t == 0) {
         if (b.key) {
           atomicMax(&sc->g_thr, b.key);
+          atomicMax(&sc->g_keep, (unsigned long long)b.word());
           // in id order the rows that a CTA still has to scan when it sees this bound come
           // after every published one: they lose a tie with it
           atomicMax(&sc->g_app, b.key + (p.row_ids ? 0u : 1u));
         }
-        if (epoch == 0) atomicExch(&sc->epoch0_ready, b.key + 1u);
+        if (epoch == 0) {
+          __threadfence();
+          atomicExch(&sc->epoch0_ready, 1u);
+        }
       }
       ++epoch;
       continue;
     }
-    const uint32_t np = ld_volatile_u32(&sc->pub_n), hid_key = ld_volatile_u32(&sc->hid_key);
+    const uint32_t np = ld_volatile_u32(&sc->pub_n);
+    const uint64_t hid = ld_volatile_u64(&sc->g_hid);
     unsigned long long *comp = reinterpret_cast<unsigned long long *>(buf);
     const bool few = np <= kRankMax;  // ranked at once, no bound needed first
-    KthBound b{0u, np, true};
-    // more equal scores than a CTA or this block can hold: the tree takes them as they are
-    if (hid_key == 0xFFFFFFFFu || np > kScanThreads * kKthRegs + stage_cap) {
-      b.covered = false;
-    } else if (few) {
+    KthBound b{0u, 0u, 0u};
+    if (t == 0) {
+      ctl->sel.wcount = 0;
+      ctl->keep = 0;
+    }
+    bsync();
+    if (few) {
       unsigned long long mine = 0ull;
       if (t < (int)np) {
         const uint2 e = __ldcg(p.pub + t);
         mine = composite(e.x, e.y);
         comp[t] = mine;
       }
-      if (t == 0) ctl->red_g = 0;
       bsync();
-      uint32_t r = rank_of(comp, np, mine);
-      if (t < (int)np && r == p.k - 1u) ctl->red_g = (uint32_t)(mine >> 32);  // the k-th key
+      if (t < (int)np && rank_of(comp, np, mine) == p.k - 1u) ctl->keep = mine;  // the k-th
       bsync();
-      b.key = ctl->red_g;
-      if (np < p.k) b.key = 0;
+      b.key = (uint32_t)(ctl->keep >> 32);
+      b.low = (uint32_t)ctl->keep;
     } else {
-      b = block_kth_bound<kScanThreads, 2>(reinterpret_cast<const uint32_t *>(p.pub), np, p.k, stage, stage_cap, bins,
-                                           hist);
+      b = block_kth_bound<kScanThreads>(p.pub, np, p.k, stage, stage_cap, bins, hist);
     }
-    // (no bound: fewer than k keys above 0 were published, and all count)
-    const uint32_t cnt = few || !b.key ? np : b.count;
-    const bool complete = b.covered && (b.key ? hid_key <= b.key : hid_key == 0u);
-    if (t == 0) {
-      if (b.key) atomicMax(&sc->g_thr, b.key);
-      __threadfence();
-      const bool want = complete && cnt <= stage_cap / 3u;  // (an entry and its place in the order: 3 words)
-      const uint32_t old = atomicCAS(&sc->gen, gen0, want ? gen0 + 2u : gen0 | 1u);
-      ctl->state = want && old == gen0 ? kEndDone : kEndTree;  // (a CTA that waited out takes the tree)
-      ctl->sel.wcount = 0;
-      ctl->red_g = 0;
+    const uint64_t least = b.key ? b.word() : 0ull;
+    const uint32_t room = stage_cap / 3u;  // (an entry and its place in the order: 3 words)
+    if (!few && hid != ~0ull) {  // the entries at or above the bound (no bound: all of them)
+      for (uint32_t base = 0; base < np; base += kScanThreads * 8u) {  // uniform trip count
+        uint2 e[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const uint32_t j = base + (uint32_t)u * kScanThreads + t;
+          e[u] = j < np ? __ldcg(p.pub + j) : make_uint2(0u, 0xFFFFFFFFu);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const bool in = base + (uint32_t)u * kScanThreads + t < np && composite(e[u].x, e[u].y) >= least;
+          const unsigned bal = __ballot_sync(0xFFFFFFFFu, in);
+          if (!bal) continue;
+          uint32_t at = 0;
+          if ((t & 31) == 0) at = atomicAdd(&ctl->sel.wcount, (uint32_t)__popc(bal));
+          at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(bal & ((1u << (t & 31)) - 1u));
+          if (in && at < room) buf[at] = e[u];
+        }
+      }
+      bsync();
     }
-    bsync();
-    if (ctl->state == kEndTree) break;
+    const uint32_t cnt = few ? np : ctl->sel.wcount;
+    const bool complete = hid != ~0ull && cnt <= room && (b.key ? hid <= least : hid == 0ull);
+    if (!complete) {
+      if (t == 0) {
+        if (b.key) atomicMax(&sc->g_thr, b.key);
+        __threadfence();
+        atomicCAS(&sc->gen, gen0, gen0 | 1u);
+      }
+      break;
+    }
+    // (the answer is exact whoever decides: it is written while the decision is on its way)
+    if (t == 0) owner = atomicCAS(&sc->gen, gen0, gen0 + 2u) == gen0;
     // rank every entry at or above the bound; the best k are the result, ascending
     const uint32_t res_n = min(cnt, p.k);
     auto emit = [&](uint32_t r, uint32_t key, uint32_t id) {
       if (r >= res_n) return;
       const uint32_t pos = res_n - 1u - r;
-      if (p.out_ids) {
-        p.out_ids[pos] = (uint64_t)id;
-        p.out_scores[pos] = key2f(key);
-      }
-      if (pos == 0) {
-        if (p.out_threshold) *p.out_threshold = key2f(key);
-        ctl->red_g = key;
-      }
+      p.out_ids[pos] = (uint64_t)id;
+      p.out_scores[pos] = key2f(key);
+      if (pos == 0 && p.out_threshold) *p.out_threshold = key2f(key);
     };
-    if (!few) {
-#pragma unroll 4
-      for (uint32_t j = t; j < np; j += kScanThreads) {
-        const uint2 e = __ldcg(p.pub + j);
-        if (e.x >= b.key) {
-          const uint32_t at = atomicAdd(&ctl->sel.wcount, 1u);  // < cnt
-          if (cnt <= kRankMax) comp[at] = composite(e.x, e.y);
-          else buf[at] = e;
-        }
+    if (cnt <= kRankMax) {  // by counting alone
+      if (!few) {
+        const uint2 e = t < (int)cnt ? buf[t] : make_uint2(0u, 0u);
+        bsync();
+        comp[t] = composite(e.x, e.y);
+        bsync();
       }
-      bsync();
-    }
-    if (cnt <= kRankMax) {
       if (t < (int)cnt) {
         const unsigned long long mine = comp[t];
         emit(rank_of(comp, cnt, mine), (uint32_t)(mine >> 32), 0xFFFFFFFFu - (uint32_t)mine);
@@ -559,13 +607,15 @@ __device__ __noinline__ void coordinate(const ScanParams &p, SmemCtl *ctl, uint2
     bsync();
     if (t == 0) {
       if (!res_n && p.out_threshold) *p.out_threshold = 0.0f;
-      write_stats(p, cnt, res_n, ctl->red_g);
+      write_stats(p, cnt, res_n);
     }
-    if (t == 0) reset_scratch(sc);
-    return;
+    break;
   }
-  // through the tree: the later of this block and the tree's root resets the scratch
-  if (t == 0) {
+  if (t != 0) return;
+  if (owner) {
+    reset_scratch(sc);
+  } else {
+    // through the tree: the later of this block and the tree's root resets the scratch
     __threadfence();
     if (atomicAdd(&sc->finishers, 1u) == 1u) {
       reset_scratch(sc);
@@ -574,57 +624,11 @@ __device__ __noinline__ void coordinate(const ScanParams &p, SmemCtl *ctl, uint2
   }
 }
 
-// A threshold pass ends here (KTH): each warp publishes the best pub_m / 8 of its
-// threads' words, the last CTA writes the k-th largest published key (0 when fewer than
-// k were published).
-template <int NB>
-__device__ __forceinline__ void kth_pass_end(const ScanParams &p, uint64_t (&best)[NB], uint2 *cand0, SmemCtl *ctl,
-                                          uint32_t *hist) {
-  const int t = threadIdx.x;
-  const int lane = t & 31;
-  const uint32_t r = p.pub_m / 8u;
-  uint2 *mine = p.pub + (size_t)blockIdx.x * p.pub_m + (size_t)(t >> 5) * r;
-  for (uint32_t i = 0; i < r; ++i) {
-    uint64_t m = best[0];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const uint64_t y = __shfl_xor_sync(0xFFFFFFFFu, m, o);
-      m = y > m ? y : m;
-    }
-    if (m != 0ull && best[0] == m) {  // the one lane that holds it pops it
-#pragma unroll
-      for (int x = 0; x + 1 < NB; ++x) best[x] = best[x + 1];
-      best[NB - 1] = 0ull;
-    }
-    if (lane == 0) mine[i] = make_uint2((uint32_t)(m >> 32), 0u);
-  }
-  __threadfence();
-  bsync();
-  if (t == 0) ctl->is_last = atomicAdd(&p.scratch->pub_arrived, 1u) == gridDim.x - 1u ? 1u : 0u;
-  bsync();
-  if (!ctl->is_last) return;
-  __threadfence();
-  const KthBound b = block_kth_bound<kScanThreads, 2>(reinterpret_cast<const uint32_t *>(p.pub), gridDim.x * p.pub_m,
-                                                      p.k, reinterpret_cast<uint32_t *>(cand0), 2u * p.mcap - kLinBins,
-                                                      reinterpret_cast<uint32_t *>(cand0 + p.mcap) - kLinBins, hist);
-  if (t == 0) {
-    *p.out_kth_key = b.key;
-    p.scratch->g_thr = 0;
-    p.scratch->acc_reductions = 0;
-    p.scratch->acc_tiles = 0;
-    p.scratch->pub_arrived = 0;
-    __threadfence();
-  }
-}
-
 // QQ: compile-time attribute count (0 = runtime, any qq <= kMaxQ).  PART: partition
-// mode (p.part_list set): tiles of listed partitions of a reordered copy.  KTH: a
-// threshold pass (p.kth_only, p.pub set): no candidate buffer, no select and no merge;
-// each thread keeps the best kPubMaxPerWarp (key, row) words of its own objects in
-// registers, each warp publishes its best pub_m / 8 of them, and the last CTA writes
-// the k-th largest published key.
-template <int QQ, bool PART, bool KTH>
-__global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_select_kernel(const __grid_constant__ ScanParams p) {
+// mode (p.part_list set): tiles of listed partitions of a reordered copy.
+template <int QQ, bool PART>
+__global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ, PART>())
+    scan_select_kernel(const __grid_constant__ ScanParams p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   SmemCtl *ctl = reinterpret_cast<SmemCtl *>(smem + kOffCtl);
   uint64_t *never = reinterpret_cast<uint64_t *>(smem + kOffNever);
@@ -642,7 +646,7 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
   const uint32_t qq = QQ > 0 ? (uint32_t)QQ : p.qq;
   const uint32_t cap = p.cap;
   // scanning CTAs: all blocks, or all but block 0, the coordinator (p.pub)
-  const uint32_t ncta = p.ncta, cta = blockIdx.x - (!KTH && p.pub ? 1u : 0u);
+  const uint32_t ncta = p.ncta, cta = blockIdx.x - (p.pub ? 1u : 0u);
 
   if (QQ == 0 && t < (int)kMaxQ && t < (int)qq) wsm[t] = p.w[t];
   if (t == 0) {
@@ -659,7 +663,7 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
     // (without the tree's flag: a CTA may start after another one has waited out)
     ctl->gen0 = ld_volatile_u32(&p.scratch->gen) & ~1u;
     ctl->epoch0_seen = 0;
-    ctl->keep_min = 0;
+    ctl->keep = 0;
     ctl->epoch = 0;
     ctl->my_tiles = cta < p.num_tiles ? (p.num_tiles - cta + ncta - 1) / ncta : 0;
   }
@@ -675,7 +679,7 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
     }
   }
 
-  if (!KTH && p.pub && blockIdx.x == 0) {
+  if (p.pub && blockIdx.x == 0) {
     coordinate(p, ctl, cand0, hist);
     return;
   }
@@ -727,19 +731,16 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
   uint32_t after = 0;  // fill after this thread's warp last appended, since the last vote
   // the tiles run in segments, each ended by a threshold epoch (the last by the end)
   uint32_t seg = 0, seg_len = p.epochs ? 1u : ctl->my_tiles;  // the segment's first tile and length
-  uint64_t kbest[KTH ? kPubMaxPerWarp : 1];  // KTH: this thread's best words, descending
-#pragma unroll
-  for (int b = 0; b < (KTH ? (int)kPubMaxPerWarp : 1); ++b) kbest[b] = 0ull;
   // q <= 2 in id order: two tiles per loop pass, so the prefetched registers swap roles
   // instead of being copied (q = 2 on 2^28 rows: 0.420 -> 0.406 ms)
   constexpr int kUnroll = kVoteTiles == 2 ? 2 : 1;
   bool stopped = false;
   for (;;) {
-    // the segment's first loads; its last tile prefetches nothing, so the epoch's code
-    // holds no loads in flight in registers
+    // the segment's first loads; in id order its last tile prefetches nothing, so the
+    // epoch's code holds no loads in flight in registers (partition mode has the registers)
     if (prefetch && seg_len) {
       if constexpr (PART) {
-        load_rows(tile_row(seg, part_cur), xn);
+        if (seg == 0) load_rows(tile_row(0, part_cur), xn);
       } else {
         next_row = p.tile_begin + ((uint64_t)cta + (uint64_t)seg * ncta) * p.tile_step;
         next_tix = cta + seg * ncta;
@@ -755,7 +756,7 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
       // every thread reads the same thresholds in tile i (see SmemCtl::thr_g); in id
       // order they are read after the scores, so they hold no register across the loads
       uint32_t thr = 0;
-      if constexpr (PART && !KTH) {
+      if constexpr (PART) {
         thr = max(ctl->thr_local, ctl->thr_g[i & 1u]);
         // nothing in this partition (nor in any later one of this CTA) can reach thr
         if (key_cur < thr) {
@@ -772,14 +773,12 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
         float4 x[kPQ];
 #pragma unroll
         for (int m = 0; m < kPQ; ++m) x[m] = xn[m];
-        if (i + 1 < seg_len) {
-          if constexpr (PART) {
-            load_rows(tile_row(seg + i + 1, part_nx), xn);
-          } else {
-            next_row += p.grid_rows;
-            next_tix += ncta;
-            load_next(xn);
-          }
+        if constexpr (PART) {
+          if (seg + i + 1 < ctl->my_tiles) load_rows(tile_row(seg + i + 1, part_nx), xn);
+        } else if (i + 1 < seg_len) {
+          next_row += p.grid_rows;
+          next_tix += ncta;
+          load_next(xn);
         }
         s = score_cols<kPQ>(p, x);
       } else {
@@ -791,23 +790,6 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
         if (seg + i + 2 < ctl->my_tiles) part_of(seg + i + 2, part_nx, key_nx);
       }
 
-      if constexpr (KTH) {
-        // a threshold pass: every object of the tile against this thread's best words
-        const float sk[4] = {s.x, s.y, s.z, s.w};
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const bool ok = interior || (row0 + v >= p.row_begin && row0 + v < p.row_end);
-          uint64_t c = ok ? composite(f2key(sk[v]), (uint32_t)(row0 + v)) : 0ull;
-#pragma unroll
-          for (int b = 0; b < (int)kPubMaxPerWarp; ++b)
-            if (c > kbest[b]) {
-              const uint64_t x = kbest[b];
-              kbest[b] = c;
-              c = x;
-            }
-        }
-        continue;
-      }
       if constexpr (!PART) thr = max(ctl->thr_local, ctl->thr_g[i & 1u]);
       // key(score) >= thr  <=>  thr == 0 (everything, NaN included) or score >= thr_float(thr)
       const bool take_all = thr == 0u;
@@ -849,11 +831,13 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
       }
       // thread 0 hands the CTA its copy of the global threshold (see SmemCtl::thr_g): it
       // loads the global word every 4 tiles and applies it 3 tiles later, so the L2 round
-      // trip is never waited on.  The new value goes to the slot the next tile reads, and
-      // on the tile after into the other slot too; between updates both slots agree.
+      // trip is never waited on (every 2 and 1 later in partition mode, where it ends the
+      // scan).  The new value goes to the slot the next tile reads, and on the tile after
+      // into the other slot too; between updates both slots agree.
+      constexpr uint32_t kPoll = PART ? 1u : 3u;
       if (t == 0) {
-        if ((i & 3u) == 3u) ctl->thr_g[(i + 1u) & 1u] = max(ctl->thr_g[i & 1u], g_pending);
-        if ((i & 3u) == 0u) {
+        if ((i & kPoll) == kPoll) ctl->thr_g[(i + 1u) & 1u] = max(ctl->thr_g[i & 1u], g_pending);
+        if ((i & kPoll) == 0u) {
           ctl->thr_g[(i + 1u) & 1u] = ctl->thr_g[i & 1u];
           g_pending = max(ld_volatile_u32(&p.scratch->g_thr), ld_volatile_u32(&p.scratch->g_app));
         }
@@ -864,27 +848,14 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
       after = 0;
       if (full && seg + i + 1 < ctl->my_tiles) {
         if (t == 0) {
-          uint32_t g = ctl->keep_min;  // (k entries of this CTA or k published objects reach it)
           // the first fill may come before any bound: epoch 0's is on its way, and dropping
           // what lies below it costs one pass over the buffer instead of a select
-          if (p.epochs && !ctl->epoch0_seen) {
-            uint32_t w = ld_volatile_u32(&p.scratch->epoch0_ready);
-            for (uint32_t it = 0; it < p.epoch_wait && !w && !g; ++it) {
-              __nanosleep(kEpochWaitNs);
-              w = ld_volatile_u32(&p.scratch->epoch0_ready);
-            }
-            ctl->epoch0_seen = (w || !g) ? 1u : 0u;
-            if (w) g = max(g, w - 1u);
-          }
-          g = max(g, ld_volatile_u32(&p.scratch->g_thr));
-          ctl->red_g = ctl->keep_min = g;
-          ctl->thr_g[0] = ctl->thr_g[1] =
-              max(max(ctl->thr_g[0], ctl->thr_g[1]), max(g, ld_volatile_u32(&p.scratch->g_app)));
+          take_bound(p, ctl, ctl->keep == 0ull);
           ctl->sel.wcount = 0;
         }
         bsync();
         // what lies below the bound out of the buffer, in place; a select when much is left
-        const uint32_t left = block_compact<kScanThreads>(cand0, ctl->count, ctl->red_g, &ctl->sel);
+        const uint32_t left = block_compact<kScanThreads>(cand0, ctl->count, ctl->keep, &ctl->sel);
         if (left <= (cap - kVoteTiles * kTile) / 2u) {
           if (t == 0) ctl->count = left;
           bsync();
@@ -910,6 +881,10 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
     seg += i;
     if (stopped || ctl->epoch >= p.epochs) break;
     epoch_publish(p, cand0, ctl, hist);
+    if (PART && p.epoch_hold && ctl->epoch == 1u) {  // (a small copy: few tiles to stop before)
+      if (t == 0) take_bound(p, ctl, true);
+      bsync();
+    }
     seg_len = (ctl->epoch < p.epochs ? seg << p.epoch_shift : ctl->my_tiles) - seg;
   }
 
@@ -918,10 +893,6 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
   if (t == 0 && ctl->reductions) atomicAdd(&p.scratch->acc_reductions, ctl->reductions);
   if (PART && t == 0) atomicAdd(&p.scratch->acc_tiles, seg);
 
-  if constexpr (KTH) {
-    kth_pass_end(p, kbest, cand0, ctl, hist);
-    return;
-  }
   if (p.pub && !publish_entries(p, cand0, ctl, hist)) return;
 
   // ---- merge tree: this CTA's best k first ----
@@ -1048,32 +1019,27 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ>()) scan_sele
 
 using ScanKernel = void (*)(ScanParams);
 
-// [kth][part][q] for q = 1..16; [..][0] is the runtime-q kernel used for q > 16
-#define TOPK_SCAN_ROW(P, K)                                                                                   \
-  {scan_select_kernel<0, P, K>,  scan_select_kernel<1, P, K>,  scan_select_kernel<2, P, K>,                   \
-   scan_select_kernel<3, P, K>,  scan_select_kernel<4, P, K>,  scan_select_kernel<5, P, K>,                   \
-   scan_select_kernel<6, P, K>,  scan_select_kernel<7, P, K>,  scan_select_kernel<8, P, K>,                   \
-   scan_select_kernel<9, P, K>,  scan_select_kernel<10, P, K>, scan_select_kernel<11, P, K>,                  \
-   scan_select_kernel<12, P, K>, scan_select_kernel<13, P, K>, scan_select_kernel<14, P, K>,                  \
-   scan_select_kernel<15, P, K>, scan_select_kernel<16, P, K>}
-const ScanKernel kKernels[2][2][17] = {{TOPK_SCAN_ROW(false, false), TOPK_SCAN_ROW(true, false)},
-                                       {TOPK_SCAN_ROW(false, true), TOPK_SCAN_ROW(true, true)}};
+// [part][q] for q = 1..16; [..][0] is the runtime-q kernel used for q > 16
+#define TOPK_SCAN_ROW(P)                                                                                        \
+  {scan_select_kernel<0, P>,  scan_select_kernel<1, P>,  scan_select_kernel<2, P>,  scan_select_kernel<3, P>,   \
+   scan_select_kernel<4, P>,  scan_select_kernel<5, P>,  scan_select_kernel<6, P>,  scan_select_kernel<7, P>,   \
+   scan_select_kernel<8, P>,  scan_select_kernel<9, P>,  scan_select_kernel<10, P>, scan_select_kernel<11, P>,  \
+   scan_select_kernel<12, P>, scan_select_kernel<13, P>, scan_select_kernel<14, P>, scan_select_kernel<15, P>,  \
+   scan_select_kernel<16, P>}
+const ScanKernel kKernels[2][17] = {TOPK_SCAN_ROW(false), TOPK_SCAN_ROW(true)};
 #undef TOPK_SCAN_ROW
 
-ScanKernel kernel_for(uint32_t qq, bool part, bool kth = false) {
-  return kKernels[kth ? 1 : 0][part ? 1 : 0][qq <= 16 ? qq : 0];
-}
+ScanKernel kernel_for(uint32_t qq, bool part) { return kKernels[part ? 1 : 0][qq <= 16 ? qq : 0]; }
 
 }  // namespace
 
 cudaError_t scan_set_attributes(size_t smem_optin) {
-  for (const auto &mode : kKernels)
-    for (const auto &row : mode)
-      for (ScanKernel f : row) {
-        const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void *>(f),
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_optin);
-        if (e != cudaSuccess) return e;
-      }
+  for (const auto &row : kKernels)
+    for (ScanKernel f : row) {
+      const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void *>(f),
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_optin);
+      if (e != cudaSuccess) return e;
+    }
   return cudaSuccess;
 }
 
@@ -1089,13 +1055,13 @@ constexpr size_t kSmemPerCtaReserve = 1024;
 // The shared-memory carveout last set on each scan kernel, per device (the attribute
 // is per function and device; setting it again costs a driver call).
 std::mutex g_carveout_mu;
-int g_carveout[64][2][2][17];
+int g_carveout[64][2][17];
 
-void set_carveout(const void *fn, bool part, uint32_t qq, int percent, bool kth = false) {
+void set_carveout(const void *fn, bool part, uint32_t qq, int percent) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
   std::lock_guard<std::mutex> lk(g_carveout_mu);
-  int &cur = g_carveout[dev][kth ? 1 : 0][part ? 1 : 0][qq <= 16 ? qq : 0];
+  int &cur = g_carveout[dev][part ? 1 : 0][qq <= 16 ? qq : 0];
   if (cur == percent + 1) return;  // stored plus one: 0 means not set yet
   if (cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, percent) == cudaSuccess)
     cur = percent + 1;
@@ -1127,7 +1093,6 @@ ScanPlan plan_scan(uint32_t qq, uint32_t k, uint64_t rows, int num_sms, size_t s
   }
   const auto key = std::make_tuple(dev, qq <= 16 ? qq : 0u, k, part, max_ctas_per_sm);
   const void *fn = reinterpret_cast<const void *>(kernel_for(qq, part));
-  const void *fn_kth = reinterpret_cast<const void *>(kernel_for(qq, part, true));
   const uint64_t tiles = (rows + 3 + kTile) / kTile;
   auto finish = [&](ScanPlan pl) {
     uint64_t grid = (uint64_t)num_sms * (uint64_t)pl.ctas_per_sm - 1u;  // one place for the coordinator
@@ -1143,7 +1108,6 @@ ScanPlan plan_scan(uint32_t qq, uint32_t k, uint64_t rows, int num_sms, size_t s
       const PlanEntry pe = it->second;
       // the carveout is per function: another plan may have changed it since
       set_carveout(fn, part, qq, pe.carveout);
-      set_carveout(fn_kth, part, qq, pe.carveout, true);
       return finish(pe.pl);
     }
   }
@@ -1157,6 +1121,9 @@ ScanPlan plan_scan(uint32_t qq, uint32_t k, uint64_t rows, int num_sms, size_t s
   // rounding below leaves some, and more would cost q <= 2 a CTA per SM)
   const uint32_t vote_tiles = scan_vote_tiles(qq <= 16 ? (int)qq : 0, part);
   uint32_t cap = k + vote_tiles * kTile + (vote_tiles == 1 ? kTile / 2 : 0u);
+  // partition mode: room for two tiles more, so that no CTA waits for epoch 0's bound with a
+  // full buffer (its few CTAs per SM leave the shared memory)
+  if (part) cap += 2 * kTile;
   if (cap < P) cap = P;
   if (cap < 2048) cap = 2048;
   cap = (cap + kScanThreads - 1) / kScanThreads * kScanThreads;
@@ -1195,8 +1162,6 @@ ScanPlan plan_scan(uint32_t qq, uint32_t k, uint64_t rows, int num_sms, size_t s
     }
   const int carveout = (int)((size_kb * 100 + 227) / 228);
   set_carveout(fn, part, qq, carveout);
-  // the threshold-pass form of the kernel runs with the same plan
-  set_carveout(fn_kth, part, qq, carveout, true);
   int fit = 0;  // what the driver reports with that preference
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, kScanThreads, pl.smem) == cudaSuccess && fit >= 1)
     occ = std::min(occ, fit);
@@ -1232,9 +1197,6 @@ void plan_merge_tree(ScanParams &p, uint32_t grid, uint32_t fanin, uint32_t *tot
 
 cudaError_t launch_scan(const ScanPlan &pl, const ScanParams &p, cudaStream_t stream) {
   if (pl.stages < 1) return cudaErrorInvalidValue;
-  // a threshold pass needs the published-keys area
-  if (p.kth_only && (!p.pub || !p.out_kth_key || p.pub_m == 0 || p.pub_m > 8 * kPubMaxPerWarp))
-    return cudaErrorInvalidValue;
   ScanParams q = p;
   for (uint32_t m = 0; m < 4; ++m) q.colp[m] = m < p.qq ? p.table + (uint64_t)p.attr[m] * p.ld : p.table;
   q.ncta = (uint32_t)pl.grid;
@@ -1245,8 +1207,8 @@ cudaError_t launch_scan(const ScanPlan &pl, const ScanParams &p, cudaStream_t st
   if (p.row_end >= p.tile_begin + kTile) hi = (p.row_end - p.tile_begin - kTile) / p.tile_step + 1;
   if (hi > p.num_tiles) hi = p.num_tiles;
   q.int_n = hi > q.int_lo ? (uint32_t)(hi - q.int_lo) : 0u;
-  const int grid = pl.grid + (p.pub && !p.kth_only ? 1 : 0);  // and the coordinator
-  kernel_for(p.qq, p.part_list != nullptr, p.kth_only != 0)<<<grid, kScanThreads, pl.smem, stream>>>(q);
+  const int grid = pl.grid + (p.pub ? 1 : 0);  // and the coordinator
+  kernel_for(p.qq, p.part_list != nullptr)<<<grid, kScanThreads, pl.smem, stream>>>(q);
   return cudaGetLastError();
 }
 

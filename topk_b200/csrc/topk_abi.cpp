@@ -92,12 +92,11 @@ struct Ctx {
   // published best entries (kPubMaxEntries per CTA of the largest grid), one allocation:
   // pub[max_grid * kPubMaxEntries] | epub[kMaxEpochs][max_grid * kPubMaxKeys]
   uint2 *pub = nullptr;
-  uint32_t *epub = nullptr;
+  uint2 *epub = nullptr;
   uint32_t epub_stride = 0;
   uint32_t max_slots = 0, max_groups = 0;
   size_t slot_entries = 0;  // capacity of `slots`
   size_t meta_bytes = 0;    // bytes that must be zero between queries (header + done)
-  unsigned char *d_res = nullptr;  // device result block (kMaxK capacity)
   unsigned char *h_res = nullptr;  // pinned mirror
   // Result block of the synchronous queries in mapped pinned memory (h_out on the host,
   // d_out its device address): the scan's root writes ids, scores and the header
@@ -215,7 +214,6 @@ int ctx_create(topk_table_t h, Ctx **out) {
     if (c->stream) cudaStreamDestroy(c->stream);
     cudaFree(c->scratch);
     cudaFree(c->pub);
-    cudaFree(c->d_res);
     cudaFree(c->d_count2);
     if (c->h_res) cudaFreeHost(c->h_res);
     if (c->h_out) cudaFreeHost(c->h_out);
@@ -244,11 +242,10 @@ int ctx_create(topk_table_t h, Ctx **out) {
   if ((e = cudaMemset(blk, 0, slots_off)) != cudaSuccess) return bail(e, "scratch memset");
   c->epub_stride = kPubMaxKeys * max_grid;
   const size_t pub_entries_max = (size_t)kPubMaxEntries * max_grid;
-  if ((e = cudaMalloc(&c->pub, pub_entries_max * sizeof(uint2) +
-                                   (size_t)kMaxEpochs * c->epub_stride * sizeof(uint32_t))) != cudaSuccess)
+  if ((e = cudaMalloc(&c->pub, (pub_entries_max + (size_t)kMaxEpochs * c->epub_stride) * sizeof(uint2))) !=
+      cudaSuccess)
     return bail(e, "publish area");
-  c->epub = reinterpret_cast<uint32_t *>(c->pub + pub_entries_max);
-  if ((e = cudaMalloc(&c->d_res, result_bytes(kMaxK))) != cudaSuccess) return bail(e, "result block");
+  c->epub = c->pub + pub_entries_max;
   if ((e = cudaMalloc(&c->d_count2, 2 * sizeof(unsigned long long))) != cudaSuccess) return bail(e, "count");
   if ((e = cudaHostAlloc(&c->h_res, result_bytes(kMaxK) + kStageBytes, cudaHostAllocDefault)) != cudaSuccess)
     return bail(e, "pinned result");
@@ -266,7 +263,6 @@ void ctx_free(Ctx *c) {
   if (c->stream) cudaStreamDestroy(c->stream);
   cudaFree(c->scratch);
   cudaFree(c->pub);
-  cudaFree(c->d_res);
   cudaFree(c->d_count2);
   cudaFree(c->d_ids_scratch);
   cudaFree(c->d_rows);
@@ -334,9 +330,7 @@ struct PartScan {
   uint32_t seed;           // objects need key >= seed (0: none)
   const uint32_t *d_key;   // bound key of each listed partition (null: no stop rule)
   const uint32_t *d_seed;  // a further seed in device memory (null: none)
-  uint32_t *d_kth;         // receives the k-th key when k objects were found, else 0 (may be null)
   uint32_t max_ctas_per_sm;  // 0: as many as fit
-  bool kth_only;           // threshold pass: only the bound from the published keys, into d_kth
 };
 
 // Enqueue one fused scan over rows [r0, r1) (or over the partitions of `ps`)
@@ -378,7 +372,6 @@ int enqueue_scan(topk_table_t h, Ctx *c, cudaStream_t stream, uint64_t r0, uint6
     p.thr_seed = ps->seed;
     p.part_key = ps->d_key;
     p.thr_seed_dev = ps->d_seed;
-    p.out_kth_key = ps->d_kth;
     tiles = (uint64_t)ps->count << p.part_shift;
     if (tiles > 0xFFFFFFFFull) return fail(TOPK_ERR_UNSUPPORTED, "too many tiles");
   }
@@ -404,18 +397,19 @@ int enqueue_scan(topk_table_t h, Ctx *c, cudaStream_t stream, uint64_t r0, uint6
     return fail(TOPK_ERR_UNSUPPORTED, "merge tree of %d CTAs does not fit the scratch", pl.grid);
   p.wait_limit = h->wait_limit;
   p.fault_mode = (uint32_t)h->fault_mode;
-  if (const uint32_t m = pub_entries((uint32_t)k, (uint32_t)pl.grid)) {
+  const uint32_t shift = ps ? kPartEpochShift : kEpochShift;
+  const uint32_t epochs = scan_epochs(tiles, (uint32_t)pl.grid, shift);
+  if (const uint32_t m = pub_entries((uint32_t)k, (uint32_t)pl.grid, epochs)) {
     p.pub = c->pub;
     p.pub_m = m;
     p.pub_wait = kPubWaitPolls;
-    if (!ps) {
-      p.epub = c->epub;
-      p.epub_stride = c->epub_stride;
-      p.epoch_shift = kEpochShift;
-      p.epochs = scan_epochs(tiles, (uint32_t)pl.grid, kEpochShift);
-      p.epoch_keys = epoch_keys((uint32_t)k, (uint32_t)pl.grid);
-      p.epoch_wait = kEpochWaitPolls;
-    }
+    p.epub = c->epub;
+    p.epub_stride = c->epub_stride;
+    p.epoch_shift = shift;
+    p.epochs = epochs;
+    p.epoch_keys = epoch_keys((uint32_t)k, (uint32_t)pl.grid, ps != nullptr);
+    p.epoch_wait = kEpochWaitPolls;
+    p.epoch_hold = ps && epochs && tiles <= 16u * (uint64_t)pl.grid;
   }
   p.scratch = c->scratch;
   p.slots = c->slots;
@@ -429,26 +423,6 @@ int enqueue_scan(topk_table_t h, Ctx *c, cudaStream_t stream, uint64_t r0, uint6
   for (uint32_t m = 0; m < qq; m++) {
     p.attr[m] = attr[m];
     p.w[m] = weights[attr[m]];
-  }
-  if (ps && ps->kth_only) {
-    // Every CTA publishes up to 4k / grid keys (at most 8 * kPubMaxPerWarp), so the
-    // bound stays close to the k-th of the scanned rows even when their best objects
-    // sit in few CTAs.  When the grid is too small for that (few tiles, large k) the
-    // round runs the merge tree instead, whose root writes the exact k-th key of the
-    // rows it scanned.
-    const uint32_t m = pub_keys_per_cta(4 * (uint32_t)k, (uint32_t)pl.grid);
-    if ((uint64_t)m * (uint64_t)pl.grid >= 4 * k) {
-      p.pub = c->pub;
-      p.pub_m = m;
-      p.pub_wait = kPubWaitPolls;
-      p.kth_only = 1;
-    }
-    p.out_kth_key = ps->d_kth;
-    p.out_ids = nullptr;
-    p.out_scores = nullptr;
-    p.out_threshold = nullptr;
-    p.out_count = nullptr;
-    p.out_stats = nullptr;
   }
   CK(launch_scan(pl, p, stream));
   return TOPK_OK;
@@ -524,29 +498,28 @@ float host_key2f(uint32_t k) {
 std::vector<BatchQuery> pack_queries(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *qqs,
                                      const float *weights, uint64_t wstride, const uint8_t *attrs, uint64_t astride);
 
-// CTAs per SM of a pruned scan and of its first round (measured on 2^27 x 8, kd order:
-// 4 and 3 take 148 us a query against 153 for 3 and 4)
+// CTAs per SM of a pruned scan: it reads a small part of the table, and a few CTAs per SM
+// keep enough loads in flight for it.
 constexpr uint32_t kPrunedCtasPerSm = 4;
-constexpr uint32_t kRound1CtasPerSm = 3;
 
 // Exact top-k over the partitioned copy as one device pipeline on the context's
 // stream; nothing is decided on the host between the launches.
 //   1. A kernel orders the partitions by the query's bound (the reference-order FP32
 //      sum over each partition's extremes: an exact upper bound of its scores).
-//   2. Round 1 scans the first partitions of that order, about one wave of CTAs (and
-//      enough rows for k), and leaves its k-th key t1 in device memory: the k-th score
-//      of a subset, a lower bound of the true k-th.
-//   3. Round 2 scans the partitions in the same order seeded with t1 (ties at t1 kept),
-//      each CTA stopping at its first partition whose bound is below its running
+//   2. One scan over the partitions in that order.  Its threshold epochs (after tiles 1,
+//      2, 4, ... of every CTA) give all CTAs the k-th best of the partitions read so far,
+//      and each CTA stops at its first partition whose bound is below its running
 //      threshold -- the reference's stop rule per block (cpu/VTA.h:210-216,
-//      cpu/PTA.h:636-641); its merge tree gives the result.  (Round 1's partitions
-//      come again; rescanning them is cheaper than merging two results.)
+//      cpu/PTA.h:636-641).  (A launch of its own for a first threshold, over the best
+//      1/32 of the partitions, read those twice: over 96 random queries on 2^27 x 8 in kd order 4 attributes took 89 us a
+//      query at k = 128 and 205 with 8, now 66 and 158.)
 // With a seed (a predicted lower bound of the k-th score: `cut`, or the learned
-// model's cut computed on the device) round 2 alone runs with it, and its result is
+// model's cut computed on the device) the scan starts from it, and its result is
 // accepted when it holds min(k, n) objects (then the true k-th score is at least the
-// seed, so every object of the true top-k was scanned); otherwise the two rounds run
+// seed, so every object of the true top-k was scanned); otherwise the scan runs again
 // without it.  stats: partitions scanned (tiles scanned / tiles per partition, over
-// every scan), partitions, seed accepted (1/0), scans.
+// every scan), partitions, seed accepted (1/0), rounds: one for a scan with a seed, two
+// for a scan that finds its threshold on the way.
 int run_pruned(topk_table_t h, uint64_t k, uint32_t qq, const float *weights, const uint8_t *attr, float cut,
                bool learned, uint64_t *ids, float *scores, uint64_t *count, float *threshold, uint64_t *stats,
                float *cut_out) {
@@ -586,9 +559,7 @@ int run_pruned(topk_table_t h, uint64_t k, uint32_t qq, const float *weights, co
     if (c->ptemp_bytes) CK(cudaMalloc(&c->d_ptemp, c->ptemp_bytes));
     c->plist_cap = P;
   }
-  // device-side words (round 1's bound) in the device block; the result and the cut
-  // the host reads go straight to the mapped block
-  ResultHeader *dh = reinterpret_cast<ResultHeader *>(c->d_res);
+  // the result and the cut the host reads go straight to the mapped block
   unsigned char *dro = c->d_out;
   ResultHeader *dho = reinterpret_cast<ResultHeader *>(dro);
   uint64_t *d_ids = reinterpret_cast<uint64_t *>(dro + kHdr);
@@ -624,34 +595,16 @@ int run_pruned(topk_table_t h, uint64_t k, uint32_t qq, const float *weights, co
   const uint32_t seed_host = std::isfinite(cut) ? host_f2key(cut) : 0u;
   const bool seeded = learned || seed_host != 0u;
   const uint64_t tiles_per_part = (1ull << h->part_log2) / 1024u;
-  // round 1: about one wave of CTAs worth of the best partitions, and rows for k
-  const uint64_t R = 1ull << h->part_log2;
-  // A pruned scan reads a small part of the table: a few CTAs per SM keep enough loads
-  // in flight for it, and fewer CTAs mean a shallower merge tree (kPrunedCtasPerSm).
-  // Round 1 takes the best 1/32 of the partitions (and rows for k).
-  const uint32_t m1 = (uint32_t)std::min<uint64_t>(P, std::max<uint64_t>((kk + R - 1) / R + 1, (P + 31) / 32));
-  uint32_t *d_t1 = reinterpret_cast<uint32_t *>(&dh->pad[0]);  // round 1's k-th key
   uint64_t tiles = 0, scans = 0, accepted = 0;
   float cut_seen = cut;
-  // the seeded attempt (if any), then the two rounds without a seed
+  // the seeded attempt (if any), then the scan without a seed
   for (int attempt = seeded ? 0 : 1; attempt < 2; attempt++) {
     hh->count = 0xFFFFFFFFu;  // sentinel: a completed scan writes its count
-    if (attempt == 0) {
-      PartScan ps{c->d_plist, P, seed_host, c->d_pkey, d_seed, nullptr, kPrunedCtasPerSm, false};
-      st = enqueue_scan(h, c, s, 0, h->n, k, qq, weights, attr, d_ids, d_scores, &dho->threshold, &dho->count,
-                        dho->stats, &ps);
-      scans += 1;
-    } else {
-      // round 1: a threshold pass (no merge, no result) over its partitions
-      PartScan p1{c->d_plist, m1, 0u, nullptr, nullptr, d_t1, kRound1CtasPerSm, true};
-      st = enqueue_scan(h, c, s, 0, h->n, k, qq, weights, attr, d_ids, d_scores, &dho->threshold, &dho->count,
-                        nullptr, &p1);
-      if (st != TOPK_OK) return st;
-      PartScan p2{c->d_plist, P, 0u, c->d_pkey, d_t1, nullptr, kPrunedCtasPerSm, false};
-      st = enqueue_scan(h, c, s, 0, h->n, k, qq, weights, attr, d_ids, d_scores, &dho->threshold, &dho->count,
-                        dho->stats, &p2);
-      scans += 2;
-    }
+    const PartScan ps{c->d_plist, P, attempt == 0 ? seed_host : 0u, c->d_pkey, attempt == 0 ? d_seed : nullptr,
+                      kPrunedCtasPerSm};
+    st = enqueue_scan(h, c, s, 0, h->n, k, qq, weights, attr, d_ids, d_scores, &dho->threshold, &dho->count,
+                      dho->stats, &ps);
+    scans += attempt == 0 ? 1u : 2u;
     if (st != TOPK_OK) return st;
     CK(cudaStreamSynchronize(s));
     if (hh->count > kk) {
@@ -663,7 +616,7 @@ int run_pruned(topk_table_t h, uint64_t k, uint32_t qq, const float *weights, co
                   sc.error);
     }
     if (learned && attempt == 0) cut_seen = hh->cut;
-    tiles += hh->stats[2] + (attempt == 1 ? (uint64_t)m1 * tiles_per_part : 0u);
+    tiles += hh->stats[2];
     if (attempt == 1) break;
     if (hh->count == kk) {
       accepted = 1;

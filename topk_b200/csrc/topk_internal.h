@@ -16,15 +16,17 @@ constexpr int kMaxLevels = 12;        // merge-tree levels (fan-in >= 2, <= 4096
 constexpr int kScanSmemFixed = 1536;  // barriers, control block, radix histogram, weights
 
 // Threshold epochs of a scan (ScanParams::epochs): at most kMaxEpochs; in id order after
-// tiles 1, 4, 16, ... of every CTA.
-constexpr uint32_t kMaxEpochs = 6;
-constexpr uint32_t kEpochShift = 2;
+// tiles 1, 4, 16, ... of every CTA, in partition mode, where the threshold decides how far
+// the scan goes, after 1, 2, 4, 8, ...
+constexpr uint32_t kMaxEpochs = 8;
+constexpr uint32_t kEpochShift = 2, kPartEpochShift = 1;
 
 // Device-side per-context scratch of the fused scan.  Zero between queries (but for
 // `gen`): the kernel puts every counter back before it ends.
 struct ScanScratch {
   uint32_t g_thr;           // running global threshold key (objects below it cannot win)
   uint32_t g_app;           // the same for rows still to be scanned (ScanParams::epub)
+  unsigned long long g_keep;  // the last epoch's bound: objects below this (key, ~id) cannot win
   uint32_t error;           // nonzero after a device wait gave up (bit 0: stage wait)
   uint32_t acc_reductions;  // CTA block-selects during this scan
   uint32_t last_cands;      // entries merged at the root of the last scan
@@ -33,22 +35,22 @@ struct ScanScratch {
   // tile, two values); the access it guarded was skipped.
   uint32_t diag[5];
   uint32_t acc_tiles;       // tiles scanned during this scan (partition mode)
-  uint32_t pad0[20];
+  uint32_t pad0[18];
   // The words that CTAs count on or poll sit in lines of their own: hundreds of polls a
   // microsecond on one line hold up every other access to it.
+  unsigned long long g_hid; // no CTA holds an unpublished entry at or above this (key, ~id)
   uint32_t pub_arrived;     // CTAs that published their best entries (ScanParams::pub)
   uint32_t pub_n;           // entries published
-  uint32_t hid_key;         // no CTA holds an unpublished entry with a key at or above it
-  uint32_t epoch_arrived[kMaxEpochs];  // eight per CTA
+  uint32_t epoch_arrived[kMaxEpochs];  // CTAs that published for an epoch
   uint32_t finishers;       // merge tree: its root and the coordinator, the later resets
-  uint32_t pad1[22];
+  uint32_t pad1[19];
   // How the scan in flight ends: twice the number of scans finished on this scratch,
   // plus one while the current scan ends through its merge tree.  It moves on by two
   // when a scan is answered, so a CTA that waits for the decision sees it however
   // late it looks.
   uint32_t gen;
   uint32_t pad2[31];
-  uint32_t epoch0_ready;    // 1 once epoch 0's bound is in g_thr
+  uint32_t epoch0_ready;    // 1 once epoch 0's bound is in g_thr, g_app and g_keep
   uint32_t pad3[31];
 };
 static_assert(sizeof(ScanScratch) == 512, "four 128-byte lines");
@@ -72,7 +74,7 @@ struct ScanParams {
   uint64_t row_end;
   uint64_t tile_begin;  // row_begin rounded down to 4 (16-byte copies)
   uint64_t tile_end;    // row_end rounded up to 4 (<= ld)
-  uint64_t tile_step;   // rows from one tile to the next (the tile size; a multiple for a sample)
+  uint64_t tile_step;   // rows from one tile to the next (the tile size)
   uint32_t num_tiles;
   uint32_t qq;
   uint32_t k;
@@ -100,30 +102,26 @@ struct ScanParams {
   uint32_t pub_m;
   uint32_t pub_wait;
   // Threshold epochs (needs pub): after its tile 1, then 2^epoch_shift times as many,
-  // and so on (`epochs` of them) each CTA publishes the largest keys it holds (epoch_keys
-  // of them, 1 or a multiple of 8) in epub[epoch] (epub_stride keys each); the coordinator
-  // raises the global threshold to the k-th largest of them.  A CTA whose
+  // and so on (`epochs` of them) each CTA publishes the best entries it holds (epoch_keys
+  // of them, at most 32) in epub[epoch] (epub_stride entries each); the
+  // coordinator raises the global threshold to the k-th best of them.  A CTA whose
   // buffer fills before epoch 0's bound is there waits for it, at most epoch_wait polls.
-  uint32_t *epub;
+  uint2 *epub;
   uint32_t epub_stride;
   uint32_t epochs;
   uint32_t epoch_shift;
   uint32_t epoch_keys;
   uint32_t epoch_wait;
-  // Threshold pass (needs pub and out_kth_key): the published keys' k-th largest goes
-  // to *out_kth_key (0 when fewer than k were published) and the scan ends there, no
-  // merge and no result.  Run over a sample of the tiles (tile_step) it seeds the full
-  // scan that follows: k real objects score at least that key.  It runs the kernel's
-  // threshold-pass form: each thread keeps its best kPubMaxPerWarp (key, row) words in
-  // registers (no candidate buffer, no select), so pub_m <= 8 * kPubMaxPerWarp.
-  uint32_t kth_only;
+  // Partition mode: every CTA waits for epoch 0's bound after its first tile.  On a small
+  // copy the few tiles it could scan meanwhile are most of what the stop rule would skip
+  // (2^20 rows in 129 partitions: 66 % of them scanned without, 54 % with the wait).
+  uint32_t epoch_hold;
   uint32_t *slot_count; // entries per slot
   uint32_t *done;       // per-group arrival counters (zero between queries)
-  uint64_t *out_ids;    // min(k, rows) ids, ascending by score (null with out_scores: none written)
+  uint64_t *out_ids;    // min(k, rows) ids, ascending by score
   float *out_scores;
   float *out_threshold; // may be null
   uint32_t *out_count;  // may be null
-  uint32_t *out_kth_key; // may be null: the k-th entry's key when k entries were found, else 0
   uint32_t *out_stats;  // may be null: [0] entries merged at the root, [1] block-selects,
                         // [2] tiles scanned (partition mode)
   // Partition mode (part_list != null): tile t covers rows
@@ -153,49 +151,47 @@ struct ScanParams {
 };
 
 // Publishing (ScanParams::pub): grids of at least kPubMinGrid CTAs; the arrays need
-// grid * kPubMaxEntries entries and grid * kPubMaxKeys keys per epoch.
+// grid * kPubMaxEntries entries and grid * kPubMaxKeys entries per epoch.
 constexpr uint32_t kPubMinGrid = 2;
 // Polls of the two waits, about 1 us and 0.25 us apart (a decision wait hides behind the
 // answering CTA's last microseconds; waiting longer for epoch 0 costs more than a select).
 constexpr uint32_t kPubWaitPolls = 256, kPubWaitNs = 1000;
 constexpr uint32_t kEpochWaitPolls = 64, kEpochWaitNs = 250;
-constexpr uint32_t kPubMaxPerWarp = 4;
-constexpr uint32_t kPubMaxKeys = 8 * kPubMaxPerWarp;  // of an epoch
-constexpr uint32_t kPubMaxEntries = 96;               // at the end
+constexpr uint32_t kPubMaxKeys = 32;     // of an epoch: 4 per warp
+constexpr uint32_t kPubMaxEntries = 96;  // at the end (the list and 32 words in 1 KB)
 // Entries a CTA that holds more than kPubMaxEntries aims to publish.  With the k best
-// spread over the CTAs it holds lambda = k / grid of them; lambda + 3 sqrt(lambda) + 2
-// leaves one out in under 1-2 % of queries (then the merge tree answers).  0: no
-// publishing, too few CTAs for k entries.
-inline uint32_t pub_entries(uint32_t k, uint32_t grid) {
+// spread over the CTAs it holds lambda = k / grid of them; lambda + 3 sqrt(lambda) + 1.6
+// leaves one out in under 1-3 % of queries (then the merge tree answers).  In a scan with
+// epochs it holds that many only when much of the result is in it, and publishes about as
+// many as it can bound (24 of the 32 best of its threads).  Where lambda is too large for
+// that, grids of at least 16 CTAs publish 28 each, whose k-th bounds what the tree carries
+// (40,000 rows, k = 1000: 63 us a query against 104 without); below, or with too few CTAs
+// for k entries, publishing is in vain (14 us of 57) and the tree answers alone: 0.
+inline uint32_t pub_entries(uint32_t k, uint32_t grid, uint32_t epochs) {
   if (grid < kPubMinGrid || (uint64_t)grid * kPubMaxEntries < k) return 0;
+  if (epochs) return 24;
   const double l = (double)k / grid;
-  const uint32_t r = (uint32_t)__builtin_ceil(l + 3.0 * __builtin_sqrt(l) + 2.0);
-  return r < 24u ? r : 24u;
+  const uint32_t r = (uint32_t)__builtin_ceil(l + 3.0 * __builtin_sqrt(l) + 1.6);
+  if (r <= 24) return r;
+  return grid >= 16 && 28.0 * grid >= 1.2 * k ? 28 : 0;
 }
 // Epochs of a scan over `tiles` tiles, after 1, m, m^2, ... tiles (m = 2^shift): each ends
-// before the scan does, with every CTA still taking part; none when no CTA has a third
-// tile (its buffer holds two without a select).
+// before the scan does, with every CTA still taking part.
 inline uint32_t scan_epochs(uint64_t tiles, uint32_t grid, uint32_t shift) {
   uint32_t e = 0;
-  if ((tiles + grid - 1) / grid >= 3)
-    for (uint64_t at = 1; at * grid < tiles && e < kMaxEpochs; at <<= shift) ++e;
+  for (uint64_t at = 1; at * grid < tiles && e < kMaxEpochs; at <<= shift) ++e;
   return e;
 }
-// Keys a CTA publishes per epoch: its largest while that is at least 4k keys in all, else
-// 1, 2 or 4 per warp (at least 2k in all, when the grid has them): the k-th largest of
-// them then lies close to the k-th largest key seen so far.
-inline uint32_t epoch_keys(uint32_t k, uint32_t grid) {
-  if ((uint64_t)grid >= 4ull * k) return 1;
-  uint32_t r = 1;
-  while (r < kPubMaxPerWarp && 8ull * r * grid < 2ull * k) r *= 2;
-  return 8 * r;
-}
-// Keys a threshold pass (kth_only) publishes per CTA: a multiple of its 8 warps, at
-// least ceil(k / grid) + 1, at most 8 * kPubMaxPerWarp.
-inline uint32_t pub_keys_per_cta(uint32_t k, uint32_t grid) {
-  const uint32_t want = (k + grid - 1) / grid + 1;
-  const uint32_t r = (want + 7) / 8;
-  return 8 * (r < kPubMaxPerWarp ? r : kPubMaxPerWarp);
+// Entries a CTA publishes per epoch, at least 3k / 2 in all: with k = 256 of 739 CTAs the
+// k-th best of every CTA's best lies at rank ~315 of all.  More would tighten the bound
+// a little and lengthen the coordinator's pass, which every CTA waits for in epoch 0
+// (8 per CTA at k = 256 cost 13 us a query on 2^24 rows).  In partition mode, where the
+// best objects sit close together and the bound decides how far the scan goes, 4k in all
+// and 4 per CTA at least.
+inline uint32_t epoch_keys(uint32_t k, uint32_t grid, bool part) {
+  const uint32_t want = part ? 4u * k : 3u * k / 2u, least = part ? 4u : 1u;
+  const uint32_t r = (want + grid - 1u) / grid;
+  return r < least ? least : r < kPubMaxKeys ? r : kPubMaxKeys;
 }
 
 struct ScanPlan {
