@@ -55,7 +55,8 @@ __device__ __forceinline__ uint32_t bq_attr(const BatchQuery *qs, uint32_t q, in
 // ---------------------------------------------------------------- bootstrap
 // One block per query: exact top-k of rows [0, rows).  Shared: entries[rows] and
 // best[k] (dynamic), histogram, select state, the query's attr/weights.
-__global__ void __launch_bounds__(kBT) batch_bootstrap_kernel(const float *__restrict__ table, uint64_t ld,
+constexpr int kBootThreads = 1024;  // 8 rows a thread; 256 threads took 46 us for 100 queries
+__global__ void __launch_bounds__(kBootThreads) batch_bootstrap_kernel(const float *__restrict__ table, uint64_t ld,
                                                               uint32_t rows, const BatchQuery *__restrict__ qs,
                                                               BatchState *__restrict__ st, uint2 *__restrict__ best) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -77,11 +78,11 @@ __global__ void __launch_bounds__(kBT) batch_bootstrap_kernel(const float *__res
   __syncthreads();
   const uint32_t qq = sh->qq, k = sh->k;
   uint2 *out = ent + rows;
-  for (uint32_t i = t; i < rows; i += kBT) ent[i] = make_uint2(f2key(score_row(table, ld, i, attr, w, qq)), i);
+  for (uint32_t i = t; i < rows; i += kBootThreads) ent[i] = make_uint2(f2key(score_row(table, ld, i, attr, w, qq)), i);
   __syncthreads();
-  const uint32_t kept = block_reduce<kBT>(ent, rows, out, k, 0u, hist, &sh->sel);
+  const uint32_t kept = block_reduce<kBootThreads>(ent, rows, out, k, 0u, hist, &sh->sel);
   uint2 *dst = best + q.best_off;
-  for (uint32_t j = t; j < kept; j += kBT) dst[j] = out[j];
+  for (uint32_t j = t; j < kept; j += kBootThreads) dst[j] = out[j];
   if (t == 0) {
     BatchState s{};
     s.cnt = kept;
@@ -401,7 +402,7 @@ cudaError_t launch_batch_bootstrap(const float *table, uint64_t ld, uint32_t row
   const size_t smem = batch_bootstrap_smem(rows, kmax);
   cudaError_t e = cudaFuncSetAttribute(batch_bootstrap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  batch_bootstrap_kernel<<<nq, kBT, smem, s>>>(table, ld, rows, qs, st, best);
+  batch_bootstrap_kernel<<<nq, kBootThreads, smem, s>>>(table, ld, rows, qs, st, best);
   return cudaGetLastError();
 }
 

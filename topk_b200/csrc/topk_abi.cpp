@@ -511,8 +511,8 @@ constexpr uint32_t kPrunedCtasPerSm = 4;
 //      and each CTA stops at its first partition whose bound is below its running
 //      threshold -- the reference's stop rule per block (cpu/VTA.h:210-216,
 //      cpu/PTA.h:636-641).  (A launch of its own for a first threshold, over the best
-//      1/32 of the partitions, read those twice: over 96 random queries on 2^27 x 8 in kd order 4 attributes took 89 us a
-//      query at k = 128 and 205 with 8, now 66 and 158.)
+//      1/32 of the partitions, read those twice: random queries on 2^27 x 8 in kd order
+//      took 89 us at q = 4, k = 128 and 205 at q = 8, now 66 and 158.)
 // With a seed (a predicted lower bound of the k-th score: `cut`, or the learned
 // model's cut computed on the device) the scan starts from it, and its result is
 // accepted when it holds min(k, n) objects (then the true k-th score is at least the
@@ -873,6 +873,14 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   }
   const uint64_t boot = std::min<uint64_t>(h->n, h->batch_boot);
   const uint64_t r_start = use_learned ? 0 : boot;
+  // Chunks double the rows seen; for a small batch they quadruple them: a chunk costs
+  // about 25 us of launches whatever it holds, and passes 3k candidates a query instead of
+  // 2k in two (from about 2^16 results on those cost more than the launches).  Beyond
+  // k = 1024 3k candidates would come close to what moves a query to the FP32 scorer.
+  // Boundaries stay multiples of 256 rows (the filter's object tiles).
+  const bool quadruple = best_total <= (1u << 16) && kmax <= 1024;
+  auto next_chunk = [&](uint64_t r, uint64_t size) { return quadruple ? 3 * r : 2 * size; };
+  const uint64_t first_chunk = quadruple && r_start ? 3 * r_start : h->batch_boot;
   // Hybrid batch under the filter: a query for which the filter passes too much
   // (scores tied or dense at its threshold) moves to the exact FP32 scorer for the
   // rest of the batch.  The reduce lists it: sw[0] counts the moved queries (list A at
@@ -907,8 +915,7 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
     CK(launch_batch_bootstrap(h->table, h->ld, (uint32_t)boot, kmax, dq, nqq, dst, dbest, s));
   }
   uint64_t prev_r = r_start;
-  // chunk boundaries stay multiples of 256 rows (the filter's object tiles)
-  for (uint64_t r = r_start, size = h->batch_boot; r < h->n; size *= 2) {
+  for (uint64_t r = r_start, size = first_chunk; r < h->n; size = next_chunk(r, size)) {
     const uint64_t e = std::min<uint64_t>(h->n, r + size);
     if (use_bf16) {
       const FilterPlan fp = plan_bf16_filter(nqq, r, e, h->num_sms, h->batch_qt);
@@ -953,7 +960,8 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   // margin makes a new shape).  The graph reads the query descriptors and states that
   // the stream uploaded and cleared before it.
   std::vector<uint64_t> key = {nq, kmax, capmax, qmax, use_bf16, use_learned, h->n, h->d, h->ld, boot,
-                               (uint64_t)h->num_sms, log_ctas, h->wait_limit, h->num_parts, h->batch_qt};
+                               (uint64_t)h->num_sms, log_ctas, h->wait_limit, h->num_parts, h->batch_qt,
+                               quadruple};
   const void *key_ptrs[] = {h->table, dq, dst, dbest, dcand, h->b_ids.p, h->b_scores.p, h->b_count.p,
                             h->b_thr.p, h->xbf.p, h->b_abf.p, h->b_log.p, h->b_logh.p, h->b_err.p, h->b_sw.p,
                             h->b_feat.p, h->b_pred.p, h->pstats, h->mlp, h->b_abf_act.p, h->b_amap.p, dorder};
@@ -1028,7 +1036,7 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   double filter_flops = 0;
   if (use_bf16) {
     uint32_t c = 0;  // the chunks as issued (the graph replays the same sequence)
-    for (uint64_t r = r_start, size = h->batch_boot; r < h->n && c < kMaxChunkLog; size *= 2, ++c) {
+    for (uint64_t r = r_start, size = first_chunk; r < h->n && c < kMaxChunkLog; size = next_chunk(r, size), ++c) {
       const uint64_t e = std::min<uint64_t>(h->n, r + size);
       filter_flops += (double)((hact[c] + 127) / 128 * 128) * (double)((e - r + 255) / 256 * 256) * 96.0;
       r = e;

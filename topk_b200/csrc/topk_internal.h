@@ -173,7 +173,7 @@ inline uint32_t pub_entries(uint32_t k, uint32_t grid, uint32_t epochs) {
   const double l = (double)k / grid;
   const uint32_t r = (uint32_t)__builtin_ceil(l + 3.0 * __builtin_sqrt(l) + 1.6);
   if (r <= 24) return r;
-  return grid >= 16 && 28.0 * grid >= 1.2 * k ? 28 : 0;
+  return grid >= 16 && 28u * grid >= k ? 28 : 0;
 }
 // Epochs of a scan over `tiles` tiles, after 1, m, m^2, ... tiles (m = 2^shift): each ends
 // before the scan does, with every CTA still taking part.
