@@ -415,8 +415,10 @@ int topk_set_fault_injection(topk_table_t h, int mode);
 #define TOPK_BATCH_FP32 2  /* batched plain FP32: each table tile scored for 64 queries */
 #define TOPK_BATCH_BF16 3  /* BF16 tensor-core filter (tcgen05) with a per-query error
                             * bound; candidates rescored exactly in FP32.  Applies to
-                            * d <= 16 with finite table values and weights of magnitude
-                            * <= 2^60; other batches run TOPK_BATCH_FP32.  Hybrid: a
+                            * d <= 16, and from 2^17 rows on to d <= 64 (where the split
+                            * copy takes at most half of the free memory), with finite
+                            * table values and weights of magnitude <= 2^60; other
+                            * batches run TOPK_BATCH_FP32.  Hybrid: a
                             * query for which the filter passes too much (tied or dense
                             * scores at its threshold: more than 2k + 2048 candidates in
                             * a chunk, or lost ones) moves to the exact FP32 scorer for

@@ -10,7 +10,9 @@ constexpr uint32_t kBatchMaxQ = 32;    // attributes per query on the batched pa
 constexpr uint32_t kBatchMaxD = 64;    // table width the FP32 scorer stages
 constexpr uint32_t kBatchBootRows = 8192;  // rows of the exact bootstrap (default)
 constexpr uint32_t kBatchBootMax = 16384;  // its shared-memory limit
-constexpr uint32_t kBf16MaxD = 16;         // table width of the BF16 tensor-core filter (MMA K)
+constexpr uint32_t kBf16K = 16;            // attributes of one MMA (K) of the BF16 tensor-core filter
+constexpr uint32_t kBf16MaxD = 64;         // table width of the filter: four K blocks
+inline uint32_t bf16_kblocks(uint32_t d) { return (d + kBf16K - 1) / kBf16K; }
 constexpr uint32_t kBf16LogCap = 32768;    // survivor records (32 values + header, 136 B) per filter CTA
 
 // Per-query descriptor (device, read-only during a batch).
@@ -66,24 +68,27 @@ cudaError_t launch_batch_reduce(const float *table, uint64_t ld, const BatchQuer
                                 uint2 *best, const uint2 *cand, uint32_t kmax, uint32_t capmax, bool rescore,
                                 uint32_t *sw, cudaStream_t s);
 // BF16 tensor-core filter (bf16_filter.cu).
-uint64_t bf16_table_bytes(uint64_t n);
+uint64_t bf16_table_bytes(uint64_t n, uint32_t d);
 // Also the column extremes: ext[m] = largest |x| bits, ext[d + m] = largest order key,
 // ext[2d + m] = smallest order key (NaN left out) of column m.
 cudaError_t launch_bf16_pack(const float *table, uint64_t ld, uint32_t d, uint64_t n, uint8_t *xbf, uint32_t *ext,
                              int num_sms, cudaStream_t s);
-size_t bf16_query_bytes(uint32_t nq);
-// Host: write query j's 16-wide row a[] (hi and lo) into the tiled query buffer.
-void bf16_pack_query(const float *a, uint32_t j, uint8_t *abf);
+size_t bf16_query_bytes(uint32_t nq, uint32_t d);
+// Host: write query j's row a[] (16 * bf16_kblocks(d) wide; hi and lo) into the tiled
+// query buffer.
+void bf16_pack_query(const float *a, uint32_t d, uint32_t j, uint8_t *abf);
 // One filter launch over rows [r0, r1): its object tiles, the most query tiles of 128
 // one CTA takes (qt_cap) and the grid (the work split itself is made on the device
 // from the active count, see launch_bf16_filter).
 struct FilterPlan {
   uint64_t tile0, tile1;
+  uint32_t kblk;  // K blocks of 16 attributes
   uint32_t qt_cap;
   uint64_t grid;
 };
 // nq: queries of the batch (the most that can be active); qt_cap 0: the kernel's maximum
-FilterPlan plan_bf16_filter(uint32_t nq, uint64_t r0, uint64_t r1, int num_sms, uint32_t qt_cap = 0);
+// for the table's width
+FilterPlan plan_bf16_filter(uint32_t nq, uint64_t r0, uint64_t r1, uint32_t d, int num_sms, uint32_t qt_cap = 0);
 // r0 must be a multiple of 256.  The filter serves the *nact active queries in the
 // compact tiles abf (slot -> query: amap); recv/rech hold grid * rec_cap records.
 cudaError_t launch_bf16_filter(const FilterPlan &f, const uint8_t *xbf, const uint8_t *abf, const uint32_t *amap,
@@ -94,8 +99,8 @@ cudaError_t launch_bf16_filter(const FilterPlan &f, const uint8_t *xbf, const ui
 // scorer nor retired by BatchQuery::maxkey), their rows of abf copied into compact
 // tiles abf_act (same size as abf), amap[slot] = query, *nact = count (and, when
 // nact_log is not null, *nact_log = count: the chunk's entry of a per-batch record).
-cudaError_t launch_batch_active(const BatchQuery *qs, const BatchState *st, uint32_t nq, const uint8_t *abf,
-                                uint8_t *abf_act, uint32_t *amap, uint32_t *nact, uint32_t *nact_log,
+cudaError_t launch_batch_active(const BatchQuery *qs, const BatchState *st, uint32_t nq, uint32_t d,
+                                const uint8_t *abf, uint8_t *abf_act, uint32_t *amap, uint32_t *nact, uint32_t *nact_log,
                                 cudaStream_t s);
 // Learned k-th-score model (mlp.cu): in -> 64 -> 64 -> 1 ReLU MLP, features of
 // feature_dim(d) values per query from the partition statistics ([P][d] each).

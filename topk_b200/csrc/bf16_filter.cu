@@ -9,19 +9,21 @@
 //
 // Operands, both K-major without swizzle (core matrices of 8 rows x 16 bytes; the
 // K-adjacent core matrix 128 B further on, the next 8 rows 256 B further on):
-//   query  a 16-wide row a[m] = sum of weights[attr[j]] over the j with attr[j] = m,
-//          split a = hi + lo (bf16 each, |a - hi - lo| <= 2^-16 |a|); tiles of 128
-//          queries: hi 4 KB, then lo 4 KB                          (MMA A, M=128);
-//   table  each object's 16 attributes split the same way; tiles of 256 objects:
-//          hi 8 KB, then lo 8 KB                                    (MMA B, N=256).
-// One (object tile, query tile) pair is three MMAs M=128 N=256 K=16 into FP32 TMEM
-// (lane = query, column = object):
+//   query  a row a[m] = sum of weights[attr[j]] over the j with attr[j] = m, padded to
+//          whole K blocks of 16 attributes (1 to 4 of them, d <= 64), split a = hi + lo
+//          (bf16 each, |a - hi - lo| <= 2^-16 |a|); tiles of 128 queries: per K block hi
+//          4 KB, then lo 4 KB                                       (MMA A, M=128);
+//   table  each object's attributes split the same way; tiles of 256 objects: per K
+//          block hi 8 KB, then lo 8 KB                              (MMA B, N=256).
+// One (object tile, query tile) pair is three MMAs M=128 N=256 K=16 per K block into FP32
+// TMEM (lane = query, column = object):
 //   D = Ahi.Xhi + Ahi.Xlo + Alo.Xhi        (the lo.lo term lies inside the bound)
 // Bound (host-computed per query, BatchQuery::err): |D - s_ref| <= E with
 //   E = 2^-13 * sum_m |weights[attr[m]]| * max|column attr[m]|  (+ 2^-100 terms for
-//   subnormal flushing).  Split and product errors give 3.1*2^-16, 48 FP32
-//   accumulations 48*2^-22, the reference's own FP32 rounding 17*2^-24: about
-//   2^-14 in all; the factor 2 covers the tensor core's accumulation rounding,
+//   subnormal flushing; 2^-12 with more than one K block).  Split and product errors
+//   give 3.1*2^-16, 48 FP32 accumulations per K block 48*2^-22 each, the reference's own
+//   FP32 rounding 33*2^-24: about 2^-14 in all (2^-13.3 with four K blocks); the factor 2
+//   covers the tensor core's accumulation rounding,
 //   which is not specified (the largest error measured on rescored candidates is
 //   below 2^-16 of the same sum).  An object with exact score >= the threshold
 //   float t has D >= t - E, so the cut t - E (rounded down) loses none.
@@ -63,15 +65,20 @@ namespace topk {
 namespace {
 
 constexpr uint32_t kOTile = 256;         // objects per tile (MMA N, TMEM columns)
-constexpr uint32_t kOTileBytes = 16384;  // hi + lo of one object tile
+constexpr uint32_t kOTileBytes = 16384;  // hi + lo of one K block of an object tile
 constexpr uint32_t kQTile = 128;         // queries per tile (MMA M, TMEM lanes)
-constexpr uint32_t kQTileBytes = 8192;   // hi + lo of one query tile
-constexpr uint32_t kStages = 5;
+constexpr uint32_t kQTileBytes = 8192;   // hi + lo of one K block of a query tile
+constexpr uint32_t kStages = 5;          // object ring, one K block
+// Object ring stages and query tiles of a CTA by K blocks: what 227 KB of shared memory
+// hold (ring + query tiles + cuts, filter_smem_bytes).  Wider rows also take longer to
+// multiply, so fewer stages hide the copies.
+__host__ __device__ constexpr uint32_t filter_stages(uint32_t kblk) { return kblk == 1 ? kStages : kblk == 2 ? 3u : 2u; }
 constexpr uint32_t kEpiWarps = 16;
 constexpr uint32_t kProducerWarp = kEpiWarps, kMmaWarp = kEpiWarps + 1;
 constexpr uint32_t kFThreads = (kEpiWarps + 2) * 32;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kMaxQTPerCta = 16;
+constexpr uint32_t filter_max_qt(uint32_t kblk) { return kblk == 1 ? kMaxQTPerCta : kblk == 2 ? 7u : kblk == 3 ? 5u : 3u; }
 constexpr uint32_t kAcc = kTmemCols / kOTile;            // TMEM accumulators in flight
 // Epilogue groups: group g drains the pairs seq = g mod kDrainGroups, so with two
 // groups each accumulator has its own eight warps (4 round trips of 32 columns each).
@@ -172,6 +179,9 @@ struct FilterArgs {
   uint32_t *err;
 };
 
+// KB: K blocks (compile-time: the one issuing thread sets the pace of a pair; read from the
+// arguments, the count cost 5 % on 16 attributes).
+template <uint32_t KB>
 __global__ void __launch_bounds__(kFThreads, 1) bf16_filter_kernel(const FilterArgs p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   // Work split from the active query count: the chunk's active queries in tiles of
@@ -196,9 +206,10 @@ __global__ void __launch_bounds__(kFThreads, 1) bf16_filter_kernel(const FilterA
   if (tb >= te) return;
 
   // shared layout: query tiles | object ring | cut[QT*kQTile] | barriers and words
+  constexpr uint32_t stages = filter_stages(KB), otile = KB * kOTileBytes, qtile = KB * kQTileBytes;
   unsigned char *sq = smem;
-  unsigned char *so = smem + (size_t)p.qt_cap * kQTileBytes;
-  float *scut = reinterpret_cast<float *>(so + (size_t)kStages * kOTileBytes);
+  unsigned char *so = smem + (size_t)p.qt_cap * qtile;
+  float *scut = reinterpret_cast<float *>(so + (size_t)stages * otile);
   uint64_t *bars = reinterpret_cast<uint64_t *>(scut + p.qt_cap * kQTile);
   uint64_t *full = bars, *empty = bars + kStages, *accf = bars + 2 * kStages, *acce = accf + kAcc;
   uint64_t *qfull = acce + kAcc, *mdone = qfull + 1;
@@ -256,20 +267,20 @@ __global__ void __launch_bounds__(kFThreads, 1) bf16_filter_kernel(const FilterA
   if (warp == kProducerWarp) {
     // ---------------------------------------------------------------- producer
     if (lane == 0) {
-      mbar_arrive_expect_tx(qfull, nqt * kQTileBytes);
+      mbar_arrive_expect_tx(qfull, nqt * qtile);
       for (uint32_t i = 0; i < nqt; ++i)
-        bulk_g2s(sq + (size_t)i * kQTileBytes, p.abf + (size_t)(qt0 + i) * kQTileBytes, kQTileBytes, qfull);
+        bulk_g2s(sq + (size_t)i * qtile, p.abf + (size_t)(qt0 + i) * qtile, qtile, qfull);
       uint64_t it = 0;
       for (uint64_t t = tb; t < te; ++t, ++it) {
-        const uint32_t s = (uint32_t)(it % kStages);
-        if (it >= kStages && !fwait(empty + s, (uint32_t)((it / kStages - 1) & 1), limit, abort_flag)) break;
-        mbar_arrive_expect_tx(full + s, kOTileBytes);
-        bulk_g2s(so + (size_t)s * kOTileBytes, p.xbf + t * kOTileBytes, kOTileBytes, full + s);
+        const uint32_t s = (uint32_t)(it % stages);
+        if (it >= stages && !fwait(empty + s, (uint32_t)((it / stages - 1) & 1), limit, abort_flag)) break;
+        mbar_arrive_expect_tx(full + s, otile);
+        bulk_g2s(so + (size_t)s * otile, p.xbf + t * otile, otile, full + s);
       }
       // the CTA must not exit with copies in flight: wait for the last use of each stage
-      const uint64_t first = it > kStages ? it - kStages : 0;
+      const uint64_t first = it > stages ? it - stages : 0;
       for (uint64_t j = first; j < it; ++j)
-        if (!mbar_wait_bounded(full + (j % kStages), (uint32_t)((j / kStages) & 1), limit)) *abort_flag = 1u;
+        if (!mbar_wait_bounded(full + (j % stages), (uint32_t)((j / stages) & 1), limit)) *abort_flag = 1u;
       if (!mbar_wait_bounded(qfull, 0, limit)) *abort_flag = 1u;
     }
   } else if (warp == kMmaWarp) {
@@ -279,11 +290,10 @@ __global__ void __launch_bounds__(kFThreads, 1) bf16_filter_kernel(const FilterA
       uint64_t it = 0;
       uint32_t seq = 0;
       for (uint64_t t = tb; ok && t < te; ++t, ++it) {
-        const uint32_t s = (uint32_t)(it % kStages);
-        if (!fwait(full + s, (uint32_t)((it / kStages) & 1), limit, abort_flag)) break;
+        const uint32_t s = (uint32_t)(it % stages);
+        if (!fwait(full + s, (uint32_t)((it / stages) & 1), limit, abort_flag)) break;
         tc_fence_after();
-        const uint32_t os = smem_u32(so + (size_t)s * kOTileBytes);
-        const uint64_t xhi = smem_desc(os), xlo = smem_desc(os + kOTileBytes / 2);
+        const uint32_t os = smem_u32(so + (size_t)s * otile);
         for (uint32_t i = 0; i < nqt; ++i, ++seq) {
           const uint32_t buf = seq % kAcc;
           if (seq >= kAcc && !fwait(acce + buf, (seq / kAcc - 1) & 1u, limit, abort_flag)) {
@@ -291,12 +301,16 @@ __global__ void __launch_bounds__(kFThreads, 1) bf16_filter_kernel(const FilterA
             break;
           }
           tc_fence_after();
-          const uint32_t qsa = smem_u32(sq + (size_t)i * kQTileBytes);
-          const uint64_t ahi = smem_desc(qsa), alo = smem_desc(qsa + kQTileBytes / 2);
+          const uint32_t qsa = smem_u32(sq + (size_t)i * qtile);
           const uint32_t d = tmem + buf * kOTile;
-          tc_mma(d, ahi, xhi, 0u);
-          tc_mma(d, ahi, xlo, 1u);
-          tc_mma(d, alo, xhi, 1u);
+#pragma unroll
+          for (uint32_t kb = 0; kb < KB; ++kb) {
+            const uint64_t xhi = smem_desc(os + kb * kOTileBytes), xlo = smem_desc(os + kb * kOTileBytes + kOTileBytes / 2);
+            const uint64_t ahi = smem_desc(qsa + kb * kQTileBytes), alo = smem_desc(qsa + kb * kQTileBytes + kQTileBytes / 2);
+            tc_mma(d, ahi, xhi, kb ? 1u : 0u);
+            tc_mma(d, ahi, xlo, 1u);
+            tc_mma(d, alo, xhi, 1u);
+          }
           tc_commit(accf + buf);
         }
         if (!ok) break;
@@ -425,14 +439,16 @@ __global__ void __launch_bounds__(kFThreads, 1) bf16_filter_kernel(const FilterA
 }
 
 // ---------------------------------------------------------------- table split
-// One thread per object (grid-stride): reads its 16 attributes (columns >= d and
-// rows >= n are zero), writes hi and lo in the tiled core-matrix layout, and keeps
+// One thread per object (grid-stride) and K block (blockIdx.y): reads its 16 attributes
+// (columns >= d and rows >= n are zero), writes hi and lo in the tiled core-matrix layout,
+// and keeps
 // per column the largest |x| bit pattern (NaN and inf show as >= 0x7F800000) and the
 // largest and smallest order keys (NaN left out of both).
 __global__ void __launch_bounds__(256) bf16_pack_kernel(const float *__restrict__ table, uint64_t ld, uint32_t d,
                                                         uint64_t n, uint64_t nobj, uint8_t *__restrict__ xbf,
                                                         uint32_t *__restrict__ ext) {
   uint32_t amax[16], kmax[16], kmin[16];
+  const uint32_t m0 = blockIdx.y * kBf16K;
 #pragma unroll
   for (int m = 0; m < 16; ++m) {
     amax[m] = 0u;
@@ -446,8 +462,8 @@ __global__ void __launch_bounds__(256) bf16_pack_kernel(const float *__restrict_
       float x[2];
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const bool in = (uint32_t)(m + e) < d && o < n;
-        x[e] = in ? __ldg(table + (uint64_t)(m + e) * ld + o) : 0.0f;
+        const bool in = m0 + (uint32_t)(m + e) < d && o < n;
+        x[e] = in ? __ldg(table + (uint64_t)(m0 + m + e) * ld + o) : 0.0f;
         amax[m + e] = max(amax[m + e], __float_as_uint(x[e]) & 0x7FFFFFFFu);
         if (in && x[e] == x[e]) {
           const uint32_t k = f2key(x[e]);
@@ -463,7 +479,7 @@ __global__ void __launch_bounds__(256) bf16_pack_kernel(const float *__restrict_
     }
     const uint64_t t = o / kOTile;
     const uint32_t r = (uint32_t)(o % kOTile);
-    uint8_t *base = xbf + t * kOTileBytes + (r >> 3) * 256u + (r & 7u) * 16u;
+    uint8_t *base = xbf + (t * gridDim.y + blockIdx.y) * kOTileBytes + (r >> 3) * 256u + (r & 7u) * 16u;
     *reinterpret_cast<uint4 *>(base) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     *reinterpret_cast<uint4 *>(base + 128) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
     *reinterpret_cast<uint4 *>(base + kOTileBytes / 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
@@ -485,7 +501,7 @@ __global__ void __launch_bounds__(256) bf16_pack_kernel(const float *__restrict_
     }
   }
   __syncthreads();
-  const uint32_t m = threadIdx.x & 15u;
+  const uint32_t m = m0 + (threadIdx.x & 15u);
   if (threadIdx.x < 48 && m < d) {
     if (threadIdx.x < 32) atomicMax(ext + (threadIdx.x < 16 ? 0u : d) + m, bext[threadIdx.x]);
     else atomicMin(ext + 2 * d + m, bext[threadIdx.x]);
@@ -495,7 +511,7 @@ __global__ void __launch_bounds__(256) bf16_pack_kernel(const float *__restrict_
 // ---------------------------------------------------------------- active queries
 // One block, before each chunk's filter: lists the queries the filter still has to
 // serve, in query order, as compact slots (amap[slot] = query, *nact = count), and
-// copies each one's operand row (hi and lo, 64 bytes) from the batch's query tiles to
+// copies each one's operand row (hi and lo, 64 bytes a K block) from the batch's query tiles to
 // its slot in the compact tiles.  A query is left out once it has moved to the exact
 // FP32 scorer, or once its threshold is above the largest score any row can have
 // (BatchQuery::maxkey: the reference-order FP32 sum over the column extremes, an
@@ -505,13 +521,14 @@ __global__ void __launch_bounds__(256) bf16_pack_kernel(const float *__restrict_
 // the block.  The rows of the last tile past the count are zeroed.
 constexpr uint32_t kActThreads = 1024;
 
-__device__ __forceinline__ size_t qrow_off(uint32_t j) {  // query j's hi row in the tile layout
-  return (size_t)(j / kQTile) * kQTileBytes + ((j % kQTile) >> 3) * 256u + (j & 7u) * 16u;
+// Query j's hi row in the tile layout, first K block (the next ones kQTileBytes on).
+__device__ __forceinline__ size_t qrow_off(uint32_t j, uint32_t kblk) {
+  return (size_t)(j / kQTile) * kblk * kQTileBytes + ((j % kQTile) >> 3) * 256u + (j & 7u) * 16u;
 }
 
 __global__ void __launch_bounds__(kActThreads) batch_active_kernel(const BatchQuery *__restrict__ qs,
                                                                  const BatchState *__restrict__ st, uint32_t nq,
-                                                                 const uint8_t *__restrict__ abf,
+                                                                 uint32_t kblk, const uint8_t *__restrict__ abf,
                                                                  uint8_t *__restrict__ abf_act,
                                                                  uint32_t *__restrict__ amap,
                                                                  uint32_t *__restrict__ nact,
@@ -545,12 +562,14 @@ __global__ void __launch_bounds__(kActThreads) batch_active_kernel(const BatchQu
     const uint32_t slot = base + wsum[warp] + __popc(b & ((1u << lane) - 1u));
     if (act) {
       amap[slot] = j;
-      const uint4 *src = reinterpret_cast<const uint4 *>(abf + qrow_off(j));
-      uint4 *dst = reinterpret_cast<uint4 *>(abf_act + qrow_off(slot));
-      dst[0] = src[0];                      // hi, attributes 0-7
-      dst[8] = src[8];                      // hi, attributes 8-15 (128 bytes on)
-      dst[kQTileBytes / 32] = src[kQTileBytes / 32];          // lo
-      dst[kQTileBytes / 32 + 8] = src[kQTileBytes / 32 + 8];
+      for (uint32_t kb = 0; kb < kblk; ++kb) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(abf + qrow_off(j, kblk) + (size_t)kb * kQTileBytes);
+        uint4 *dst = reinterpret_cast<uint4 *>(abf_act + qrow_off(slot, kblk) + (size_t)kb * kQTileBytes);
+        dst[0] = src[0];                      // hi, attributes 0-7 of the K block
+        dst[8] = src[8];                      // hi, attributes 8-15 (128 bytes on)
+        dst[kQTileBytes / 32] = src[kQTileBytes / 32];          // lo
+        dst[kQTileBytes / 32 + 8] = src[kQTileBytes / 32 + 8];
+      }
     }
     __syncthreads();
     if (t == kActThreads - 1) base = slot + (act ? 1u : 0u);
@@ -558,12 +577,14 @@ __global__ void __launch_bounds__(kActThreads) batch_active_kernel(const BatchQu
   }
   const uint32_t total = base;
   for (uint32_t sl = total + t; sl < (total + kQTile - 1) / kQTile * kQTile; sl += kActThreads) {
-    uint4 *dst = reinterpret_cast<uint4 *>(abf_act + qrow_off(sl));
     const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-    dst[0] = z;
-    dst[8] = z;
-    dst[kQTileBytes / 32] = z;
-    dst[kQTileBytes / 32 + 8] = z;
+    for (uint32_t kb = 0; kb < kblk; ++kb) {
+      uint4 *dst = reinterpret_cast<uint4 *>(abf_act + qrow_off(sl, kblk) + (size_t)kb * kQTileBytes);
+      dst[0] = z;
+      dst[8] = z;
+      dst[kQTileBytes / 32] = z;
+      dst[kQTileBytes / 32 + 8] = z;
+    }
   }
   if (t == 0) {
     *nact = total;
@@ -575,11 +596,14 @@ __global__ void __launch_bounds__(kActThreads) batch_active_kernel(const BatchQu
 
 // ---------------------------------------------------------------- launchers
 // query tiles | object ring | cuts | barriers and words
-size_t filter_smem_bytes(uint32_t qt) {
-  return (size_t)qt * (kQTileBytes + kQTile * 4) + (size_t)kStages * kOTileBytes + 512;
+constexpr size_t filter_smem_bytes(uint32_t qt, uint32_t kblk) {
+  return (size_t)qt * (kblk * kQTileBytes + kQTile * 4) + (size_t)filter_stages(kblk) * kblk * kOTileBytes + 512;
 }
+static_assert(filter_smem_bytes(filter_max_qt(1), 1) <= 232448 && filter_smem_bytes(filter_max_qt(2), 2) <= 232448 &&
+                  filter_smem_bytes(filter_max_qt(3), 3) <= 232448 && filter_smem_bytes(filter_max_qt(4), 4) <= 232448,
+              "227 KB of shared memory");
 
-uint64_t bf16_table_bytes(uint64_t n) { return (n + kOTile - 1) / kOTile * kOTileBytes; }
+uint64_t bf16_table_bytes(uint64_t n, uint32_t d) { return (n + kOTile - 1) / kOTile * kOTileBytes * bf16_kblocks(d); }
 
 cudaError_t launch_bf16_pack(const float *table, uint64_t ld, uint32_t d, uint64_t n, uint8_t *xbf, uint32_t *ext,
                              int num_sms, cudaStream_t s) {
@@ -589,13 +613,15 @@ cudaError_t launch_bf16_pack(const float *table, uint64_t ld, uint32_t d, uint64
   if (e != cudaSuccess) return e;
   const uint64_t nobj = (n + kOTile - 1) / kOTile * kOTile;
   const uint64_t blocks = std::min<uint64_t>((nobj + 255) / 256, (uint64_t)num_sms * 8);
-  bf16_pack_kernel<<<(unsigned)blocks, 256, 0, s>>>(table, ld, d, n, nobj, xbf, ext);
+  bf16_pack_kernel<<<dim3((unsigned)blocks, bf16_kblocks(d)), 256, 0, s>>>(table, ld, d, n, nobj, xbf, ext);
   return cudaGetLastError();
 }
 
-size_t bf16_query_bytes(uint32_t nq) { return (size_t)((nq + kQTile - 1) / kQTile) * kQTileBytes; }
+size_t bf16_query_bytes(uint32_t nq, uint32_t d) {
+  return (size_t)((nq + kQTile - 1) / kQTile) * kQTileBytes * bf16_kblocks(d);
+}
 
-void bf16_pack_query(const float *a, uint32_t j, uint8_t *abf) {
+void bf16_pack_query(const float *a, uint32_t d, uint32_t j, uint8_t *abf) {
   auto f2bf = [](float f) -> uint16_t {  // round to nearest even (finite inputs)
     uint32_t u;
     __builtin_memcpy(&u, &f, 4);
@@ -608,24 +634,25 @@ void bf16_pack_query(const float *a, uint32_t j, uint8_t *abf) {
     __builtin_memcpy(&f, &u, 4);
     return f;
   };
-  const uint32_t tile = j / kQTile, r = j % kQTile;
-  uint8_t *base = abf + (size_t)tile * kQTileBytes + (r >> 3) * 256u + (r & 7u) * 16u;
-  for (uint32_t m = 0; m < kBf16MaxD; ++m) {
+  const uint32_t tile = j / kQTile, r = j % kQTile, kblk = bf16_kblocks(d);
+  uint8_t *base = abf + (size_t)tile * kblk * kQTileBytes + (r >> 3) * 256u + (r & 7u) * 16u;
+  for (uint32_t m = 0; m < kblk * kBf16K; ++m) {
     const uint16_t h = f2bf(a[m]);
     const volatile float res = a[m] - bf2f(h);  // exact: hi is within a factor 2 of a[m]
     const uint16_t l = f2bf(res);
-    const size_t off = (m >> 3) * 128u + (m & 7u) * 2u;
+    const size_t off = (size_t)(m / kBf16K) * kQTileBytes + ((m >> 3) & 1u) * 128u + (m & 7u) * 2u;
     __builtin_memcpy(base + off, &h, 2);
     __builtin_memcpy(base + kQTileBytes / 2 + off, &l, 2);
   }
 }
 
-FilterPlan plan_bf16_filter(uint32_t nq, uint64_t r0, uint64_t r1, int num_sms, uint32_t qt_cap) {
+FilterPlan plan_bf16_filter(uint32_t nq, uint64_t r0, uint64_t r1, uint32_t d, int num_sms, uint32_t qt_cap) {
   FilterPlan f{};
+  f.kblk = bf16_kblocks(d);
   f.tile0 = r0 / kOTile;
   f.tile1 = (r1 + kOTile - 1) / kOTile;
   const uint32_t nqt = (nq + kQTile - 1) / kQTile;
-  f.qt_cap = (qt_cap >= 1 && qt_cap < kMaxQTPerCta) ? qt_cap : kMaxQTPerCta;
+  f.qt_cap = (qt_cap >= 1 && qt_cap < filter_max_qt(f.kblk)) ? qt_cap : filter_max_qt(f.kblk);
   // enough CTAs for every group the active count can need, and at least one per SM
   const uint64_t groups = (nqt + f.qt_cap - 1) / f.qt_cap;
   f.grid = std::max<uint64_t>((uint64_t)std::max(1, num_sms), groups);
@@ -654,17 +681,21 @@ cudaError_t launch_bf16_filter(const FilterPlan &f, const uint8_t *xbf, const ui
   p.r1 = r1;
   p.wait_limit = wait_limit;
   p.err = err;
-  const size_t smem = std::max(kMinFilterSmem, filter_smem_bytes(f.qt_cap));
-  cudaError_t e = cudaFuncSetAttribute(bf16_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = std::max(kMinFilterSmem, filter_smem_bytes(f.qt_cap, f.kblk));
+  if (f.kblk < 1 || f.kblk > 4) return cudaErrorInvalidValue;
+  static void (*const kernels[])(FilterArgs) = {bf16_filter_kernel<1>, bf16_filter_kernel<2>, bf16_filter_kernel<3>,
+                                                bf16_filter_kernel<4>};
+  const auto kernel = kernels[f.kblk - 1];
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  bf16_filter_kernel<<<(unsigned)f.grid, kFThreads, smem, s>>>(p);
+  kernel<<<(unsigned)f.grid, kFThreads, smem, s>>>(p);
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_active(const BatchQuery *qs, const BatchState *st, uint32_t nq, const uint8_t *abf,
-                                uint8_t *abf_act, uint32_t *amap, uint32_t *nact, uint32_t *nact_log,
+cudaError_t launch_batch_active(const BatchQuery *qs, const BatchState *st, uint32_t nq, uint32_t d,
+                                const uint8_t *abf, uint8_t *abf_act, uint32_t *amap, uint32_t *nact, uint32_t *nact_log,
                                 cudaStream_t s) {
-  batch_active_kernel<<<1, kActThreads, 0, s>>>(qs, st, nq, abf, abf_act, amap, nact, nact_log);
+  batch_active_kernel<<<1, kActThreads, 0, s>>>(qs, st, nq, bf16_kblocks(d), abf, abf_act, amap, nact, nact_log);
   return cudaGetLastError();
 }
 

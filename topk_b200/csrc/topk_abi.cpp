@@ -683,16 +683,25 @@ void table_changed(topk_table_t h) {
 constexpr float kBf16MaxAbs = 1.152921504606846976e18f;  // 2^60
 
 // Build (or reuse) the BF16 split of the table; caller holds batch_mu.  Sets
-// h->xbf_usable: false for tables wider than 16 or holding non-finite or huge values.
+// h->xbf_usable: false for tables wider than 64 or holding non-finite or huge values, and
+// for tables wider than 16 (which the FP32 scorer serves as well) when their split would
+// take more than half of the free memory.
 int ensure_bf16_table(topk_table_t h, cudaStream_t s) {
   if (h->xbf_version == h->data_version) return TOPK_OK;
   h->xbf_usable = false;
-  if (h->d > kBf16MaxD) {
+  const uint64_t bytes = bf16_table_bytes(h->n, h->d);
+  bool fits = h->d <= kBf16MaxD;
+  if (fits && h->d > kBf16K && h->xbf.bytes < bytes) {
+    size_t avail = 0, total = 0;
+    CK(cudaMemGetInfo(&avail, &total));
+    fits = bytes <= (avail + h->xbf.bytes) / 2;
+  }
+  if (!fits) {
     h->xbf_version = h->data_version;
     return TOPK_OK;
   }
   int st;
-  if ((st = ensure(h->xbf, bf16_table_bytes(h->n))) != TOPK_OK) return st;
+  if ((st = ensure(h->xbf, bytes)) != TOPK_OK) return st;
   if ((st = ensure(h->xbf_absmax, (size_t)h->d * 12)) != TOPK_OK) return st;
   CK(launch_bf16_pack(h->table, h->ld, h->d, h->n, static_cast<uint8_t *>(h->xbf.p),
                       static_cast<uint32_t *>(h->xbf_absmax.p), h->num_sms, s));
@@ -734,18 +743,26 @@ uint32_t score_bound_key(const BatchQuery &b, const std::vector<float> &cmax, co
 }
 
 // Per-query bound of the BF16 filter, rounded up to a float:
-// 2^-13 * sum_m |w_m| * absmax[attr_m] + 2^-100 * sum_m (|w_m| + absmax[attr_m]).
+// 2^-13 * sum_m |w_m| * absmax[attr_m] + 2^-100 * sum_m (|w_m| + absmax[attr_m]), with
+// 2^-12 for tables of more than one K block (bf16_filter.cu).
 // Summed in FP32: each sum of at most 32 nonnegative terms is within 33 * 2^-24 of
 // its exact value, so scaling by 1 + 2^-16 and rounding up keeps an upper bound.
-float bf16_error_bound(const BatchQuery &b, const std::vector<float> &absmax) {
+float bf16_error_bound(const BatchQuery &b, const std::vector<float> &absmax, uint32_t kblk) {
   float rel = 0.0f, tiny = 0.0f;
   for (uint32_t m = 0; m < b.qq; m++) {
     rel += std::fabs(b.w[m]) * absmax[b.attr[m]];
     tiny += std::fabs(b.w[m]) + absmax[b.attr[m]];
   }
-  const float e = std::ldexp(rel, -13) * (1.0f + 0x1p-16f) + std::ldexp(tiny, -100) * (1.0f + 0x1p-16f);
+  const float e = std::ldexp(rel, kblk > 1 ? -12 : -13) * (1.0f + 0x1p-16f) + std::ldexp(tiny, -100) * (1.0f + 0x1p-16f);
   return std::nextafter(e, INFINITY);
 }
+
+// Tables wider than one K block (16 attributes) take the filter from this many rows on:
+// below, its launches per chunk cost what the FP32 scorer does.  A batch of 300 queries on
+// 24 attributes, FP32 / filter in us: 20,000 rows 330 / 377, 70,000 409 / 425, 300,000 778
+// / 515, 2,000,003 2899 / 666; 20 queries on 64 attributes: 183 / 203, 231 / 254, 423 / 338,
+// 1359 / 479.
+constexpr uint64_t kWideFilterRows = 1u << 17;
 
 // Chunks of a batch whose served query counts are recorded (a 2^32-row table needs 20).
 constexpr uint32_t kMaxChunkLog = 64;
@@ -790,7 +807,9 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   cudaStream_t s = h->primary->stream;
   // scorer: the BF16 tensor-core filter where the table and every weight allow it
   bool use_bf16 = false;
-  if (!force_fp32 && (h->batch_method == TOPK_BATCH_AUTO || h->batch_method == TOPK_BATCH_BF16 ||
+  const uint32_t kblk = bf16_kblocks(h->d);
+  const bool small_wide = h->d > kBf16K && h->n < kWideFilterRows;
+  if (!force_fp32 && !small_wide && (h->batch_method == TOPK_BATCH_AUTO || h->batch_method == TOPK_BATCH_BF16 ||
                       h->batch_method == TOPK_BATCH_LEARNED)) {
     if ((st = ensure_bf16_table(h, s)) != TOPK_OK) return st;
     use_bf16 = h->xbf_usable && nq <= 0xFFFFFFFFull;
@@ -811,14 +830,14 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   const uint32_t nqq_all = (uint32_t)nq;
   uint64_t log_ctas = 0;
   if (use_bf16) {
-    std::vector<uint8_t> habf(bf16_query_bytes((uint32_t)nq), 0);
+    std::vector<uint8_t> habf(bf16_query_bytes((uint32_t)nq, h->d), 0);
     for (uint64_t j = 0; j < nq; j++) {
       // a[m] = the sum of the weights on attribute m (repeated attributes add up; FP32,
       // within 2^-19 of the exact sum for <= 32 terms, well inside the filter's bound)
       float a[kBf16MaxD] = {0.0f};
       for (uint32_t m = 0; m < q[j].qq; m++) a[q[j].attr[m]] += q[j].w[m];
-      bf16_pack_query(a, (uint32_t)j, habf.data());
-      q[j].err = bf16_error_bound(q[j], h->absmax);
+      bf16_pack_query(a, h->d, (uint32_t)j, habf.data());
+      q[j].err = bf16_error_bound(q[j], h->absmax, kblk);
       q[j].maxkey = score_bound_key(q[j], h->colmax, h->colmin);
     }
     if ((st = ensure(h->b_abf, habf.size())) != TOPK_OK) return st;
@@ -826,7 +845,7 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
     if ((st = ensure(h->b_amap, (nq + 1 + kMaxChunkLog) * sizeof(uint32_t))) != TOPK_OK) return st;
     if ((st = ensure(h->b_err, sizeof(uint32_t))) != TOPK_OK) return st;
     // survivor records: one log per filter CTA
-    const FilterPlan fp = plan_bf16_filter(nqq_all, 0, h->n, h->num_sms, h->batch_qt);
+    const FilterPlan fp = plan_bf16_filter(nqq_all, 0, h->n, h->d, h->num_sms, h->batch_qt);
     log_ctas = fp.grid;
     if ((st = ensure(h->b_log, log_ctas * kBf16LogCap * 8 * sizeof(uint4))) != TOPK_OK) return st;
     if ((st = ensure(h->b_logh, log_ctas * kBf16LogCap * sizeof(uint2))) != TOPK_OK) return st;
@@ -918,14 +937,14 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   for (uint64_t r = r_start, size = first_chunk; r < h->n; size = next_chunk(r, size)) {
     const uint64_t e = std::min<uint64_t>(h->n, r + size);
     if (use_bf16) {
-      const FilterPlan fp = plan_bf16_filter(nqq, r, e, h->num_sms, h->batch_qt);
+      const FilterPlan fp = plan_bf16_filter(nqq, r, e, h->d, h->num_sms, h->batch_qt);
       if (fp.grid > log_ctas) return fail(TOPK_ERR_STATE, "filter grid %llu above its logs", (unsigned long long)fp.grid);
       // the queries still served by the filter, as compact tiles
       uint32_t *amap = static_cast<uint32_t *>(h->b_amap.p);
       // the chunk's active count also goes to its slot of the per-batch record
       uint32_t *logslot = chunk < kMaxChunkLog ? amap + nq + 1 + chunk : nullptr;
       ++chunk;
-      CK(launch_batch_active(dq, dst, nqq, static_cast<const uint8_t *>(h->b_abf.p),
+      CK(launch_batch_active(dq, dst, nqq, h->d, static_cast<const uint8_t *>(h->b_abf.p),
                              static_cast<uint8_t *>(h->b_abf_act.p), amap, amap + nq, logslot, s));
       CK(launch_bf16_filter(fp, static_cast<const uint8_t *>(h->xbf.p), static_cast<const uint8_t *>(h->b_abf_act.p),
                             amap, amap + nq, r, e, dq, dst, dcand, static_cast<uint4 *>(h->b_log.p),
@@ -1038,7 +1057,7 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
     uint32_t c = 0;  // the chunks as issued (the graph replays the same sequence)
     for (uint64_t r = r_start, size = first_chunk; r < h->n && c < kMaxChunkLog; size = next_chunk(r, size), ++c) {
       const uint64_t e = std::min<uint64_t>(h->n, r + size);
-      filter_flops += (double)((hact[c] + 127) / 128 * 128) * (double)((e - r + 255) / 256 * 256) * 96.0;
+      filter_flops += (double)((hact[c] + 127) / 128 * 128) * (double)((e - r + 255) / 256 * 256) * 96.0 * kblk;
       r = e;
     }
   }
