@@ -95,7 +95,37 @@ __global__ void gather_rows_kernel(const float *__restrict__ table, uint64_t ld,
   }
 }
 
-// One block per partition: per-attribute min, max and mean of its rows.
+// A row-major copy of the table for the index builds (row i at rows + i * dp, dp = d
+// rounded up to 4, padded with zeros): a build reads whole rows in an order that is random
+// to the table, and d values of a row are d / 8 sectors of 32 bytes here against d in the
+// columns (6,000,011 x 8: the extremes of a level take 90 us against 242 from the columns,
+// the final gather 138 against 620; 2^27 x 8: 23 ms a level from the columns).
+__global__ void rows_kernel(const float *__restrict__ table, uint64_t ld, uint32_t d, uint64_t n, uint32_t dp,
+                            float *__restrict__ rows) {
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    for (uint32_t m = 0; m < dp; m += 4) {
+      float v[4];
+#pragma unroll
+      for (uint32_t u = 0; u < 4; ++u) v[u] = m + u < d ? __ldcs(table + (uint64_t)(m + u) * ld + i) : 0.0f;
+      *reinterpret_cast<float4 *>(rows + i * dp + m) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+__global__ void gather_rm_kernel(const float *__restrict__ rows, uint32_t dp, uint64_t ld, uint32_t d, uint64_t n,
+                                 const uint32_t *__restrict__ perm, float *__restrict__ ptable) {
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    const float *src = rows + (uint64_t)perm[i] * dp;
+    for (uint32_t m = 0; m < dp; m += 4) {
+      const float4 x = __ldg(reinterpret_cast<const float4 *>(src + m));
+      const float v[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (uint32_t u = 0; u < 4; ++u)
+        if (m + u < d) __stcs(ptable + (uint64_t)(m + u) * ld + i, v[u]);
+    }
+  }
+}
+
+// One block per partition and attribute: min, max and mean of its rows.
 __global__ void __launch_bounds__(256) part_stats_kernel(const float *__restrict__ ptable, uint64_t ld, uint32_t d,
                                                          uint64_t n, uint32_t rows_log2, float *__restrict__ mins,
                                                          float *__restrict__ maxs, float *__restrict__ means) {
@@ -103,39 +133,38 @@ __global__ void __launch_bounds__(256) part_stats_kernel(const float *__restrict
   const uint64_t r0 = (uint64_t)blockIdx.x << rows_log2;
   const uint64_t r1 = min((uint64_t)n, r0 + (uint64_t)(1ull << rows_log2));
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (uint32_t m = 0; m < d; ++m) {
-    const float *col = ptable + (uint64_t)m * ld;
-    float mn = __int_as_float(0x7F800000), mx = __int_as_float(0xFF800000);
-    float sum = 0.0f;  // the mean is a model feature only: FP32 partial sums suffice
-    for (uint64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
-      const float x = col[r];
-      mn = fminf(mn, x);
-      mx = fmaxf(mx, x);
-      sum += x;
+  const uint32_t m = blockIdx.y;
+  const float *col = ptable + (uint64_t)m * ld;
+  float mn = __int_as_float(0x7F800000), mx = __int_as_float(0xFF800000);
+  float sum = 0.0f;  // the mean is a model feature only: FP32 partial sums suffice
+#pragma unroll 8
+  for (uint64_t r = r0 + threadIdx.x; r < r1; r += 256) {
+    const float x = col[r];
+    mn = fminf(mn, x);
+    mx = fmaxf(mx, x);
+    sum += x;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    mn = fminf(mn, __shfl_xor_sync(0xFFFFFFFFu, mn, o));
+    mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+  }
+  if (lane == 0) {
+    smn[warp] = mn;
+    smx[warp] = mx;
+    ssum[warp] = sum;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (uint32_t w = 1; w < blockDim.x / 32; ++w) {
+      mn = fminf(mn, smn[w]);
+      mx = fmaxf(mx, smx[w]);
+      sum += ssum[w];
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      mn = fminf(mn, __shfl_xor_sync(0xFFFFFFFFu, mn, o));
-      mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-      sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-    }
-    if (lane == 0) {
-      smn[warp] = mn;
-      smx[warp] = mx;
-      ssum[warp] = sum;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (uint32_t w = 1; w < blockDim.x / 32; ++w) {
-        mn = fminf(mn, smn[w]);
-        mx = fmaxf(mx, smx[w]);
-        sum += ssum[w];
-      }
-      const size_t o = (size_t)blockIdx.x * d + m;
-      mins[o] = mn;
-      maxs[o] = mx;
-      means[o] = r1 > r0 ? sum / (float)(r1 - r0) : 0.0f;
-    }
-    __syncthreads();
+    const size_t o = (size_t)blockIdx.x * d + m;
+    mins[o] = mn;
+    maxs[o] = mx;
+    means[o] = r1 > r0 ? sum / (float)(r1 - r0) : 0.0f;
   }
 }
 
@@ -443,48 +472,51 @@ __device__ __forceinline__ uint32_t kd_node_of(uint32_t part, uint32_t P, uint32
   return id;
 }
 
-// Per node and attribute: the largest and smallest order key of the node's values
-// (NaN left out).  One block per chunk of 1024 positions (a chunk lies in one
-// partition, so in one node); stats: [node][d] max keys, then [node][d] min keys.
-__global__ void __launch_bounds__(256) kd_stats_kernel(const float *__restrict__ table, uint64_t ld, uint32_t d,
-                                                       uint64_t n, const uint32_t *__restrict__ perm, uint32_t lg,
-                                                       uint32_t P, uint32_t level, uint32_t nodes,
-                                                       uint32_t *__restrict__ stats) {
-  __shared__ uint32_t smax[32], smin[32];
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t chunks = (n + 1023) / 1024;
-  for (uint64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
-    const uint64_t base = c * 1024;
-    const uint32_t node = kd_node_of((uint32_t)(base >> lg), P, level);
-    uint32_t id[4];
+// Values [m0, m0 + 4) of row id: from the row-major copy when there is one, else from the
+// columns (a build without the memory for the copy).
+struct RowSource {
+  const float *table, *rows;  // rows may be null
+  uint64_t ld;
+  uint32_t d, dp;
+  __device__ __forceinline__ float4 load4(uint32_t id, uint32_t m0) const {
+    if (rows) return __ldg(reinterpret_cast<const float4 *>(rows + (uint64_t)id * dp + m0));
+    float v[4];
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const uint64_t pos = base + threadIdx.x + 256u * v;
-      id[v] = pos < n ? perm[pos] : 0xFFFFFFFFu;
-    }
-    for (uint32_t m0 = 0; m0 < d; m0 += 32) {
-      const uint32_t dm = min(32u, d - m0);
-      if (threadIdx.x < dm) {
+    for (uint32_t u = 0; u < 4; ++u) v[u] = m0 + u < d ? __ldg(table + (uint64_t)(m0 + u) * ld + id) : 0.0f;
+    return make_float4(v[0], v[1], v[2], v[3]);
+  }
+};
+
+// Per node and attribute: the largest and smallest order key of the node's values
+// (NaN left out).  A block takes a run of chunks of 1024 positions (a chunk lies in one
+// partition, so in one node) and eight attributes at a time -- a sector of a row -- and
+// keeps each thread's extremes in registers until the node changes; stats: [node][d] max
+// keys, then [node][d] min keys.
+constexpr uint32_t kKdStatAttrs = 8;
+__global__ void __launch_bounds__(256) kd_stats_kernel(const RowSource src, uint64_t n,
+                                                       const uint32_t *__restrict__ perm, uint32_t lg, uint32_t P,
+                                                       uint32_t level, uint32_t nodes, uint32_t *__restrict__ stats) {
+  __shared__ uint32_t smax[kKdStatAttrs], smin[kKdStatAttrs];
+  const uint32_t lane = threadIdx.x & 31, d = src.d;
+  const uint64_t chunks = (n + 1023) / 1024, per = (chunks + gridDim.x - 1) / gridDim.x;
+  const uint64_t c0 = (uint64_t)blockIdx.x * per, c1 = min(chunks, c0 + per);
+  for (uint32_t m0 = 0; m0 < d; m0 += kKdStatAttrs) {
+    const uint32_t dm = min(kKdStatAttrs, d - m0);
+    uint32_t kmax[kKdStatAttrs], kmin[kKdStatAttrs];
+    uint32_t node = 0;
+    auto flush = [&]() {  // (uniform) the run's extremes into its node's
+      if (threadIdx.x < kKdStatAttrs) {
         smax[threadIdx.x] = 0u;
         smin[threadIdx.x] = 0xFFFFFFFFu;
       }
       __syncthreads();
-      for (uint32_t m = 0; m < dm; ++m) {
-        uint32_t kmax = 0u, kmin = 0xFFFFFFFFu;
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          if (id[v] == 0xFFFFFFFFu) continue;
-          const float x = __ldg(table + (uint64_t)(m0 + m) * ld + id[v]);
-          if (x != x) continue;
-          const uint32_t k = f2key(x);
-          kmax = max(kmax, k);
-          kmin = min(kmin, k);
-        }
-        kmax = __reduce_max_sync(0xFFFFFFFFu, kmax);
-        kmin = __reduce_min_sync(0xFFFFFFFFu, kmin);
+      for (uint32_t m = 0; m < kKdStatAttrs; ++m) {
+        if (m >= dm) break;
+        const uint32_t hi = __reduce_max_sync(0xFFFFFFFFu, kmax[m]), lo = __reduce_min_sync(0xFFFFFFFFu, kmin[m]);
         if (lane == 0) {
-          atomicMax(&smax[m], kmax);
-          atomicMin(&smin[m], kmin);
+          atomicMax(&smax[m], hi);
+          atomicMin(&smin[m], lo);
         }
       }
       __syncthreads();
@@ -493,7 +525,46 @@ __global__ void __launch_bounds__(256) kd_stats_kernel(const float *__restrict__
         atomicMin(stats + (size_t)nodes * d + (size_t)node * d + m0 + threadIdx.x, smin[threadIdx.x]);
       }
       __syncthreads();
+    };
+    for (uint64_t c = c0; c < c1; ++c) {
+      const uint64_t base = c * 1024;
+      const uint32_t nd = kd_node_of((uint32_t)(base >> lg), P, level);
+      if (c == c0 || nd != node) {
+        if (c != c0) flush();
+        node = nd;
+#pragma unroll
+        for (uint32_t m = 0; m < kKdStatAttrs; ++m) {
+          kmax[m] = 0u;
+          kmin[m] = 0xFFFFFFFFu;
+        }
+      }
+      uint32_t id[4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const uint64_t pos = base + threadIdx.x + 256u * v;
+        id[v] = pos < n ? perm[pos] : 0xFFFFFFFFu;
+      }
+#pragma unroll
+      for (uint32_t g = 0; g < kKdStatAttrs; g += 4) {
+        if (g >= dm) break;
+        float4 x[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          x[v] = id[v] != 0xFFFFFFFFu ? src.load4(id[v], m0 + g) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const float f[4] = {x[v].x, x[v].y, x[v].z, x[v].w};
+#pragma unroll
+          for (uint32_t u = 0; u < 4; ++u)
+            if (id[v] != 0xFFFFFFFFu && f[u] == f[u]) {
+              const uint32_t k = f2key(f[u]);
+              kmax[g + u] = max(kmax[g + u], k);
+              kmin[g + u] = min(kmin[g + u], k);
+            }
+        }
+      }
     }
+    if (c0 < c1) flush();
   }
 }
 
@@ -520,17 +591,14 @@ __global__ void kd_split_kernel(const uint32_t *__restrict__ stats, uint32_t d, 
 }
 
 // Sort keys of level `level`: (node << 32 | order key of the row's value in the node's
-// split attribute), with the row ids.
-__global__ void kd_keys_kernel(const float *__restrict__ table, uint64_t ld, uint64_t n,
-                               const uint32_t *__restrict__ perm, uint32_t lg, uint32_t P, uint32_t level,
-                               const uint32_t *__restrict__ attr, unsigned long long *__restrict__ keys,
-                               uint32_t *__restrict__ ids) {
+// split attribute).  One value a row: from the columns, whose share of L2 is larger (6
+// million rows: 69 us a level against 96 from the row-major copy).
+__global__ void kd_keys_kernel(const float *__restrict__ table, uint64_t ld, uint64_t n, const uint32_t *__restrict__ perm, uint32_t lg,
+                               uint32_t P, uint32_t level, const uint32_t *__restrict__ attr,
+                               unsigned long long *__restrict__ keys) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t node = kd_node_of((uint32_t)(i >> lg), P, level);
-    const uint32_t id = perm[i];
-    const float x = __ldg(table + (uint64_t)attr[node] * ld + id);
-    keys[i] = ((unsigned long long)node << 32) | f2key(x);
-    ids[i] = id;
+    keys[i] = ((unsigned long long)node << 32) | f2key(__ldg(table + (uint64_t)attr[node] * ld + perm[i]));
   }
 }
 
@@ -546,9 +614,15 @@ uint64_t kd_order_work_words(uint64_t n, uint32_t d, uint32_t P) {
   return 5 * n + 2 * (uint64_t)P * d + P;
 }
 
+cudaError_t launch_rows(const float *table, uint64_t ld, uint32_t d, uint64_t n, float *rows, int num_sms,
+                        cudaStream_t s) {
+  rows_kernel<<<grid_for(n, num_sms), 256, 0, s>>>(table, ld, d, n, row_stride(d), rows);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_kd_order(const float *table, uint64_t ld, uint32_t d, uint64_t n, uint32_t part_log2,
                             uint32_t *perm, uint32_t *work, void *temp, size_t *temp_bytes, int num_sms,
-                            cudaStream_t s) {
+                            cudaStream_t s, const float *rows) {
   if (n > 0x7FFFFFFFull || d == 0) return cudaErrorInvalidValue;
   const uint32_t P = (uint32_t)((n + (1ull << part_log2) - 1) >> part_log2);
   const uint32_t L = kd_levels(P);
@@ -562,9 +636,11 @@ cudaError_t launch_kd_order(const float *table, uint64_t ld, uint32_t d, uint64_
   if (!temp) {  // size query
     return cub::DeviceRadixSort::SortPairs(nullptr, *temp_bytes, kin, kout, ids, perm, nn, 0, 64, s);
   }
+  const RowSource src{table, rows, ld, d, row_stride(d)};
   const int g = grid_for(n, num_sms);
   size_t tb = *temp_bytes;
-  iota_kernel<<<g, 256, 0, s>>>(perm, n);
+  uint32_t *cur = perm, *next = ids;  // the order so far, and where the next level's goes
+  iota_kernel<<<g, 256, 0, s>>>(cur, n);
   cudaError_t e = cudaGetLastError();
   for (uint32_t level = 0; e == cudaSuccess && level < L; ++level) {
     const uint32_t nodes = 1u << level;
@@ -573,25 +649,28 @@ cudaError_t launch_kd_order(const float *table, uint64_t ld, uint32_t d, uint64_
     if (e != cudaSuccess) break;
     const uint64_t chunks = (n + 1023) / 1024;
     const int gs = (int)std::min<uint64_t>(chunks, (uint64_t)num_sms * 8);
-    kd_stats_kernel<<<gs, 256, 0, s>>>(table, ld, d, n, perm, part_log2, P, level, nodes, stats);
+    kd_stats_kernel<<<gs, 256, 0, s>>>(src, n, cur, part_log2, P, level, nodes, stats);
     kd_split_kernel<<<(nodes + 255) / 256, 256, 0, s>>>(stats, d, nodes, attr);
-    kd_keys_kernel<<<g, 256, 0, s>>>(table, ld, n, perm, part_log2, P, level, attr, kin, ids);
+    kd_keys_kernel<<<g, 256, 0, s>>>(table, ld, n, cur, part_log2, P, level, attr, kin);
     e = cudaGetLastError();
     // the sorted ids are the next order; node ids < 2^level sit above the 32 key bits
-    if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(temp, tb, kin, kout, ids, perm, nn, 0, 32 + (int)level, s);
+    if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(temp, tb, kin, kout, cur, next, nn, 0, 32 + (int)level, s);
+    std::swap(cur, next);
   }
+  if (e == cudaSuccess && cur != perm) e = cudaMemcpyAsync(perm, cur, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
   return e;
 }
 
 cudaError_t launch_gather_rows(const float *table, uint64_t ld, uint32_t d, uint64_t n, const uint32_t *perm,
-                               float *ptable, int num_sms, cudaStream_t s) {
-  gather_rows_kernel<<<grid_for(n, num_sms), 256, 0, s>>>(table, ld, d, n, perm, ptable);
+                               float *ptable, int num_sms, cudaStream_t s, const float *rows) {
+  if (rows) gather_rm_kernel<<<grid_for(n, num_sms), 256, 0, s>>>(rows, row_stride(d), ld, d, n, perm, ptable);
+  else gather_rows_kernel<<<grid_for(n, num_sms), 256, 0, s>>>(table, ld, d, n, perm, ptable);
   return cudaGetLastError();
 }
 
 cudaError_t launch_partition_stats(const float *ptable, uint64_t ld, uint32_t d, uint64_t n, uint32_t rows_log2,
                                    uint32_t num_parts, float *mins, float *maxs, float *means, cudaStream_t s) {
-  part_stats_kernel<<<num_parts, 256, 0, s>>>(ptable, ld, d, n, rows_log2, mins, maxs, means);
+  part_stats_kernel<<<dim3(num_parts, d), 256, 0, s>>>(ptable, ld, d, n, rows_log2, mins, maxs, means);
   return cudaGetLastError();
 }
 

@@ -1754,104 +1754,110 @@ int topk_build_partitions_ordered(topk_table_t h, uint32_t part_rows, int order)
     while (sla_bits < 31 && (1ull << sla_bits) < nl) ++sla_bits;
   }
   // column extremes: the Morton code quantises each attribute over [min, max]
-  CK(launch_minmax(h->table, h->ld, h->d, h->n, h->d_minmax, s));
-  std::vector<uint32_t> w((size_t)h->d * kMinmaxWords);
-  CK(cudaMemcpyAsync(w.data(), h->d_minmax, w.size() * 4, cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
   const uint32_t dims = std::min<uint32_t>(h->d, 16u);
   const uint32_t bits = std::max<uint32_t>(1u, 16u / dims);
   std::vector<float> lo_scale(2 * (size_t)h->d, 0.0f);
-  for (uint32_t m = 0; m < h->d; m++) {
-    auto k2f = [](uint32_t k) {
-      uint32_t u = (k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k;
-      float f;
-      std::memcpy(&f, &u, 4);
-      return f;
-    };
-    const float mx = k2f(w[(size_t)m * kMinmaxWords]), mn = k2f(w[(size_t)m * kMinmaxWords + 1]);
-    const float range = mx - mn;  // only decides the order of the rows, never a result
-    lo_scale[m] = std::isfinite(mn) ? mn : 0.0f;
-    lo_scale[h->d + m] = (range > 0.0f && std::isfinite(range)) ? std::ldexp(1.0f, (int)bits) / range : 0.0f;
+  if (order == TOPK_ORDER_MORTON) {
+    CK(launch_minmax(h->table, h->ld, h->d, h->n, h->d_minmax, s));
+    std::vector<uint32_t> w((size_t)h->d * kMinmaxWords);
+    CK(cudaMemcpyAsync(w.data(), h->d_minmax, w.size() * 4, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    for (uint32_t m = 0; m < h->d; m++) {
+      const float mx = host_key2f(w[(size_t)m * kMinmaxWords]), mn = host_key2f(w[(size_t)m * kMinmaxWords + 1]);
+      const float range = mx - mn;  // only decides the order of the rows, never a result
+      lo_scale[m] = std::isfinite(mn) ? mn : 0.0f;
+      lo_scale[h->d + m] = (range > 0.0f && std::isfinite(range)) ? std::ldexp(1.0f, (int)bits) / range : 0.0f;
+    }
   }
-  // release an older copy first (its memory may be needed)
-  cudaFree(h->ptable);
-  cudaFree(h->pids);
-  cudaFree(h->pstats);
-  h->ptable = nullptr;
-  h->pids = nullptr;
-  h->pstats = nullptr;
+  // An older copy of this table's size is written over (a rebuild's cudaFree and cudaMalloc
+  // of gigabytes cost more than the build); it is no copy of anything until this returns.
+  h->part_version = 0;
+  if (h->num_parts != P) {
+    cudaFree(h->pstats);
+    h->pstats = nullptr;
+  }
   h->num_parts = 0;
-  uint16_t *keys = nullptr;
-  uint32_t *hist = nullptr;
-  float *dls = nullptr;
-  auto cleanup = [&]() {
-    cudaFree(keys);
-    cudaFree(hist);
-    cudaFree(dls);
-  };
-  cudaError_t e = cudaMalloc(&keys, h->n * sizeof(uint16_t));
-  if (e == cudaSuccess) e = cudaMalloc(&hist, (1u << 16) * sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMalloc(&dls, lo_scale.size() * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&h->pids, h->n * sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMalloc(&h->ptable, h->ld * h->d * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&h->pstats, 3 * P * h->d * sizeof(float));
-  if (e == cudaSuccess) e = cudaMemsetAsync(h->ptable, 0, h->ld * h->d * sizeof(float), s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dls, lo_scale.data(), lo_scale.size() * 4, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess && order == TOPK_ORDER_MORTON)
-    e = launch_partition_build(h->table, h->ld, h->d, h->n, dls, dls + h->d, bits, keys, hist, h->pids, h->ptable,
-                               h->num_sms, s);
-  if (e == cudaSuccess && order == TOPK_ORDER_KD) {
-    uint32_t *work = nullptr;
-    void *temp = nullptr;
-    size_t temp_bytes = 0;
-    e = launch_kd_order(h->table, h->ld, h->d, h->n, lg, h->pids, nullptr, nullptr, &temp_bytes, h->num_sms, s);
-    if (e == cudaSuccess) e = cudaMalloc(&work, kd_order_work_words(h->n, h->d, (uint32_t)P) * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&temp, std::max<size_t>(temp_bytes, 16));
-    if (e == cudaSuccess)
-      e = launch_kd_order(h->table, h->ld, h->d, h->n, lg, h->pids, work, temp, &temp_bytes, h->num_sms, s);
-    if (e == cudaSuccess) e = launch_gather_rows(h->table, h->ld, h->d, h->n, h->pids, h->ptable, h->num_sms, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // before the scratch goes
-    cudaFree(work);
-    cudaFree(temp);
+  cudaError_t e = cudaSuccess;
+  if (!h->pids) e = cudaMalloc(&h->pids, h->n * sizeof(uint32_t));
+  if (e == cudaSuccess && !h->ptable) {
+    e = cudaMalloc(&h->ptable, h->ld * h->d * sizeof(float));
+    if (e == cudaSuccess) e = cudaMemsetAsync(h->ptable, 0, h->ld * h->d * sizeof(float), s);
   }
-  if (e == cudaSuccess && order != TOPK_ORDER_MORTON && order != TOPK_ORDER_KD) {
+  if (e == cudaSuccess && !h->pstats) e = cudaMalloc(&h->pstats, 3 * P * h->d * sizeof(float));
+  // the build's scratch: work | radix sort scratch | row-major copy (left out when there is
+  // no memory for it) in one allocation
+  unsigned char *scratch = nullptr;
+  size_t temp_bytes = 0;
+  auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+  float *rows = nullptr;
+  uint32_t *work = nullptr;
+  void *temp = nullptr;
+  auto allocate = [&](size_t work_bytes) -> cudaError_t {
+    const size_t fixed = up(work_bytes) + up(std::max<size_t>(temp_bytes, 16));
+    const size_t rows_bytes = (size_t)h->n * row_stride(h->d) * sizeof(float);
+    cudaError_t ce = cudaMalloc(&scratch, fixed + rows_bytes);
+    const bool with_rows = ce == cudaSuccess;
+    if (!with_rows) {
+      (void)cudaGetLastError();
+      ce = cudaMalloc(&scratch, fixed);
+    }
+    if (ce != cudaSuccess) return ce;
+    work = reinterpret_cast<uint32_t *>(scratch);
+    temp = scratch + up(work_bytes);
+    if (with_rows) {
+      rows = reinterpret_cast<float *>(scratch + fixed);
+      ce = launch_rows(h->table, h->ld, h->d, h->n, rows, h->num_sms, s);
+    }
+    return ce;
+  };
+  if (e == cudaSuccess && order == TOPK_ORDER_MORTON) {
+    // scratch: keys | histogram | column minima and scales
+    const size_t kb = up(h->n * sizeof(uint16_t)), hb = (1u << 16) * sizeof(uint32_t);
+    e = cudaMalloc(&scratch, kb + hb + lo_scale.size() * sizeof(float));
+    float *dls = reinterpret_cast<float *>(scratch + kb + hb);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dls, lo_scale.data(), lo_scale.size() * 4, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess)
+      e = launch_partition_build(h->table, h->ld, h->d, h->n, dls, dls + h->d, bits,
+                                 reinterpret_cast<uint16_t *>(scratch), reinterpret_cast<uint32_t *>(scratch + kb),
+                                 h->pids, h->ptable, h->num_sms, s);
+  } else if (e == cudaSuccess && order == TOPK_ORDER_KD) {
+    e = launch_kd_order(h->table, h->ld, h->d, h->n, lg, h->pids, nullptr, nullptr, &temp_bytes, h->num_sms, s,
+                        nullptr);
+    if (e == cudaSuccess) e = allocate(kd_order_work_words(h->n, h->d, (uint32_t)P) * sizeof(uint32_t));
+    if (e == cudaSuccess)
+      e = launch_kd_order(h->table, h->ld, h->d, h->n, lg, h->pids, work, temp, &temp_bytes, h->num_sms, s, rows);
+    if (e == cudaSuccess) e = launch_gather_rows(h->table, h->ld, h->d, h->n, h->pids, h->ptable, h->num_sms, s, rows);
+  } else if (e == cudaSuccess) {
     const IndexOrder kind = order == TOPK_ORDER_PTA           ? IndexOrder::kPta
                             : order == TOPK_ORDER_VTA_THREADS ? IndexOrder::kVtaThreads
                             : order == TOPK_ORDER_SLA         ? IndexOrder::kGroups
                                                               : IndexOrder::kVta;
-    uint32_t *work = nullptr, *groups = nullptr;
-    void *temp = nullptr;
-    size_t temp_bytes = 0;
-    if (kind == IndexOrder::kGroups) {
-      e = cudaMalloc(&groups, h->n * sizeof(uint32_t));
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(groups, sla_layers.data(), h->n * sizeof(uint32_t), cudaMemcpyHostToDevice, s);
+    const uint64_t words = index_order_work_words(h->n, kind);
+    uint32_t *groups = nullptr;
+    e = launch_index_order(h->table, h->ld, h->d, h->n, kind, h->pids, nullptr, nullptr, &temp_bytes, h->num_sms, s,
+                           h->pids, sla_bits);  // (sizes only)
+    if (e == cudaSuccess) e = allocate((words + (kind == IndexOrder::kGroups ? h->n : 0)) * sizeof(uint32_t));
+    if (e == cudaSuccess && kind == IndexOrder::kGroups) {
+      groups = work + words;
+      e = cudaMemcpyAsync(groups, sla_layers.data(), h->n * sizeof(uint32_t), cudaMemcpyHostToDevice, s);
     }
-    if (e == cudaSuccess)
-      e = launch_index_order(h->table, h->ld, h->d, h->n, kind, h->pids, nullptr, nullptr, &temp_bytes, h->num_sms, s,
-                             groups, sla_bits);
-    if (e == cudaSuccess) e = cudaMalloc(&work, index_order_work_words(h->n, kind) * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&temp, std::max<size_t>(temp_bytes, 16));
     if (e == cudaSuccess)
       e = launch_index_order(h->table, h->ld, h->d, h->n, kind, h->pids, work, temp, &temp_bytes, h->num_sms, s,
                              groups, sla_bits);
-    if (e == cudaSuccess) e = launch_gather_rows(h->table, h->ld, h->d, h->n, h->pids, h->ptable, h->num_sms, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // before the scratch goes
-    cudaFree(work);
-    cudaFree(temp);
-    cudaFree(groups);
+    if (e == cudaSuccess) e = launch_gather_rows(h->table, h->ld, h->d, h->n, h->pids, h->ptable, h->num_sms, s, rows);
   }
   float *pmin = h->pstats, *pmax = h->pstats + P * h->d, *pmean = h->pstats + 2 * P * h->d;
   if (e == cudaSuccess) e = launch_partition_stats(h->ptable, h->ld, h->d, h->n, lg, (uint32_t)P, pmin, pmax, pmean, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cleanup();
-  if (e != cudaSuccess) return cuda_fail(e, "topk_build_partitions");
   h->pmin.resize(P * h->d);
   h->pmax.resize(P * h->d);
   h->pmean.resize(P * h->d);
-  CK(cudaMemcpy(h->pmin.data(), pmin, P * h->d * 4, cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(h->pmax.data(), pmax, P * h->d * 4, cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(h->pmean.data(), pmean, P * h->d * 4, cudaMemcpyDeviceToHost));
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h->pmin.data(), pmin, P * h->d * 4, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h->pmax.data(), pmax, P * h->d * 4, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h->pmean.data(), pmean, P * h->d * 4, cudaMemcpyDeviceToHost, s);
+  const cudaError_t es = cudaStreamSynchronize(s);  // before the scratch goes
+  if (e == cudaSuccess) e = es;
+  cudaFree(scratch);
+  if (e != cudaSuccess) return cuda_fail(e, "topk_build_partitions");
   h->part_log2 = lg;
   h->num_parts = (uint32_t)P;
   h->part_version = h->data_version;

@@ -274,8 +274,13 @@ cudaError_t launch_index_order(const float *table, uint64_t ld, uint32_t d, uint
 // d <= 32, n < 2^31.  layers: n entries on the host.
 int skyline_layers_device(const float *table, uint64_t ld, uint32_t d, uint64_t n, int num_sms, uint32_t *layers,
                           uint64_t *num_layers, std::string *msg);
+// A row-major copy of the table for an index build (n * row_stride(d) floats), which reads
+// whole rows in random order; `rows` below may be null (then the columns are read).
+inline uint32_t row_stride(uint32_t d) { return (d + 3u) / 4u * 4u; }
+cudaError_t launch_rows(const float *table, uint64_t ld, uint32_t d, uint64_t n, float *rows, int num_sms,
+                        cudaStream_t s);
 cudaError_t launch_gather_rows(const float *table, uint64_t ld, uint32_t d, uint64_t n, const uint32_t *perm,
-                               float *ptable, int num_sms, cudaStream_t s);
+                               float *ptable, int num_sms, cudaStream_t s, const float *rows);
 // kd order (partition.cu): the partitions of 2^part_log2 rows are the leaves of a
 // balanced binary tree; each node is split at its middle partition boundary after its
 // rows are sorted by the attribute of widest spread in it.  n < 2^31.  work:
@@ -284,7 +289,7 @@ uint32_t kd_levels(uint32_t P);
 uint64_t kd_order_work_words(uint64_t n, uint32_t d, uint32_t P);
 cudaError_t launch_kd_order(const float *table, uint64_t ld, uint32_t d, uint64_t n, uint32_t part_log2,
                             uint32_t *perm, uint32_t *work, void *temp, size_t *temp_bytes, int num_sms,
-                            cudaStream_t s);
+                            cudaStream_t s, const float *rows);
 // One query's attributes and gathered weights, for partition bounds.
 struct PartQuery {
   uint32_t qq;
