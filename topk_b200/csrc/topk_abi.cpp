@@ -3,9 +3,9 @@
 // A handle owns the device copy of the table (column-major, stride ld = n rounded
 // up to 64 rows so every column starts 256-byte aligned, which the bulk copies
 // need) and a pool of query contexts.  A context is one stream, one device
-// scratch block for the fused scan, one device result block and a pinned host
-// mirror of it, so a synchronous query costs one kernel launch, one
-// device-to-host copy and one stream synchronisation.  Concurrent callers (the
+// scratch block for the fused scan and one result block in mapped pinned memory,
+// so a synchronous query costs one kernel launch and one stream synchronisation
+// (the kernel writes the result to the host).  Concurrent callers (the
 // reference's findTopKsimdMQ threads, validation/bench_cpu.h:204-212) each take
 // their own context from the pool.
 #include "../../include/topk_b200.h"
@@ -21,6 +21,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "batch_internal.h"
@@ -68,7 +69,7 @@ struct DeviceGuard {
   }
 };
 
-// Result block layout (device and pinned host mirror): header, ids[k], scores[k].
+// Result block layout: header, ids[k], scores[k].
 struct ResultHeader {
   uint32_t count;
   float threshold;
@@ -78,26 +79,24 @@ struct ResultHeader {
 };
 constexpr size_t kHdr = sizeof(ResultHeader);  // 64 bytes
 size_t result_bytes(uint32_t k) { return kHdr + (size_t)k * 8 + (size_t)k * 4; }
-// The pinned result mirror also stages a pruned query's descriptor after the result.
+// The pinned result block also stages a pruned query's descriptor after the result.
 constexpr size_t kStageBytes = 256;
 
 struct Ctx {
   cudaStream_t stream = nullptr;
   // Device scratch of the fused scan, one allocation:
-  //   ScanScratch | done[max_groups] | slot_count[max_slots] | pad | slots[max_slots * kMaxK]
+  //   ScanScratch | done[max_groups] | slot_count[max_slots] | pad | slots[max_slots * kMaxK] |
+  //   pub[max_grid * kPubMaxEntries] | epub[kMaxEpochs][max_grid * kPubMaxKeys] | two counts
   ScanScratch *scratch = nullptr;
   uint32_t *done = nullptr;
   uint32_t *slot_count = nullptr;
   uint2 *slots = nullptr;
-  // published best entries (kPubMaxEntries per CTA of the largest grid), one allocation:
-  // pub[max_grid * kPubMaxEntries] | epub[kMaxEpochs][max_grid * kPubMaxKeys]
-  uint2 *pub = nullptr;
-  uint2 *epub = nullptr;
+  uint2 *pub = nullptr;   // published best entries (kPubMaxEntries per CTA of the largest grid)
+  uint2 *epub = nullptr;  // and those of each threshold epoch
   uint32_t epub_stride = 0;
   uint32_t max_slots = 0, max_groups = 0;
   size_t slot_entries = 0;  // capacity of `slots`
   size_t meta_bytes = 0;    // bytes that must be zero between queries (header + done)
-  unsigned char *h_res = nullptr;  // pinned mirror
   // Result block of the synchronous queries in mapped pinned memory (h_out on the host,
   // d_out its device address): the scan's root writes ids, scores and the header
   // straight to the host, so no copy follows the scan.
@@ -148,13 +147,15 @@ struct topk_table_s {
     void *p = nullptr;
     size_t bytes = 0;
   };
-  DevBuf b_q, b_st, b_best, b_cand, b_ids, b_scores, b_count, b_thr;
+  // a batch's inputs (query descriptors, the filter's query tiles, the FP32 scorer's query
+  // order) and what it reports (ids, scores, counts, thresholds, states, per-chunk counts,
+  // error and hybrid words), one buffer and one copy each way
+  DevBuf b_in, b_out, b_best, b_cand;
   // BF16 filter: split copy of the table (rebuilt when the table changed), the
-  // per-column max |x| it was built from, the batch's query tiles and error word
-  DevBuf xbf, xbf_absmax, b_abf, b_err, b_log, b_logh, b_sw, b_feat, b_pred;
-  // compact active query tiles of the filter, slot -> query map and count; the plain
-  // FP32 scorer's query order (by attribute count)
-  DevBuf b_abf_act, b_amap, b_order;
+  // per-column max |x| it was built from, the survivor records
+  DevBuf xbf, xbf_absmax, b_log, b_logh, b_feat, b_pred;
+  // compact active query tiles of the filter, slot -> query map and count
+  DevBuf b_abf_act, b_amap;
   uint64_t data_version = 1, xbf_version = 0;
   std::vector<float> absmax, colmax, colmin;  // per column: max |x|, max, min (NaN left out)
   bool xbf_usable = false;
@@ -185,10 +186,13 @@ struct topk_table_s {
   uint64_t last_batch_switched = 0;  // queries a hybrid batch moved from the filter to the FP32 scorer
   uint64_t last_batch_retired = 0;   // queries the filter retired (threshold above their score bound)
   double last_batch_filter_flops = 0;  // MMA flops the filter ran (three BF16 passes)
-  // pinned host copies of a batch's results (grow-only): copied at full link speed,
-  // no page faults on the critical path
-  void *hb_res = nullptr;
-  size_t hb_bytes = 0;
+  // pinned host copies of b_in and b_out (grow-only): copied at full link speed, no page
+  // faults on the critical path
+  struct HostBuf {
+    unsigned char *p = nullptr;
+    size_t bytes = 0;
+  };
+  HostBuf hb_in, hb_out;
   // the device work of a batch, captured once per shape and replayed (a few shapes:
   // a learned batch's rerun of its misses is a second one)
   struct BatchGraph {
@@ -213,9 +217,6 @@ int ctx_create(topk_table_t h, Ctx **out) {
   auto bail = [&](cudaError_t e, const char *what) {
     if (c->stream) cudaStreamDestroy(c->stream);
     cudaFree(c->scratch);
-    cudaFree(c->pub);
-    cudaFree(c->d_count2);
-    if (c->h_res) cudaFreeHost(c->h_res);
     if (c->h_out) cudaFreeHost(c->h_out);
     delete c;
     return cuda_fail(e, what);
@@ -232,7 +233,11 @@ int ctx_create(topk_table_t h, Ctx **out) {
   c->slot_entries = (size_t)4 * (size_t)h->num_sms * kMaxK;
   c->meta_bytes = sizeof(ScanScratch) + (size_t)c->max_groups * 4;
   const size_t slots_off = (c->meta_bytes + (size_t)c->max_slots * 4 + 255) / 256 * 256;
-  const size_t bytes = slots_off + c->slot_entries * sizeof(uint2);
+  c->epub_stride = kPubMaxKeys * max_grid;
+  const size_t pub_off = slots_off + c->slot_entries * sizeof(uint2),
+               epub_off = pub_off + (size_t)kPubMaxEntries * max_grid * sizeof(uint2),
+               count_off = epub_off + (size_t)kMaxEpochs * c->epub_stride * sizeof(uint2);
+  const size_t bytes = count_off + 2 * sizeof(unsigned long long);
   unsigned char *blk = nullptr;
   if ((e = cudaMalloc(&blk, bytes)) != cudaSuccess) return bail(e, "scan scratch");
   c->scratch = reinterpret_cast<ScanScratch *>(blk);
@@ -240,16 +245,10 @@ int ctx_create(topk_table_t h, Ctx **out) {
   c->slot_count = reinterpret_cast<uint32_t *>(blk + c->meta_bytes);
   c->slots = reinterpret_cast<uint2 *>(blk + slots_off);
   if ((e = cudaMemset(blk, 0, slots_off)) != cudaSuccess) return bail(e, "scratch memset");
-  c->epub_stride = kPubMaxKeys * max_grid;
-  const size_t pub_entries_max = (size_t)kPubMaxEntries * max_grid;
-  if ((e = cudaMalloc(&c->pub, (pub_entries_max + (size_t)kMaxEpochs * c->epub_stride) * sizeof(uint2))) !=
-      cudaSuccess)
-    return bail(e, "publish area");
-  c->epub = c->pub + pub_entries_max;
-  if ((e = cudaMalloc(&c->d_count2, 2 * sizeof(unsigned long long))) != cudaSuccess) return bail(e, "count");
-  if ((e = cudaHostAlloc(&c->h_res, result_bytes(kMaxK) + kStageBytes, cudaHostAllocDefault)) != cudaSuccess)
-    return bail(e, "pinned result");
-  if ((e = cudaHostAlloc(&c->h_out, result_bytes(kMaxK), cudaHostAllocMapped)) != cudaSuccess)
+  c->pub = reinterpret_cast<uint2 *>(blk + pub_off);
+  c->epub = reinterpret_cast<uint2 *>(blk + epub_off);
+  c->d_count2 = reinterpret_cast<unsigned long long *>(blk + count_off);
+  if ((e = cudaHostAlloc(&c->h_out, result_bytes(kMaxK) + kStageBytes, cudaHostAllocMapped)) != cudaSuccess)
     return bail(e, "mapped result");
   if ((e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&c->d_out), c->h_out, 0)) != cudaSuccess)
     return bail(e, "mapped result address");
@@ -262,15 +261,12 @@ void ctx_free(Ctx *c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->stream) cudaStreamDestroy(c->stream);
   cudaFree(c->scratch);
-  cudaFree(c->pub);
-  cudaFree(c->d_count2);
   cudaFree(c->d_ids_scratch);
   cudaFree(c->d_rows);
   cudaFree(c->d_plist);
   cudaFree(c->d_pkey);
   cudaFree(c->d_ptemp);
   cudaFree(c->d_lq);
-  if (c->h_res) cudaFreeHost(c->h_res);
   if (c->h_out) cudaFreeHost(c->h_out);
   delete c;
 }
@@ -573,7 +569,7 @@ int run_pruned(topk_table_t h, uint64_t k, uint32_t qq, const float *weights, co
     const uint64_t k1 = k;
     const std::vector<BatchQuery> bq = pack_queries(h, 1, &k1, &qq, weights, 0, attr, 0);
     static_assert(sizeof(BatchQuery) <= kStageBytes, "descriptor staging");
-    unsigned char *stage = c->h_res + result_bytes(kMaxK);  // pinned, after the result area
+    unsigned char *stage = c->h_out + result_bytes(kMaxK);  // pinned, after the result area
     std::memcpy(stage, &bq[0], sizeof(BatchQuery));
     BatchQuery *dq = reinterpret_cast<BatchQuery *>(c->d_lq);
     float *X = reinterpret_cast<float *>(c->d_lq + qb);
@@ -651,11 +647,46 @@ int ensure(topk_table_s::DevBuf &b, size_t bytes) {
   return TOPK_OK;
 }
 
+// Grow a cached pinned buffer to at least `bytes`.
+int ensure(topk_table_s::HostBuf &b, size_t bytes) {
+  if (b.bytes >= bytes) return TOPK_OK;
+  if (b.p) cudaFreeHost(b.p);
+  b = topk_table_s::HostBuf{};
+  if (cudaHostAlloc(reinterpret_cast<void **>(&b.p), bytes, cudaHostAllocDefault) != cudaSuccess) {
+    (void)cudaGetLastError();
+    b.p = nullptr;
+    return fail(TOPK_ERR_OOM, "pinned batch buffer of %zu bytes", bytes);
+  }
+  b.bytes = bytes;
+  return TOPK_OK;
+}
+
+// fn(begin, end) over [0, n) on up to four threads when `bytes` of work are worth them (a
+// thread costs ~30 us to start); on this one when no thread can be had.  4096 queries on
+// 2^26 x 16: 37.2 ms on one thread, 35.7 on two, 34.6 on four, 34.5 on eight.
+template <class Fn>
+void in_parallel(uint64_t n, size_t bytes, const Fn &fn) {
+  const uint64_t hw = std::max(1u, std::thread::hardware_concurrency());
+  const uint64_t nt = std::min<uint64_t>({4, hw, n, bytes / (2u << 20) + 1});
+  std::vector<std::thread> th;
+  uint64_t at = n / nt;  // this thread's share is [0, at)
+  const uint64_t mine = at;
+  for (uint64_t i = 1; i < nt; i++) {
+    const uint64_t end = n * (i + 1) / nt;
+    try {
+      th.emplace_back([&fn, at, end] { fn(at, end); });
+    } catch (...) {
+      fn(at, end);
+    }
+    at = end;
+  }
+  fn(0, mine);
+  for (std::thread &t : th) t.join();
+}
+
 void free_batch_buffers(topk_table_t h) {
-  for (topk_table_s::DevBuf *b : {&h->b_q, &h->b_st, &h->b_best, &h->b_cand, &h->b_ids, &h->b_scores, &h->b_count,
-                                  &h->b_thr, &h->xbf, &h->xbf_absmax, &h->b_abf, &h->b_err, &h->b_log,
-                                  &h->b_logh, &h->b_sw, &h->b_feat, &h->b_pred, &h->b_abf_act, &h->b_amap,
-                                  &h->b_order}) {
+  for (topk_table_s::DevBuf *b : {&h->b_in, &h->b_out, &h->b_best, &h->b_cand, &h->xbf, &h->xbf_absmax, &h->b_log,
+                                  &h->b_logh, &h->b_feat, &h->b_pred, &h->b_abf_act, &h->b_amap}) {
     cudaFree(b->p);
     b->p = nullptr;
     b->bytes = 0;
@@ -663,9 +694,10 @@ void free_batch_buffers(topk_table_t h) {
   if (h->b_ev0) cudaEventDestroy(h->b_ev0);
   if (h->b_ev1) cudaEventDestroy(h->b_ev1);
   h->b_ev0 = h->b_ev1 = nullptr;
-  if (h->hb_res) cudaFreeHost(h->hb_res);
-  h->hb_res = nullptr;
-  h->hb_bytes = 0;
+  for (topk_table_s::HostBuf *b : {&h->hb_in, &h->hb_out}) {
+    if (b->p) cudaFreeHost(b->p);
+    *b = topk_table_s::HostBuf{};
+  }
   for (auto &g : h->b_graphs) {
     if (g.exec) cudaGraphExecDestroy(g.exec);
     g = topk_table_s::BatchGraph{};
@@ -828,68 +860,81 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   }
   h->last_batch_method = use_learned ? TOPK_BATCH_LEARNED : use_bf16 ? TOPK_BATCH_BF16 : TOPK_BATCH_FP32;
   const uint32_t nqq_all = (uint32_t)nq;
+  // Survivor records per filter CTA: a chunk passes about 3k candidates a query, and an
+  // eighth of the batch's may fall to one CTA before queries move to the FP32 scorer.  (At
+  // kBf16LogCap the logs take 660 MB, most of a small batch's first call.)
+  const uint32_t rec_cap = (uint32_t)std::min<uint64_t>(kBf16LogCap, (4096 + 3 * best_total / 8) / 16 * 16);
   uint64_t log_ctas = 0;
+  auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+  // inputs: descriptors | query tiles of the filter, or the FP32 scorer's query order
+  const size_t abf_bytes = use_bf16 ? bf16_query_bytes(nqq_all, h->d) : 0;
+  const size_t in_abf = up(nq * sizeof(BatchQuery)), in_bytes = in_abf + (use_bf16 ? abf_bytes : nq * sizeof(uint32_t));
+  if ((st = ensure(h->b_in, in_bytes)) != TOPK_OK) return st;
+  if ((st = ensure(h->hb_in, in_bytes)) != TOPK_OK) return st;
   if (use_bf16) {
-    std::vector<uint8_t> habf(bf16_query_bytes((uint32_t)nq, h->d), 0);
-    for (uint64_t j = 0; j < nq; j++) {
-      // a[m] = the sum of the weights on attribute m (repeated attributes add up; FP32,
-      // within 2^-19 of the exact sum for <= 32 terms, well inside the filter's bound)
-      float a[kBf16MaxD] = {0.0f};
-      for (uint32_t m = 0; m < q[j].qq; m++) a[q[j].attr[m]] += q[j].w[m];
-      bf16_pack_query(a, h->d, (uint32_t)j, habf.data());
-      q[j].err = bf16_error_bound(q[j], h->absmax, kblk);
-      q[j].maxkey = score_bound_key(q[j], h->colmax, h->colmin);
-    }
-    if ((st = ensure(h->b_abf, habf.size())) != TOPK_OK) return st;
-    if ((st = ensure(h->b_abf_act, habf.size())) != TOPK_OK) return st;
-    if ((st = ensure(h->b_amap, (nq + 1 + kMaxChunkLog) * sizeof(uint32_t))) != TOPK_OK) return st;
-    if ((st = ensure(h->b_err, sizeof(uint32_t))) != TOPK_OK) return st;
+    uint8_t *habf = h->hb_in.p + in_abf;
+    std::memset(habf, 0, abf_bytes);
+    in_parallel(nq, nq * 2048, [&](uint64_t j0, uint64_t j1) {
+      for (uint64_t j = j0; j < j1; j++) {
+        // a[m] = the sum of the weights on attribute m (repeated attributes add up; FP32,
+        // within 2^-19 of the exact sum for <= 32 terms, well inside the filter's bound)
+        float a[kBf16MaxD] = {0.0f};
+        for (uint32_t m = 0; m < q[j].qq; m++) a[q[j].attr[m]] += q[j].w[m];
+        bf16_pack_query(a, h->d, (uint32_t)j, habf);
+        q[j].err = bf16_error_bound(q[j], h->absmax, kblk);
+        q[j].maxkey = score_bound_key(q[j], h->colmax, h->colmin);
+      }
+    });
+    if ((st = ensure(h->b_abf_act, abf_bytes)) != TOPK_OK) return st;
+    if ((st = ensure(h->b_amap, (nq + 1) * sizeof(uint32_t))) != TOPK_OK) return st;
     // survivor records: one log per filter CTA
     const FilterPlan fp = plan_bf16_filter(nqq_all, 0, h->n, h->d, h->num_sms, h->batch_qt);
     log_ctas = fp.grid;
-    if ((st = ensure(h->b_log, log_ctas * kBf16LogCap * 8 * sizeof(uint4))) != TOPK_OK) return st;
-    if ((st = ensure(h->b_logh, log_ctas * kBf16LogCap * sizeof(uint2))) != TOPK_OK) return st;
-    CK(cudaMemcpyAsync(h->b_abf.p, habf.data(), habf.size(), cudaMemcpyHostToDevice, s));
-    CK(cudaMemsetAsync(h->b_err.p, 0, sizeof(uint32_t), s));
-    CK(cudaStreamSynchronize(s));  // habf is pageable and goes out of scope
-  }
-  if ((st = ensure(h->b_q, nq * sizeof(BatchQuery))) != TOPK_OK) return st;
-  if ((st = ensure(h->b_st, nq * sizeof(BatchState))) != TOPK_OK) return st;
-  if ((st = ensure(h->b_best, best_total * sizeof(uint2))) != TOPK_OK) return st;
-  if ((st = ensure(h->b_cand, cand_total * sizeof(uint2))) != TOPK_OK) return st;
-  if ((st = ensure(h->b_ids, nq * kmax * sizeof(uint64_t))) != TOPK_OK) return st;
-  if ((st = ensure(h->b_scores, nq * kmax * sizeof(float))) != TOPK_OK) return st;
-  if ((st = ensure(h->b_count, nq * sizeof(uint32_t))) != TOPK_OK) return st;
-  if ((st = ensure(h->b_thr, nq * sizeof(float))) != TOPK_OK) return st;
-  if (!h->b_ev0) CK(cudaEventCreate(&h->b_ev0));
-  if (!h->b_ev1) CK(cudaEventCreate(&h->b_ev1));
-  // the plain FP32 scorer takes the queries ordered by attribute count, then by
-  // attribute list: a warp's lanes then run the same number of steps and mostly read
-  // the same rows of the staged tile at each step (shared-memory broadcast)
-  uint32_t *dorder = nullptr;
-  if (!use_bf16) {
-    std::vector<uint32_t> order(nq);
+    if ((st = ensure(h->b_log, log_ctas * rec_cap * 8 * sizeof(uint4))) != TOPK_OK) return st;
+    if ((st = ensure(h->b_logh, log_ctas * rec_cap * sizeof(uint2))) != TOPK_OK) return st;
+  } else {
+    // the plain FP32 scorer takes the queries ordered by attribute count, then by
+    // attribute list: a warp's lanes then run the same number of steps and mostly read
+    // the same rows of the staged tile at each step (shared-memory broadcast)
+    uint32_t *order = reinterpret_cast<uint32_t *>(h->hb_in.p + in_abf);
     for (uint32_t j = 0; j < (uint32_t)nq; j++) order[j] = j;
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) {
+    std::stable_sort(order, order + nq, [&](uint32_t a, uint32_t b) {
       if (q[a].qq != q[b].qq) return q[a].qq < q[b].qq;
       return std::memcmp(q[a].attr, q[b].attr, q[a].qq) < 0;
     });
-    if ((st = ensure(h->b_order, nq * sizeof(uint32_t))) != TOPK_OK) return st;
-    dorder = static_cast<uint32_t *>(h->b_order.p);
-    CK(cudaMemcpyAsync(dorder, order.data(), nq * 4, cudaMemcpyHostToDevice, s));
-    CK(cudaStreamSynchronize(s));  // `order` is pageable and goes out of scope
   }
-  BatchQuery *dq = static_cast<BatchQuery *>(h->b_q.p);
-  BatchState *dst = static_cast<BatchState *>(h->b_st.p);
+  std::memcpy(h->hb_in.p, q.data(), nq * sizeof(BatchQuery));
+  if ((st = ensure(h->b_best, best_total * sizeof(uint2))) != TOPK_OK) return st;
+  if ((st = ensure(h->b_cand, cand_total * sizeof(uint2))) != TOPK_OK) return st;
+  // outputs: ids | scores | counts | thresholds | states | active queries per chunk | error
+  // word, the hybrid lists' progress and work counter, their counts -- copied up to here --
+  // and the lists themselves
+  const size_t o_sc = up(best_total * 8), o_cnt = o_sc + up(best_total * 4), o_thr = o_cnt + up(nq * 4),
+               o_st = o_thr + up(nq * 4), o_act = o_st + up(nq * sizeof(BatchState)),
+               o_err = o_act + kMaxChunkLog * sizeof(uint32_t), o_sw = o_err + 4 * sizeof(uint32_t),
+               out_bytes = o_sw + 2 * sizeof(uint32_t);
+  if ((st = ensure(h->b_out, out_bytes + 2 * nq * sizeof(uint32_t))) != TOPK_OK) return st;
+  if (!h->b_ev0) CK(cudaEventCreate(&h->b_ev0));
+  if (!h->b_ev1) CK(cudaEventCreate(&h->b_ev1));
+  unsigned char *din = static_cast<unsigned char *>(h->b_in.p), *dout = static_cast<unsigned char *>(h->b_out.p);
+  BatchQuery *dq = reinterpret_cast<BatchQuery *>(din);
+  uint8_t *dabf = din + in_abf;
+  uint32_t *dorder = use_bf16 ? nullptr : reinterpret_cast<uint32_t *>(din + in_abf);
+  uint64_t *dids = reinterpret_cast<uint64_t *>(dout);
+  float *dscores = reinterpret_cast<float *>(dout + o_sc), *dthr = reinterpret_cast<float *>(dout + o_thr);
+  uint32_t *dcount = reinterpret_cast<uint32_t *>(dout + o_cnt), *dact = reinterpret_cast<uint32_t *>(dout + o_act);
+  BatchState *dst = reinterpret_cast<BatchState *>(dout + o_st);
+  uint32_t *derr = reinterpret_cast<uint32_t *>(dout + o_err);
   uint2 *dbest = static_cast<uint2 *>(h->b_best.p);
   uint2 *dcand = static_cast<uint2 *>(h->b_cand.p);
   const uint32_t nqq = (uint32_t)nq;
-  CK(cudaMemcpyAsync(dq, q.data(), nq * sizeof(BatchQuery), cudaMemcpyHostToDevice, s));
-  CK(cudaMemsetAsync(dst, 0, nq * sizeof(BatchState), s));
   if (use_learned) {
     if ((st = ensure(h->b_feat, nq * feature_dim(h->d) * sizeof(float))) != TOPK_OK) return st;
     if ((st = ensure(h->b_pred, nq * sizeof(float))) != TOPK_OK) return st;
   }
+  // (the pinned inputs are free again at the batch's one synchronisation)
+  CK(cudaMemcpyAsync(din, h->hb_in.p, in_bytes, cudaMemcpyHostToDevice, s));
+  CK(cudaMemsetAsync(dout + o_st, 0, out_bytes - o_st, s));  // states, counts and words
   const uint64_t boot = std::min<uint64_t>(h->n, h->batch_boot);
   const uint64_t r_start = use_learned ? 0 : boot;
   // Chunks double the rows seen; for a small batch they quadruple them: a chunk costs
@@ -903,20 +948,10 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   // Hybrid batch under the filter: a query for which the filter passes too much
   // (scores tied or dense at its threshold) moves to the exact FP32 scorer for the
   // rest of the batch.  The reduce lists it: sw[0] counts the moved queries (list A at
-  // sw + 2), sw[1] those whose last chunk was discarded (list B at sw + 2 + nq), and
-  // sw[2 + 2nq] is how far list B has been answered again, sw[3 + 2nq] the scorer's
-  // work counter.  The scorer reads the counts on the device, so the host never waits
-  // inside the batch.
-  uint32_t *dsw = nullptr, *dredo = nullptr, *dwork = nullptr;
-  if (use_bf16) {
-    if ((st = ensure(h->b_sw, (4 + 2 * nq) * sizeof(uint32_t))) != TOPK_OK) return st;
-    dsw = static_cast<uint32_t *>(h->b_sw.p);
-    dredo = dsw + 2 + 2 * nq;
-    dwork = dredo + 1;
-    CK(cudaMemsetAsync(dsw, 0, 2 * sizeof(uint32_t), s));
-    CK(cudaMemsetAsync(dredo, 0, sizeof(uint32_t), s));
-  }
-  uint32_t hsw[2] = {0, 0};
+  // sw + 2), sw[1] those whose last chunk was discarded (list B at sw + 2 + nq); dredo is
+  // how far list B has been answered again, dwork the scorer's work counter.  The scorer
+  // reads the counts on the device, so the host never waits inside the batch.
+  uint32_t *dsw = use_bf16 ? reinterpret_cast<uint32_t *>(dout + o_sw) : nullptr, *dredo = derr + 1, *dwork = derr + 2;
   uint32_t chunk = 0;  // chunk index while the launches are issued
   // the device work of the batch, from the first threshold to the results
   auto issue = [&]() -> int {
@@ -942,14 +977,13 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
       // the queries still served by the filter, as compact tiles
       uint32_t *amap = static_cast<uint32_t *>(h->b_amap.p);
       // the chunk's active count also goes to its slot of the per-batch record
-      uint32_t *logslot = chunk < kMaxChunkLog ? amap + nq + 1 + chunk : nullptr;
+      uint32_t *logslot = chunk < kMaxChunkLog ? dact + chunk : nullptr;
       ++chunk;
-      CK(launch_batch_active(dq, dst, nqq, h->d, static_cast<const uint8_t *>(h->b_abf.p),
-                             static_cast<uint8_t *>(h->b_abf_act.p), amap, amap + nq, logslot, s));
+      CK(launch_batch_active(dq, dst, nqq, h->d, dabf, static_cast<uint8_t *>(h->b_abf_act.p), amap, amap + nq,
+                             logslot, s));
       CK(launch_bf16_filter(fp, static_cast<const uint8_t *>(h->xbf.p), static_cast<const uint8_t *>(h->b_abf_act.p),
                             amap, amap + nq, r, e, dq, dst, dcand, static_cast<uint4 *>(h->b_log.p),
-                            static_cast<uint2 *>(h->b_logh.p), kBf16LogCap, h->wait_limit,
-                            static_cast<uint32_t *>(h->b_err.p), s));
+                            static_cast<uint2 *>(h->b_logh.p), rec_cap, h->wait_limit, derr, s));
       // this chunk for every moved query; the previous one again for those that discarded it
       CK(launch_batch_score_fp32_list(h->table, h->ld, h->d, r, e, dq, dst, dcand, dsw + 2, dsw, nullptr, dwork, qmax,
                                       true, h->num_sms, s));
@@ -969,9 +1003,7 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
     CK(launch_batch_reduce(h->table, h->ld, dq, nqq, dst, dbest, dcand, kmax, capmax, use_bf16, dsw, s));
   }
   // results compact (each query's at its best_off), so the download moves sum(k) entries
-  CK(launch_batch_finish(dq, nqq, dst, dbest, kmax, static_cast<uint64_t *>(h->b_ids.p),
-                         static_cast<float *>(h->b_scores.p), 0, static_cast<uint32_t *>(h->b_count.p),
-                         static_cast<float *>(h->b_thr.p), s));
+  CK(launch_batch_finish(dq, nqq, dst, dbest, kmax, dids, dscores, 0, dcount, dthr, s));
   return TOPK_OK;
   };
   // Captured into a CUDA graph once per shape and replayed: the key holds every
@@ -980,10 +1012,10 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   // the stream uploaded and cleared before it.
   std::vector<uint64_t> key = {nq, kmax, capmax, qmax, use_bf16, use_learned, h->n, h->d, h->ld, boot,
                                (uint64_t)h->num_sms, log_ctas, h->wait_limit, h->num_parts, h->batch_qt,
-                               quadruple};
-  const void *key_ptrs[] = {h->table, dq, dst, dbest, dcand, h->b_ids.p, h->b_scores.p, h->b_count.p,
-                            h->b_thr.p, h->xbf.p, h->b_abf.p, h->b_log.p, h->b_logh.p, h->b_err.p, h->b_sw.p,
-                            h->b_feat.p, h->b_pred.p, h->pstats, h->mlp, h->b_abf_act.p, h->b_amap.p, dorder};
+                               quadruple, rec_cap};
+  const void *key_ptrs[] = {h->table, dq, dabf, dorder, dst, dbest, dcand, dids, dscores, dcount, dthr, dact, derr,
+                            dsw, h->xbf.p, h->b_log.p, h->b_logh.p, h->b_feat.p, h->b_pred.p, h->pstats, h->mlp,
+                            h->b_abf_act.p, h->b_amap.p};
   for (const void *ptr : key_ptrs) key.push_back((uint64_t)(uintptr_t)ptr);
   {
     uint32_t mb;
@@ -1020,35 +1052,28 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   CK(cudaEventRecord(h->b_ev0, s));
   CK(cudaGraphLaunch(gr->exec, s));
   CK(cudaEventRecord(h->b_ev1, s));
-  // results through the handle's pinned buffers (grown once), then into the caller's
-  // arrays before anything below runs a nested batch that reuses them
-  const size_t res_bytes = (size_t)best_total * 12;
-  if (h->hb_bytes < res_bytes) {
-    if (h->hb_res) cudaFreeHost(h->hb_res);
-    h->hb_res = nullptr;
-    h->hb_bytes = 0;
-    if (cudaHostAlloc(&h->hb_res, res_bytes, cudaHostAllocDefault) != cudaSuccess)
-      return fail(TOPK_ERR_OOM, "pinned result buffer of %zu bytes", res_bytes);
-    h->hb_bytes = res_bytes;
+  // everything it reports in one copy through the handle's pinned buffer, then into the
+  // caller's arrays (and the vectors) before anything below runs a nested batch that
+  // reuses it (pinned while the device works: 24 MB take about 10 ms to pin)
+  if ((st = ensure(h->hb_out, out_bytes)) != TOPK_OK) {
+    CK(cudaStreamSynchronize(s));
+    return st;
   }
-  uint64_t *hid = static_cast<uint64_t *>(h->hb_res);
-  float *hsc = reinterpret_cast<float *>(hid + best_total);
-  std::vector<float> hth(nq);
-  std::vector<uint32_t> hcnt(nq);
-  std::vector<BatchState> hst(nq);
-  CK(cudaMemcpyAsync(hid, h->b_ids.p, best_total * 8, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(hsc, h->b_scores.p, best_total * 4, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(hcnt.data(), h->b_count.p, nq * 4, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(hth.data(), h->b_thr.p, nq * 4, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(hst.data(), dst, nq * sizeof(BatchState), cudaMemcpyDeviceToHost, s));
-  uint32_t herr = 0;
-  std::vector<uint32_t> hact(kMaxChunkLog, 0);
-  if (use_bf16) CK(cudaMemcpyAsync(&herr, h->b_err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  if (use_bf16)
-    CK(cudaMemcpyAsync(hact.data(), static_cast<uint32_t *>(h->b_amap.p) + nq + 1, kMaxChunkLog * 4,
-                       cudaMemcpyDeviceToHost, s));
-  if (use_bf16) CK(cudaMemcpyAsync(hsw, dsw, sizeof(hsw), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(h->hb_out.p, dout, out_bytes, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
+  const unsigned char *ho = h->hb_out.p;
+  const uint64_t *hid = reinterpret_cast<const uint64_t *>(ho);
+  const float *hsc = reinterpret_cast<const float *>(ho + o_sc);
+  std::vector<float> hth(nq);
+  std::vector<uint32_t> hcnt(nq), hact(kMaxChunkLog);
+  std::vector<BatchState> hst(nq);
+  std::memcpy(hth.data(), ho + o_thr, nq * 4);
+  std::memcpy(hcnt.data(), ho + o_cnt, nq * 4);
+  std::memcpy(hst.data(), ho + o_st, nq * sizeof(BatchState));
+  std::memcpy(hact.data(), ho + o_act, kMaxChunkLog * 4);
+  uint32_t herr, hsw[2];
+  std::memcpy(&herr, ho + o_err, 4);
+  std::memcpy(hsw, ho + o_sw, sizeof(hsw));
   if (herr) return fail(TOPK_ERR_TIMEOUT, "BF16 filter: a bounded device-side wait ran out");
   // MMA work of the filter: every served query tile (128 queries) against every object
   // tile of the chunk, three passes of 2 * 16 flops per (query, object)
@@ -1065,11 +1090,14 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   if (use_bf16)
     for (uint64_t j = 0; j < nq; j++)
       if (!(hst[j].flags & kFlagFp32) && hst[j].thr != 0u && hst[j].thr > q[j].maxkey) ++retired_total;
-  for (uint64_t j = 0; j < nq; j++) {  // queries answered again below overwrite theirs
-    const uint32_t c = std::min<uint32_t>(hcnt[j], (uint32_t)std::min<uint64_t>(kmax, kstride));
-    std::memcpy(ids + j * kstride, hid + q[j].best_off, (size_t)c * 8);
-    std::memcpy(scores + j * kstride, hsc + q[j].best_off, (size_t)c * 4);
-  }
+  // (queries answered again below overwrite theirs)
+  in_parallel(nq, best_total * 12, [&](uint64_t j0, uint64_t j1) {
+    for (uint64_t j = j0; j < j1; j++) {
+      const uint32_t c = std::min<uint32_t>(hcnt[j], (uint32_t)std::min<uint64_t>(kmax, kstride));
+      std::memcpy(ids + j * kstride, hid + q[j].best_off, (size_t)c * 8);
+      std::memcpy(scores + j * kstride, hsc + q[j].best_off, (size_t)c * 4);
+    }
+  });
   float ms = 0;
   CK(cudaEventElapsedTime(&ms, h->b_ev0, h->b_ev1));
   uint64_t cands = 0;
