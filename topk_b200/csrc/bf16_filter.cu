@@ -39,7 +39,7 @@
 //              no dependent work while the accumulator is held);
 //   warp 16    producer: bulk-copies (cp.async.bulk, no tensor map, no multicast)
 //              the CTA's query tiles once and object tiles into a 5-stage ring;
-//   warp 17    allocates the 512 TMEM columns; lane 0 issues the MMAs into two
+//   warp 17    allocates the 512 TMEM columns; an elected lane issues the MMAs into two
 //              accumulators of 256 columns, one per epilogue group (at N=256 an MMA
 //              takes longer to run than to issue, so one thread keeps the tensor
 //              core busy).
@@ -117,6 +117,13 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t adesc, uint64_t
 __device__ __forceinline__ void tc_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
+}
+
+// One lane of the (converged) warp, the same at every call.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t yes;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xFFFFFFFF;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(yes));
+  return yes != 0;
 }
 
 #define TOPK_R8(i) "=r"(v[i]), "=r"(v[i + 1]), "=r"(v[i + 2]), "=r"(v[i + 3]), "=r"(v[i + 4]), "=r"(v[i + 5]), \
@@ -285,41 +292,50 @@ __global__ void __launch_bounds__(kFThreads, 1) bf16_filter_kernel(const FilterA
     }
   } else if (warp == kMmaWarp) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      bool ok = fwait(qfull, 0, limit, abort_flag);
-      uint64_t it = 0;
-      uint32_t seq = 0;
-      for (uint64_t t = tb; ok && t < te; ++t, ++it) {
-        const uint32_t s = (uint32_t)(it % stages);
-        if (!fwait(full + s, (uint32_t)((it / stages) & 1), limit, abort_flag)) break;
+    // The whole warp runs the loop and one elected lane issues, so descriptors and counters
+    // are warp-uniform.  With the loop inside one lane's branch the issue of a pair took
+    // longer than its MMAs (4096 queries on 2^25 rows: 16.9 ms a batch; so 15.1).
+    const bool leader = elect_one();
+    bool ok = __all_sync(0xFFFFFFFFu, fwait(qfull, 0, limit, abort_flag));
+    uint32_t s = 0, sph = 0, seq = 0;
+    const uint64_t qd0 = smem_desc(smem_u32(sq)), od0 = smem_desc(smem_u32(so));
+    for (uint64_t t = tb; ok && t < te; ++t) {
+      if (!__all_sync(0xFFFFFFFFu, fwait(full + s, sph, limit, abort_flag))) break;
+      const uint64_t od = od0 + s * (otile >> 4);
+      uint64_t qd = qd0;
+      for (uint32_t i = 0; i < nqt; ++i, ++seq, qd += qtile >> 4) {
+        const uint32_t buf = seq % kAcc;
+        if (seq >= kAcc && !__all_sync(0xFFFFFFFFu, fwait(acce + buf, (seq / kAcc - 1) & 1u, limit, abort_flag))) {
+          ok = false;
+          break;
+        }
         tc_fence_after();
-        const uint32_t os = smem_u32(so + (size_t)s * otile);
-        for (uint32_t i = 0; i < nqt; ++i, ++seq) {
-          const uint32_t buf = seq % kAcc;
-          if (seq >= kAcc && !fwait(acce + buf, (seq / kAcc - 1) & 1u, limit, abort_flag)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t qsa = smem_u32(sq + (size_t)i * qtile);
-          const uint32_t d = tmem + buf * kOTile;
+        const uint32_t d = tmem + buf * kOTile;
+        if (leader) {
 #pragma unroll
           for (uint32_t kb = 0; kb < KB; ++kb) {
-            const uint64_t xhi = smem_desc(os + kb * kOTileBytes), xlo = smem_desc(os + kb * kOTileBytes + kOTileBytes / 2);
-            const uint64_t ahi = smem_desc(qsa + kb * kQTileBytes), alo = smem_desc(qsa + kb * kQTileBytes + kQTileBytes / 2);
+            const uint64_t xhi = od + kb * (kOTileBytes >> 4), xlo = xhi + (kOTileBytes >> 5);
+            const uint64_t ahi = qd + kb * (kQTileBytes >> 4), alo = ahi + (kQTileBytes >> 5);
             tc_mma(d, ahi, xhi, kb ? 1u : 0u);
             tc_mma(d, ahi, xlo, 1u);
             tc_mma(d, alo, xhi, 1u);
           }
           tc_commit(accf + buf);
         }
-        if (!ok) break;
-        tc_commit(empty + s);  // the stage is free once these MMAs have read it
+        __syncwarp();
       }
-      // TMEM is freed below: every issued MMA must have completed first
-      tc_commit(mdone);
-      if (!mbar_wait_bounded(mdone, 0, limit)) *abort_flag = 1u;
+      if (!ok) break;
+      if (leader) tc_commit(empty + s);  // the stage is free once these MMAs have read it
+      __syncwarp();
+      if (++s == stages) {
+        s = 0;
+        sph ^= 1u;
+      }
     }
+    // TMEM is freed below: every issued MMA must have completed first
+    if (leader) tc_commit(mdone);
+    __syncwarp();
+    if (!mbar_wait_bounded(mdone, 0, limit)) *abort_flag = 1u;
   } else {
     // ---------------------------------------------------------------- epilogue
     // warps kGroupWarps*g.. drain the pairs seq = g mod kDrainGroups, pair seq in
