@@ -213,13 +213,16 @@ __host__ __device__ constexpr uint32_t scan_vote_tiles(int qq, bool part) {
   return (qq >= 1 && qq <= 2 && !part) ? 2u : 1u;
 }
 
-// CTAs per SM the register budget is sized for: few queried columns need little data
-// in flight and gain from more CTAs (6: 42 registers); more columns need their loads
+// CTAs per SM the register budget is sized for: one queried column needs little data
+// in flight and gains from more CTAs (6: 42 registers); more columns need their loads
 // in flight without spills (5: 51 registers up to 8 columns, 4: 64 above).
-// Partition mode runs at most 4 CTAs per SM, so it has their registers.
+// Partition mode runs at most 4 CTAs per SM, so it has their registers.  Two attributes in
+// id order take 48 registers at 5 CTAs; at 6 the loop spilled (2^28 rows, independent, us
+// at k = 16 / 1024 / 4096: 430 / 534 / 1110 with 6, 400 / 448 / 819 with 5; only k = 1 is
+// slower than with 6 CTAs and no epochs, 395 against 383).
 template <int QQ, bool PART>
 constexpr int scan_min_blocks() {
-  return PART ? 4 : (QQ >= 1 && QQ <= 2) ? 6 : (QQ >= 3 && QQ <= 8) ? 5 : 4;
+  return PART ? 4 : QQ == 1 ? 6 : (QQ >= 2 && QQ <= 8) ? 5 : 4;
 }
 
 // ---------------------------------------------------------------- results
