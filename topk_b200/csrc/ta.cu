@@ -11,8 +11,9 @@
 // seen-bitmap (each object is scored once), scores it exactly in the reference order
 // and appends it when it beats the current k-th; a second one selects the best k of the
 // appended keys and the running top k through a histogram of the scores.  4M rows x 8,
-// q = 4, k = 64, one block of depth: 194 us with a radix sort of the keys, 48 us so.  The bound of the unseen objects after depth i is
-// the reference's threshold with each weight's sign respected (w < 0 takes the attribute's minimum), in the same FP32
+// q = 4, k = 64, one block of depth: 194 us with a radix sort of the keys, 48 us so.
+// The bound of the unseen objects after depth i is the reference's threshold with each
+// weight's sign respected (w < 0 takes the attribute's minimum), in the same FP32
 // operations, so it bounds their scores exactly; the walk stops when the k-th score is
 // strictly above it, so no unseen object can tie the k-th with a lower id.  Results are
 // those of the full scan.
