@@ -364,7 +364,9 @@ __device__ __noinline__ KthBound block_kth_bound(const uint2 *src, uint32_t np, 
       b.count = above + hist[13];
       if (s == 0 || b.count <= k + k / 4u + 32u) break;  // uniform
       lo = bound;
-      hi = min(hi, bound + ((1u << s) - 1u));
+      // (bound <= hi: the bin holds a value.  As a sum, the bin's end may lie past 2^32 -- the
+      // ~ids of the first rows -- and a wrapped hi would let the zeros of no entry in.)
+      hi = bound + min(hi - bound, (1u << s) - 1u);
       __syncthreads();  // hist has been read
     }
     if (part == 0) b.key = bound;
