@@ -543,7 +543,9 @@ __device__ __noinline__ void coordinate(const ScanParams &p, SmemCtl *ctl, uint2
       b = block_kth_bound<kScanThreads>(p.pub, np, p.k, stage, stage_cap, bins, hist);
     }
     const uint64_t least = b.key ? b.word() : 0ull;
-    const uint32_t room = stage_cap / 3u;  // (an entry and its place in the order: 3 words)
+    // (an entry and its place in the order take 3 words; the select for many equal keys
+    // below writes its k entries behind `cap`, and must not meet those it reads)
+    const uint32_t room = min(stage_cap / 3u, p.cap);
     if (!few && hid != ~0ull) {  // the entries at or above the bound (no bound: all of them)
       for (uint32_t base = 0; base < np; base += kScanThreads * 8u) {  // uniform trip count
         uint2 e[8];
