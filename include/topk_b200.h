@@ -400,8 +400,10 @@ int topk_set_scan_tuning(topk_table_t h, uint32_t max_ctas_per_sm);
 
 /* Test entry (no reference counterpart): mode 1 makes the next fused scans wait,
  * before any copy is issued, on a barrier that nothing completes, so the bounded
- * wait runs out and the call returns TOPK_ERR_TIMEOUT; 0 turns it off.  Host-side
- * fault injection: no GPU fault, the context stays usable. */
+ * wait runs out and the call returns TOPK_ERR_TIMEOUT; mode 2 makes the next batches
+ * take the allocation of the tensor-core filter's records for failed (TOPK_ERR_OOM
+ * where the table needs the filter's memory, else the FP32 scorer answers); 0 turns
+ * it off.  Host-side fault injection: no GPU fault, the context stays usable. */
 int topk_set_fault_injection(topk_table_t h, int mode);
 
 /* Methods of topk_query_batch (no reference counterpart; results are identical). */
@@ -416,8 +418,9 @@ int topk_set_fault_injection(topk_table_t h, int mode);
 #define TOPK_BATCH_BF16 3  /* BF16 tensor-core filter (tcgen05) with a per-query error
                             * bound; candidates rescored exactly in FP32.  Applies to
                             * d <= 16, and from 2^17 rows on to d <= 64 (where the split
-                            * copy takes at most half of the free memory), with finite
-                            * table values and weights of magnitude <= 2^60; other
+                            * copy and the filter's records take at most half of the free
+                            * memory; they are given back when memory runs out), with
+                            * finite table values and weights of magnitude <= 2^60; other
                             * batches run TOPK_BATCH_FP32.  Hybrid: a
                             * query for which the filter passes too much (tied or dense
                             * scores at its threshold: more than 2k + 2048 candidates in

@@ -640,9 +640,12 @@ int run_pruned(topk_table_t h, uint64_t k, uint32_t qq, const float *weights, co
 int ensure(topk_table_s::DevBuf &b, size_t bytes) {
   if (b.bytes >= bytes) return TOPK_OK;
   cudaFree(b.p);
-  b.p = nullptr;
-  b.bytes = 0;
-  CK(cudaMalloc(&b.p, bytes));
+  b = topk_table_s::DevBuf{};
+  if (const cudaError_t e = cudaMalloc(&b.p, bytes); e != cudaSuccess) {
+    (void)cudaGetLastError();  // (not for the next launch to report)
+    b.p = nullptr;
+    return cuda_fail(e, "batch buffer");
+  }
   b.bytes = bytes;
   return TOPK_OK;
 }
@@ -714,23 +717,45 @@ void table_changed(topk_table_t h) {
 // and 48-term sums stay far from FP32 overflow, and bf16 rounding cannot overflow.
 constexpr float kBf16MaxAbs = 1.152921504606846976e18f;  // 2^60
 
+// What the filter holds of a table wider than one K block is optional (the FP32 scorer
+// serves such a table as well): given back when memory runs out elsewhere.  False when
+// there was none.  Caller holds batch_mu.
+bool drop_wide_filter(topk_table_t h) {
+  if (h->d <= kBf16K || !(h->xbf.p || h->b_log.p)) return false;
+  (void)cudaGetLastError();  // the failed allocation's
+  cudaStreamSynchronize(h->primary->stream);
+  for (topk_table_s::DevBuf *b : {&h->xbf, &h->b_log, &h->b_logh}) {
+    cudaFree(b->p);
+    *b = topk_table_s::DevBuf{};
+  }
+  h->xbf_usable = false;
+  h->xbf_version = 0;
+  return true;
+}
+
+bool free_wide_filter(topk_table_t h) {
+  std::lock_guard<std::mutex> lk(h->batch_mu);
+  return drop_wide_filter(h);
+}
+
 // Build (or reuse) the BF16 split of the table; caller holds batch_mu.  Sets
 // h->xbf_usable: false for tables wider than 64 or holding non-finite or huge values, and
-// for tables wider than 16 (which the FP32 scorer serves as well) when their split would
-// take more than half of the free memory.
-int ensure_bf16_table(topk_table_t h, cudaStream_t s) {
+// for tables wider than 16 (which the FP32 scorer serves as well) while their split and the
+// batch's `log_bytes` of survivor records would take more than half of the free memory.
+int ensure_bf16_table(topk_table_t h, size_t log_bytes, cudaStream_t s) {
   if (h->xbf_version == h->data_version) return TOPK_OK;
   h->xbf_usable = false;
   const uint64_t bytes = bf16_table_bytes(h->n, h->d);
-  bool fits = h->d <= kBf16MaxD;
-  if (fits && h->d > kBf16K && h->xbf.bytes < bytes) {
-    size_t avail = 0, total = 0;
-    CK(cudaMemGetInfo(&avail, &total));
-    fits = bytes <= (avail + h->xbf.bytes) / 2;
-  }
-  if (!fits) {
+  if (h->d > kBf16MaxD) {
     h->xbf_version = h->data_version;
     return TOPK_OK;
+  }
+  if (h->d > kBf16K && h->xbf.bytes < bytes) {
+    size_t avail = 0, total = 0;
+    CK(cudaMemGetInfo(&avail, &total));
+    const size_t held = h->xbf.bytes + h->b_log.bytes + h->b_logh.bytes;
+    if (bytes + std::max<size_t>(log_bytes, h->b_log.bytes + h->b_logh.bytes) > (avail + held) / 2)
+      return TOPK_OK;  // (asked again by the next batch: memory may be free by then)
   }
   int st;
   if ((st = ensure(h->xbf, bytes)) != TOPK_OK) return st;
@@ -837,14 +862,22 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
     return fail(TOPK_ERR_UNSUPPORTED, "batch too large: split it");
   int st;
   cudaStream_t s = h->primary->stream;
+  const uint32_t nqq_all = (uint32_t)nq;
+  // Survivor records per filter CTA: a chunk passes about 3k candidates a query, and an
+  // eighth of the batch's may fall to one CTA before queries move to the FP32 scorer.  (At
+  // kBf16LogCap the logs take 660 MB, most of a small batch's first call.)
+  const uint32_t rec_cap = (uint32_t)std::min<uint64_t>(kBf16LogCap, (4096 + 3 * best_total / 8) / 16 * 16);
+  auto log_bytes = [&](uint64_t ctas) { return ctas * rec_cap * 8 * sizeof(uint4); };
+  auto logh_bytes = [&](uint64_t ctas) { return ctas * rec_cap * sizeof(uint2); };
   // scorer: the BF16 tensor-core filter where the table and every weight allow it
   bool use_bf16 = false;
   const uint32_t kblk = bf16_kblocks(h->d);
   const bool small_wide = h->d > kBf16K && h->n < kWideFilterRows;
   if (!force_fp32 && !small_wide && (h->batch_method == TOPK_BATCH_AUTO || h->batch_method == TOPK_BATCH_BF16 ||
                       h->batch_method == TOPK_BATCH_LEARNED)) {
-    if ((st = ensure_bf16_table(h, s)) != TOPK_OK) return st;
-    use_bf16 = h->xbf_usable && nq <= 0xFFFFFFFFull;
+    const uint64_t ctas = h->d <= kBf16MaxD ? plan_bf16_filter(nqq_all, 0, h->n, h->d, h->num_sms, h->batch_qt).grid : 0;
+    if ((st = ensure_bf16_table(h, log_bytes(ctas) + logh_bytes(ctas), s)) != TOPK_OK) return st;
+    use_bf16 = h->xbf_usable && h->xbf_version == h->data_version && nq <= 0xFFFFFFFFull;
     // AUTO: scores too dense around the thresholds for the filter on this table
     if (h->batch_method == TOPK_BATCH_AUTO && h->auto_fp32_version == h->data_version) use_bf16 = false;
     for (uint64_t j = 0; use_bf16 && j < nq; j++)
@@ -859,11 +892,6 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
                   feature_dim(h->d) <= kMlpMaxIn && h->num_parts <= kMaxFeatureParts && nq <= 0x7FFFFFFFull;
   }
   h->last_batch_method = use_learned ? TOPK_BATCH_LEARNED : use_bf16 ? TOPK_BATCH_BF16 : TOPK_BATCH_FP32;
-  const uint32_t nqq_all = (uint32_t)nq;
-  // Survivor records per filter CTA: a chunk passes about 3k candidates a query, and an
-  // eighth of the batch's may fall to one CTA before queries move to the FP32 scorer.  (At
-  // kBf16LogCap the logs take 660 MB, most of a small batch's first call.)
-  const uint32_t rec_cap = (uint32_t)std::min<uint64_t>(kBf16LogCap, (4096 + 3 * best_total / 8) / 16 * 16);
   uint64_t log_ctas = 0;
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   // inputs: descriptors | query tiles of the filter, or the FP32 scorer's query order
@@ -890,8 +918,9 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
     // survivor records: one log per filter CTA
     const FilterPlan fp = plan_bf16_filter(nqq_all, 0, h->n, h->d, h->num_sms, h->batch_qt);
     log_ctas = fp.grid;
-    if ((st = ensure(h->b_log, log_ctas * rec_cap * 8 * sizeof(uint4))) != TOPK_OK) return st;
-    if ((st = ensure(h->b_logh, log_ctas * rec_cap * sizeof(uint2))) != TOPK_OK) return st;
+    if (h->fault_mode == 2) return fail(TOPK_ERR_OOM, "batch buffer: injected");
+    if ((st = ensure(h->b_log, log_bytes(log_ctas))) != TOPK_OK) return st;
+    if ((st = ensure(h->b_logh, logh_bytes(log_ctas))) != TOPK_OK) return st;
   } else {
     // the plain FP32 scorer takes the queries ordered by attribute count, then by
     // attribute list: a warp's lanes then run the same number of steps and mostly read
@@ -1188,6 +1217,17 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   return TOPK_OK;
 }
 
+// run_batch; where memory runs out with a filter that the table can do without, again
+// without it (the call's outputs are written over).
+int run_batch_fit(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *qqs, const float *weights,
+                  uint64_t wstride, const uint8_t *attrs, uint64_t astride, uint64_t *ids, float *scores,
+                  uint64_t kstride, uint64_t *counts, float *thresholds) {
+  const int st = run_batch(h, nq, ks, qqs, weights, wstride, attrs, astride, ids, scores, kstride, counts, thresholds);
+  if (st != TOPK_ERR_OOM || !drop_wide_filter(h)) return st;
+  return run_batch(h, nq, ks, qqs, weights, wstride, attrs, astride, ids, scores, kstride, counts, thresholds, true,
+                   true);
+}
+
 }  // namespace
 
 extern "C" {
@@ -1350,7 +1390,9 @@ int topk_build_lists(topk_table_t h) {
   ta_lists_free(h->ta);
   h->ta = nullptr;
   std::string msg;
-  const int rc = ta_lists_build(&h->ta, h->table, h->ld, h->d, h->n, h->num_sms, &msg);
+  int rc = ta_lists_build(&h->ta, h->table, h->ld, h->d, h->n, h->num_sms, &msg);
+  if (rc == TOPK_ERR_OOM && free_wide_filter(h))
+    rc = ta_lists_build(&h->ta, h->table, h->ld, h->d, h->n, h->num_sms, &msg);
   if (rc != TOPK_OK) return fail(rc, "%s", msg.c_str());
   h->ta_version = h->data_version;
   return TOPK_OK;
@@ -1596,7 +1638,7 @@ int topk_query_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint
   }
   std::lock_guard<std::mutex> lk(h->batch_mu);
   if (h->batch_method != TOPK_BATCH_LOOP && batchable)
-    return run_batch(h, nq, ks, qqs, weights, wstride, attrs, astride, ids, scores, kstride, counts, thresholds);
+    return run_batch_fit(h, nq, ks, qqs, weights, wstride, attrs, astride, ids, scores, kstride, counts, thresholds);
   h->last_batch_ms = 0;
   h->last_batch_fallbacks = 0;
   h->last_batch_switched = 0;
@@ -1806,12 +1848,21 @@ int topk_build_partitions_ordered(topk_table_t h, uint32_t part_rows, int order)
   }
   h->num_parts = 0;
   cudaError_t e = cudaSuccess;
-  if (!h->pids) e = cudaMalloc(&h->pids, h->n * sizeof(uint32_t));
+  auto get = [&](auto **p, size_t bytes) {
+    cudaError_t ce = cudaMalloc(p, bytes);
+    if (ce == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();
+      *p = nullptr;
+      if (free_wide_filter(h)) ce = cudaMalloc(p, bytes);
+    }
+    return ce;
+  };
+  if (!h->pids) e = get(&h->pids, h->n * sizeof(uint32_t));
   if (e == cudaSuccess && !h->ptable) {
-    e = cudaMalloc(&h->ptable, h->ld * h->d * sizeof(float));
+    e = get(&h->ptable, h->ld * h->d * sizeof(float));
     if (e == cudaSuccess) e = cudaMemsetAsync(h->ptable, 0, h->ld * h->d * sizeof(float), s);
   }
-  if (e == cudaSuccess && !h->pstats) e = cudaMalloc(&h->pstats, 3 * P * h->d * sizeof(float));
+  if (e == cudaSuccess && !h->pstats) e = get(&h->pstats, 3 * P * h->d * sizeof(float));
   // the build's scratch: work | radix sort scratch | row-major copy (left out when there is
   // no memory for it) in one allocation
   unsigned char *scratch = nullptr;
@@ -1827,7 +1878,7 @@ int topk_build_partitions_ordered(topk_table_t h, uint32_t part_rows, int order)
     const bool with_rows = ce == cudaSuccess;
     if (!with_rows) {
       (void)cudaGetLastError();
-      ce = cudaMalloc(&scratch, fixed);
+      ce = get(&scratch, fixed);
     }
     if (ce != cudaSuccess) return ce;
     work = reinterpret_cast<uint32_t *>(scratch);
@@ -1841,7 +1892,7 @@ int topk_build_partitions_ordered(topk_table_t h, uint32_t part_rows, int order)
   if (e == cudaSuccess && order == TOPK_ORDER_MORTON) {
     // scratch: keys | histogram | column minima and scales
     const size_t kb = up(h->n * sizeof(uint16_t)), hb = (1u << 16) * sizeof(uint32_t);
-    e = cudaMalloc(&scratch, kb + hb + lo_scale.size() * sizeof(float));
+    e = get(&scratch, kb + hb + lo_scale.size() * sizeof(float));
     float *dls = reinterpret_cast<float *>(scratch + kb + hb);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dls, lo_scale.data(), lo_scale.size() * 4, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
@@ -2221,8 +2272,8 @@ extern "C" int topk_learned_fit(topk_table_t h, uint64_t n_train, uint64_t n_val
     std::vector<float> sc(chunk * kmax);
     for (uint64_t j0 = 0; j0 < N; j0 += chunk) {
       const uint64_t c = std::min(chunk, N - j0);
-      st = run_batch(h, c, &ks[j0], &qqs[j0], &W[j0 * d], d, &A[j0 * d], d, ids.data(), sc.data(), kmax, cnt.data(),
-                     &kth[j0]);
+      st = run_batch_fit(h, c, &ks[j0], &qqs[j0], &W[j0 * d], d, &A[j0 * d], d, ids.data(), sc.data(), kmax,
+                         cnt.data(), &kth[j0]);
       if (st != TOPK_OK) return st;
     }
   }
@@ -2395,7 +2446,7 @@ int topk_set_scan_tuning(topk_table_t h, uint32_t max_ctas_per_sm) {
 
 int topk_set_fault_injection(topk_table_t h, int mode) {
   if (!h) return fail(TOPK_ERR_ARG, "null handle");
-  if (mode < 0 || mode > 1) return fail(TOPK_ERR_ARG, "mode must be 0 or 1");
+  if (mode < 0 || mode > 2) return fail(TOPK_ERR_ARG, "mode must be 0, 1 or 2");
   h->fault_mode = mode;
   return TOPK_OK;
 }
