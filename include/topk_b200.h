@@ -424,7 +424,8 @@ int topk_set_fault_injection(topk_table_t h, int mode);
                             * batches run TOPK_BATCH_FP32.  Hybrid: a
                             * query for which the filter passes too much (tied or dense
                             * scores at its threshold: more than 2k + 2048 candidates in
-                            * a chunk, or lost ones) moves to the exact FP32 scorer for
+                            * a chunk, 7.5k if that is more where chunks quadruple, or
+                            * lost ones) moves to the exact FP32 scorer for
                             * the rest of the batch, inside the same call */
 #define TOPK_BATCH_LEARNED 4 /* TOPK_BATCH_BF16 (or FP32) whose per-query threshold starts
                               * at the learned cut (prediction - margin) * S instead of a

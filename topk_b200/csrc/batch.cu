@@ -264,15 +264,16 @@ __global__ void copy_word_kernel(uint32_t *dst, const uint32_t *src) { *dst = *s
 // Hybrid batches (`sw` non-null: sw[0], sw[1] counts, then two lists of nq
 // queries) move a query from the filter to the exact FP32 scorer for the rest of
 // the batch when the filter passes too much for it (scores tied or dense at its
-// threshold): with more than 2k + 2048 candidates in a chunk the chunk is merged and
-// the query is listed in the first list; when candidates were lost (its region or a
+// threshold): with more than 2k + 2048 candidates in a chunk, and in a quadrupling one
+// (which passes 3k where scores are spread evenly) more than 2.5 times 3k, the chunk is
+// merged and the query is listed in the first list; when candidates were lost (its region or a
 // filter log overflowed) the chunk is discarded and the query is listed in both, the
 // second list naming the queries whose chunk the FP32 scorer answers again.
 __global__ void __launch_bounds__(kBT) batch_reduce_kernel(const float *__restrict__ table, uint64_t ld,
                                                            const BatchQuery *__restrict__ qs,
                                                            BatchState *__restrict__ st, uint2 *__restrict__ best,
                                                            const uint2 *__restrict__ cand, int rescore,
-                                                           uint32_t *__restrict__ sw, uint32_t nq) {
+                                                           uint32_t *__restrict__ sw, uint32_t nq, int quadruple) {
   extern __shared__ __align__(16) unsigned char smem[];
   BatchShared *sh = reinterpret_cast<BatchShared *>(smem);
   uint32_t *hist = reinterpret_cast<uint32_t *>(smem + 128);
@@ -349,7 +350,7 @@ __global__ void __launch_bounds__(kBT) batch_reduce_kernel(const float *__restri
     ns.cnt = kept;
     if (kept == k) ns.thr = max(thr, sh->sel.kept_min + 1u);
     if (nc_raw > q.cand_cap) ns.flags |= kFlagOverflow;
-    if (sw && filtered && nc_raw > 2 * k + 2048) {  // tie-dense under the filter: exact scorer from now on
+    if (sw && filtered && nc_raw > max(2 * k + 2048, quadruple ? 15 * k / 2 : 0u)) {  // tie-dense under the filter: exact scorer from now on
       ns.flags |= kFlagFp32;
       sw[2 + atomicAdd(&sw[0], 1u)] = blockIdx.x;
     }
@@ -461,11 +462,12 @@ size_t batch_reduce_smem(uint32_t kmax, uint32_t capmax) { return kQueryShared +
 
 cudaError_t launch_batch_reduce(const float *table, uint64_t ld, const BatchQuery *qs, uint32_t nq, BatchState *st,
                                 uint2 *best, const uint2 *cand, uint32_t kmax, uint32_t capmax, bool rescore,
-                                uint32_t *sw, cudaStream_t s) {
+                                uint32_t *sw, bool quadruple, cudaStream_t s) {
   const size_t smem = batch_reduce_smem(kmax, capmax);
   cudaError_t e = cudaFuncSetAttribute(batch_reduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  batch_reduce_kernel<<<nq, kBT, smem, s>>>(table, ld, qs, st, best, cand, rescore ? 1 : 0, sw, nq);
+  batch_reduce_kernel<<<nq, kBT, smem, s>>>(table, ld, qs, st, best, cand, rescore ? 1 : 0, sw, nq,
+                                                  quadruple ? 1 : 0);
   return cudaGetLastError();
 }
 

@@ -66,7 +66,7 @@ cudaError_t launch_copy_word(uint32_t *dst, const uint32_t *src, cudaStream_t s)
 size_t batch_reduce_smem(uint32_t kmax, uint32_t capmax);
 cudaError_t launch_batch_reduce(const float *table, uint64_t ld, const BatchQuery *qs, uint32_t nq, BatchState *st,
                                 uint2 *best, const uint2 *cand, uint32_t kmax, uint32_t capmax, bool rescore,
-                                uint32_t *sw, cudaStream_t s);
+                                uint32_t *sw, bool quadruple, cudaStream_t s);
 // BF16 tensor-core filter (bf16_filter.cu).
 uint64_t bf16_table_bytes(uint64_t n, uint32_t d);
 // Also the column extremes: ext[m] = largest |x| bits, ext[d + m] = largest order key,

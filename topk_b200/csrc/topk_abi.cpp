@@ -969,8 +969,10 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   const uint64_t r_start = use_learned ? 0 : boot;
   // Chunks double the rows seen; for a small batch they quadruple them: a chunk costs
   // about 25 us of launches whatever it holds, and passes 3k candidates a query instead of
-  // 2k in two (from about 2^16 results on those cost more than the launches).  Beyond
-  // k = 1024 3k candidates would come close to what moves a query to the FP32 scorer.
+  // 2k in two (from about 2^16 results on those cost more than the launches).  Up to k = 1024
+  // a query's candidate region holds 2.5 times the 3k, so that rows whose scores rise through
+  // the table do not move queries to the FP32 scorer (launch_batch_reduce) more than doubled
+  // chunks do.
   // Boundaries stay multiples of 256 rows (the filter's object tiles).
   const bool quadruple = best_total <= (1u << 16) && kmax <= 1024;
   auto next_chunk = [&](uint64_t r, uint64_t size) { return quadruple ? 3 * r : 2 * size; };
@@ -1023,14 +1025,14 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
     } else {
       CK(launch_batch_score_fp32(h->table, h->ld, h->d, r, e, dq, nqq, dst, dcand, dorder, qmax, false, s));
     }
-    CK(launch_batch_reduce(h->table, h->ld, dq, nqq, dst, dbest, dcand, kmax, capmax, use_bf16, dsw, s));
+    CK(launch_batch_reduce(h->table, h->ld, dq, nqq, dst, dbest, dcand, kmax, capmax, use_bf16, dsw, quadruple, s));
     prev_r = r;
     r = e;
   }
   if (use_bf16) {  // the last chunk again for the queries that discarded it (none: two empty launches)
     CK(launch_batch_score_fp32_list(h->table, h->ld, h->d, prev_r, h->n, dq, dst, dcand, dsw + 2 + nq, dsw + 1,
                                     dredo, dwork, qmax, true, h->num_sms, s));
-    CK(launch_batch_reduce(h->table, h->ld, dq, nqq, dst, dbest, dcand, kmax, capmax, use_bf16, dsw, s));
+    CK(launch_batch_reduce(h->table, h->ld, dq, nqq, dst, dbest, dcand, kmax, capmax, use_bf16, dsw, quadruple, s));
   }
   // results compact (each query's at its best_off), so the download moves sum(k) entries
   CK(launch_batch_finish(dq, nqq, dst, dbest, kmax, dids, dscores, 0, dcount, dthr, s));
