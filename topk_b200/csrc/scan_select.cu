@@ -368,7 +368,12 @@ __device__ __forceinline__ void take_bound(const ScanParams &p, SmemCtl *ctl, bo
 // its threads' best, and keeps the largest such limit of any CTA in g_hid: no unpublished
 // entry that could belong to the result reaches it.  Then it waits for the coordinator's
 // decision; true: the merge tree answers.
-__device__ __forceinline__ bool publish_entries(const ScanParams &p, const uint2 *cand, SmemCtl *ctl, uint32_t *hist) {
+// In partition mode the best rows lie together, so one CTA often holds most of the result
+// and the limit fails; with k <= pub_exact such a CTA selects its best k instead, which
+// hide nothing.  (Its select takes a few us, the tree 20: 758,368 x 4 rows in 93 partitions,
+// k = 81: 65.1 us a query through the tree, 50.4 so.)
+template <bool PART>
+__device__ __forceinline__ bool publish_entries(const ScanParams &p, uint2 *cand, SmemCtl *ctl, uint32_t *hist) {
   const int t = threadIdx.x;
   const int lane = t & 31, warp = t >> 5;
   ScanScratch *sc = p.scratch;
@@ -394,19 +399,25 @@ __device__ __forceinline__ bool publish_entries(const ScanParams &p, const uint2
   }
   v = __reduce_add_sync(0xFFFFFFFFu, v);
   if (lane == 0) atomicAdd(&ctl->sel.valid, v);
-  if (n > kPubMaxEntries) {
+  const bool exact = PART && p.k <= p.pub_exact;
+  if (n > kPubMaxEntries && !exact) {
     if (lane < 4) keys[4 * warp + lane] = 0;
     __syncwarp();
     warp_top(m, 0u, 4u, lane, [&](uint32_t x, uint32_t key, uint32_t) { keys[4 * warp + x] = key; });
   }
   bsync();
   uint64_t limit = g, hid = 0;  // entries below the limit stay unpublished
-  if (ctl->sel.valid > kPubMaxEntries) {
+  const bool many = ctl->sel.valid > kPubMaxEntries;
+  if (exact && many) {
+    bsync();  // every thread has `many` before the select writes its state
+    list = cand + p.cap;  // the select's output area
+    block_reduce<kScanThreads>(cand, n, list, p.k, gkey, hist, &ctl->sel);
+  } else if (many) {
     const uint32_t x = __shfl_sync(0xFFFFFFFFu, warp_sort_desc<uint32_t>(keys[lane], lane), (int)p.pub_m - 1);
     if (x > gkey) limit = hid = (uint64_t)x << 32;  // (no entry below g belongs to the result)
   }
 #pragma unroll 4
-  for (uint32_t j = t; j < n; j += kScanThreads) {
+  for (uint32_t j = t; j < n && !(exact && many); j += kScanThreads) {
     const uint2 e = cand[j];
     if (composite(e.x, e.y) >= limit) {
       const uint32_t at = atomicAdd(&ctl->sel.wcount, 1u);
@@ -415,8 +426,8 @@ __device__ __forceinline__ bool publish_entries(const ScanParams &p, const uint2
   }
   bsync();
   if (warp == 0) {
-    const uint32_t c = min(ctl->sel.wcount, kPubMaxEntries);
-    if (ctl->sel.wcount > kPubMaxEntries) hid = ~0ull;  // (equal keys at the limit)
+    const uint32_t most = exact && many ? p.k : kPubMaxEntries, c = min(ctl->sel.wcount, most);
+    if (ctl->sel.wcount > most) hid = ~0ull;  // (equal keys at the limit)
     uint32_t base = 0;
     if (lane == 0) {
       if (c) base = atomicAdd(&sc->pub_n, c);
@@ -898,7 +909,7 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ, PART>())
   if (t == 0 && ctl->reductions) atomicAdd(&p.scratch->acc_reductions, ctl->reductions);
   if (PART && t == 0) atomicAdd(&p.scratch->acc_tiles, seg);
 
-  if (p.pub && !publish_entries(p, cand0, ctl, hist)) return;
+  if (p.pub && !publish_entries<PART>(p, cand0, ctl, hist)) return;
 
   // ---- merge tree: this CTA's best k first ----
   if (t == 0) {

@@ -95,6 +95,7 @@ struct Ctx {
   uint2 *epub = nullptr;  // and those of each threshold epoch
   uint32_t epub_stride = 0;
   uint32_t max_slots = 0, max_groups = 0;
+  uint32_t max_grid = 0;    // CTAs that `pub` has room for, kPubMaxEntries each
   size_t slot_entries = 0;  // capacity of `slots`
   size_t meta_bytes = 0;    // bytes that must be zero between queries (header + done)
   // Result block of the synchronous queries in mapped pinned memory (h_out on the host,
@@ -233,6 +234,7 @@ int ctx_create(topk_table_t h, Ctx **out) {
   c->slot_entries = (size_t)4 * (size_t)h->num_sms * kMaxK;
   c->meta_bytes = sizeof(ScanScratch) + (size_t)c->max_groups * 4;
   const size_t slots_off = (c->meta_bytes + (size_t)c->max_slots * 4 + 255) / 256 * 256;
+  c->max_grid = max_grid;
   c->epub_stride = kPubMaxKeys * max_grid;
   const size_t pub_off = slots_off + c->slot_entries * sizeof(uint2),
                epub_off = pub_off + (size_t)kPubMaxEntries * max_grid * sizeof(uint2),
@@ -399,6 +401,7 @@ int enqueue_scan(topk_table_t h, Ctx *c, cudaStream_t stream, uint64_t r0, uint6
     p.pub = c->pub;
     p.pub_m = m;
     p.pub_wait = kPubWaitPolls;
+    p.pub_exact = (uint32_t)((uint64_t)kPubMaxEntries * c->max_grid / (uint32_t)pl.grid);
     p.epub = c->epub;
     p.epub_stride = c->epub_stride;
     p.epoch_shift = shift;
