@@ -895,8 +895,10 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ, PART>())
       }
     }
     seg += i;
-    if (stopped || ctl->epoch >= p.epochs) break;
+    // (a CTA that a seed stopped before epoch 0 arrives there all the same: others wait for it)
+    if (ctl->epoch >= p.epochs || (stopped && ctl->epoch != 0u)) break;
     epoch_publish(p, cand0, ctl, hist);
+    if (stopped) break;
     if (PART && p.epoch_hold && ctl->epoch == 1u) {  // (a small copy: few tiles to stop before)
       if (t == 0) take_bound(p, ctl, true);
       bsync();
