@@ -488,7 +488,9 @@ int topk_last_batch_filter_flops(topk_table_t h, double *flops);
 int topk_last_stats(topk_table_t h, uint64_t *candidates, uint64_t *reductions);
 
 /* Bound (in polling iterations) on every device-side wait; 0 restores the default.
- * A wait that runs out makes the call return TOPK_ERR_TIMEOUT. */
+ * A wait that runs out makes the call return TOPK_ERR_TIMEOUT, but for the waits of a
+ * scan's blocks on each other (for a threshold, for the answer): those have limits of
+ * their own below the default, and a scan whose waits run out answers without them. */
 int topk_set_wait_limit(topk_table_t h, uint64_t iterations);
 
 /* Table shape and device stride. */

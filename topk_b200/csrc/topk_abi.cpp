@@ -400,14 +400,14 @@ int enqueue_scan(topk_table_t h, Ctx *c, cudaStream_t stream, uint64_t r0, uint6
   if (const uint32_t m = pub_entries((uint32_t)k, (uint32_t)pl.grid, epochs)) {
     p.pub = c->pub;
     p.pub_m = m;
-    p.pub_wait = kPubWaitPolls;
+    p.pub_wait = (uint32_t)std::min<uint64_t>(kPubWaitPolls, h->wait_limit);
     p.pub_exact = (uint32_t)((uint64_t)kPubMaxEntries * c->max_grid / (uint32_t)pl.grid);
     p.epub = c->epub;
     p.epub_stride = c->epub_stride;
     p.epoch_shift = shift;
     p.epochs = epochs;
     p.epoch_keys = epoch_keys((uint32_t)k, (uint32_t)pl.grid, ps != nullptr);
-    p.epoch_wait = kEpochWaitPolls;
+    p.epoch_wait = (uint32_t)std::min<uint64_t>(kEpochWaitPolls, h->wait_limit);
     p.epoch_hold = ps && epochs && tiles <= 16u * (uint64_t)pl.grid;
   }
   p.scratch = c->scratch;
