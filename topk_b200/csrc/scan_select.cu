@@ -226,7 +226,8 @@ constexpr int scan_min_blocks() {
 }
 
 // ---------------------------------------------------------------- results
-// Put the scratch back to zero for the next scan (one thread, after everything else).
+// Put the scratch back to zero for the next scan (one thread, after everything else; the
+// kernel's end makes it visible, a fence here would wait for the result's way to the host).
 __device__ __forceinline__ void reset_scratch(ScanScratch *s) {
   s->acc_reductions = 0;
   s->acc_tiles = 0;
@@ -239,7 +240,6 @@ __device__ __forceinline__ void reset_scratch(ScanScratch *s) {
   for (uint32_t e = 0; e < kMaxEpochs; ++e) s->epoch_arrived[e] = 0;
   s->g_thr = 0;
   s->g_app = 0;
-  __threadfence();
 }
 
 // The scan's statistics (thread 0 of the CTA that answers).
@@ -1027,8 +1027,12 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ, PART>())
   if (t == 0) {
     // with a coordinator, the later of it and this CTA resets the scratch (no CTA waits for
     // the decision any more: each has published a slot)
-    __threadfence();
-    if (!p.pub || atomicAdd(&p.scratch->finishers, 1u) == 1u) {
+    bool last = true;
+    if (p.pub) {
+      __threadfence();
+      last = atomicAdd(&p.scratch->finishers, 1u) == 1u;
+    }
+    if (last) {
       reset_scratch(p.scratch);
       if (p.pub) p.scratch->gen = ctl->gen0 + 2u;
     }
