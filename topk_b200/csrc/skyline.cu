@@ -206,19 +206,23 @@ int skyline_layers_device(const float *table, uint64_t ld, uint32_t d, uint64_t 
     return TOPK_ERR_UNSUPPORTED;
   }
   cudaStream_t s = nullptr;
-  unsigned char *scratch = nullptr;  // six arrays of n words | values | radix sort scratch
+  uint32_t *kin = nullptr, *kout = nullptr, *oa = nullptr, *ob = nullptr, *cand = nullptr, *depth = nullptr;
+  float *xs = nullptr;
+  void *temp = nullptr;
   size_t tb = 0;
   cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-  if (e == cudaSuccess)
-    e = cub::DeviceRadixSort::SortPairs(nullptr, tb, (const uint32_t *)nullptr, (uint32_t *)nullptr,
-                                        (const uint32_t *)nullptr, (uint32_t *)nullptr, (int)n, 0, 32, s);
-  const size_t wb = (n * sizeof(uint32_t) + 255) / 256 * 256, vb = ((size_t)d * n * sizeof(float) + 255) / 256 * 256;
-  if (e == cudaSuccess) e = cudaMalloc(&scratch, 6 * wb + vb + std::max<size_t>(tb, 16));
-  uint32_t *kin = reinterpret_cast<uint32_t *>(scratch), *kout = reinterpret_cast<uint32_t *>(scratch + wb),
-           *oa = reinterpret_cast<uint32_t *>(scratch + 2 * wb), *ob = reinterpret_cast<uint32_t *>(scratch + 3 * wb),
-           *cand = reinterpret_cast<uint32_t *>(scratch + 4 * wb), *depth = reinterpret_cast<uint32_t *>(scratch + 5 * wb);
-  float *xs = reinterpret_cast<float *>(scratch + 6 * wb);
-  void *temp = scratch + 6 * wb + vb;
+  if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(nullptr, tb, kin, kout, oa, ob, (int)n, 0, 32, s);
+  // (an allocation each: small ones come from pages that the driver keeps mapped.  All in one,
+  // 2.2 MB at 30,011 x 4, mapped its pages in every call: 0.6 ms, and now and then 5-800)
+  std::vector<void *> owned;
+  auto get = [&](auto **q, size_t bytes) {
+    if (e != cudaSuccess) return;
+    e = cudaMalloc(q, bytes);
+    if (e == cudaSuccess) owned.push_back(*q);
+  };
+  for (uint32_t **q : {&kin, &kout, &oa, &ob, &cand, &depth}) get(q, n * sizeof(uint32_t));
+  get(&xs, (size_t)d * n * sizeof(float));
+  get(&temp, std::max<size_t>(tb, 16));
   const int g = grid_n(n, num_sms);
   // order: stable passes from the least significant key (the last value) to the sum
   if (e == cudaSuccess) {
@@ -251,7 +255,7 @@ int skyline_layers_device(const float *table, uint64_t ld, uint32_t d, uint64_t 
   if (e == cudaSuccess) e = cudaMemcpyAsync(dep.data(), depth, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(ord.data(), oa, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFree(scratch);
+  for (void *q : owned) cudaFree(q);
   if (s) cudaStreamDestroy(s);
   if (e != cudaSuccess) {
     *msg = std::string("skyline layers: ") + cudaGetErrorString(e);
