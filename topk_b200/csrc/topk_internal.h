@@ -165,16 +165,17 @@ constexpr uint32_t kPubMaxEntries = 96;  // at the end (the list and 32 words in
 // leaves one out in under 1-3 % of queries (then the merge tree answers).  In a scan with
 // epochs it holds that many only when much of the result is in it, and publishes about as
 // many as it can bound (24 of the 32 best of its threads).  Where lambda is too large for
-// that, grids of at least 16 CTAs publish 28 each, whose k-th bounds what the tree carries
-// (40,000 rows, k = 1000: 63 us a query against 104 without); below, or with too few CTAs
-// for k entries, publishing is in vain (14 us of 57) and the tree answers alone: 0.
+// that, grids of at least 16 CTAs publish 28 each, or all 32 where k needs them, whose k-th
+// bounds what the tree carries (40,000 rows, k = 1000: 63 us a query against 104 without;
+// 102,000 rows, k = 3000 and 3190: 111 and 116 us with 32, 288-373 without); below, or with
+// too few CTAs for k entries, publishing is in vain (14 us of 57) and the tree answers alone: 0.
 inline uint32_t pub_entries(uint32_t k, uint32_t grid, uint32_t epochs) {
   if (grid < kPubMinGrid || (uint64_t)grid * kPubMaxEntries < k) return 0;
   if (epochs) return 24;
   const double l = (double)k / grid;
   const uint32_t r = (uint32_t)__builtin_ceil(l + 3.0 * __builtin_sqrt(l) + 1.6);
   if (r <= 24) return r;
-  return grid >= 16 && 28u * grid >= k ? 28 : 0;
+  return grid < 16 || 32u * grid < k ? 0 : 28u * grid >= k ? 28 : 32;
 }
 // Epochs of a scan over `tiles` tiles, after 1, m, m^2, ... tiles (m = 2^shift): each ends
 // before the scan does, with every CTA still taking part.
