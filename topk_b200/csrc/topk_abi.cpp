@@ -154,7 +154,7 @@ struct topk_table_s {
   DevBuf b_in, b_out, b_best, b_cand;
   // BF16 filter: split copy of the table (rebuilt when the table changed), the
   // per-column max |x| it was built from, the survivor records
-  DevBuf xbf, xbf_absmax, b_log, b_logh, b_feat, b_pred;
+  DevBuf xbf, xbf_absmax, b_log, b_feat, b_pred;
   // compact active query tiles of the filter, slot -> query map and count
   DevBuf b_abf_act, b_amap;
   uint64_t data_version = 1, xbf_version = 0;
@@ -693,7 +693,7 @@ void in_parallel(uint64_t n, size_t bytes, const Fn &fn) {
 
 void free_batch_buffers(topk_table_t h) {
   for (topk_table_s::DevBuf *b : {&h->b_in, &h->b_out, &h->b_best, &h->b_cand, &h->xbf, &h->xbf_absmax, &h->b_log,
-                                  &h->b_logh, &h->b_feat, &h->b_pred, &h->b_abf_act, &h->b_amap}) {
+                                  &h->b_feat, &h->b_pred, &h->b_abf_act, &h->b_amap}) {
     cudaFree(b->p);
     b->p = nullptr;
     b->bytes = 0;
@@ -728,7 +728,7 @@ bool drop_wide_filter(topk_table_t h) {
   if (h->d <= kBf16K || !(h->xbf.p || h->b_log.p)) return false;
   (void)cudaGetLastError();  // the failed allocation's
   cudaStreamSynchronize(h->primary->stream);
-  for (topk_table_s::DevBuf *b : {&h->xbf, &h->b_log, &h->b_logh}) {
+  for (topk_table_s::DevBuf *b : {&h->xbf, &h->b_log}) {
     cudaFree(b->p);
     *b = topk_table_s::DevBuf{};
   }
@@ -757,8 +757,8 @@ int ensure_bf16_table(topk_table_t h, size_t log_bytes, cudaStream_t s) {
   if (h->d > kBf16K && h->xbf.bytes < bytes) {
     size_t avail = 0, total = 0;
     CK(cudaMemGetInfo(&avail, &total));
-    const size_t held = h->xbf.bytes + h->b_log.bytes + h->b_logh.bytes;
-    if (bytes + std::max<size_t>(log_bytes, h->b_log.bytes + h->b_logh.bytes) > (avail + held) / 2)
+    const size_t held = h->xbf.bytes + h->b_log.bytes;
+    if (bytes + std::max<size_t>(log_bytes, h->b_log.bytes) > (avail + held) / 2)
       return TOPK_OK;  // (asked again by the next batch: memory may be free by then)
   }
   int st;
@@ -871,8 +871,7 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   // eighth of the batch's may fall to one CTA before queries move to the FP32 scorer.  (At
   // kBf16LogCap the logs take 660 MB, most of a small batch's first call.)
   const uint32_t rec_cap = (uint32_t)std::min<uint64_t>(kBf16LogCap, (4096 + 3 * best_total / 8) / 16 * 16);
-  auto log_bytes = [&](uint64_t ctas) { return ctas * rec_cap * 8 * sizeof(uint4); };
-  auto logh_bytes = [&](uint64_t ctas) { return ctas * rec_cap * sizeof(uint2); };
+  auto log_bytes = [&](uint64_t ctas) { return ctas * rec_cap * (8 * sizeof(uint4) + sizeof(uint2)); };
   // scorer: the BF16 tensor-core filter where the table and every weight allow it
   bool use_bf16 = false;
   const uint32_t kblk = bf16_kblocks(h->d);
@@ -880,7 +879,7 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   if (!force_fp32 && !small_wide && (h->batch_method == TOPK_BATCH_AUTO || h->batch_method == TOPK_BATCH_BF16 ||
                       h->batch_method == TOPK_BATCH_LEARNED)) {
     const uint64_t ctas = h->d <= kBf16MaxD ? plan_bf16_filter(nqq_all, 0, h->n, h->d, h->num_sms, h->batch_qt).grid : 0;
-    if ((st = ensure_bf16_table(h, log_bytes(ctas) + logh_bytes(ctas), s)) != TOPK_OK) return st;
+    if ((st = ensure_bf16_table(h, log_bytes(ctas), s)) != TOPK_OK) return st;
     use_bf16 = h->xbf_usable && h->xbf_version == h->data_version && nq <= 0xFFFFFFFFull;
     // AUTO: scores too dense around the thresholds for the filter on this table
     if (h->batch_method == TOPK_BATCH_AUTO && h->auto_fp32_version == h->data_version) use_bf16 = false;
@@ -924,7 +923,6 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
     log_ctas = fp.grid;
     if (h->fault_mode == 2) return fail(TOPK_ERR_OOM, "batch buffer: injected");
     if ((st = ensure(h->b_log, log_bytes(log_ctas))) != TOPK_OK) return st;
-    if ((st = ensure(h->b_logh, logh_bytes(log_ctas))) != TOPK_OK) return st;
   } else {
     // the plain FP32 scorer takes the queries ordered by attribute count, then by
     // attribute list: a warp's lanes then run the same number of steps and mostly read
@@ -960,6 +958,8 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
   uint32_t *derr = reinterpret_cast<uint32_t *>(dout + o_err);
   uint2 *dbest = static_cast<uint2 *>(h->b_best.p);
   uint2 *dcand = static_cast<uint2 *>(h->b_cand.p);
+  uint4 *dlog = static_cast<uint4 *>(h->b_log.p);  // records' values, then their headers
+  uint2 *dlogh = reinterpret_cast<uint2 *>(dlog + log_ctas * rec_cap * 8);
   const uint32_t nqq = (uint32_t)nq;
   if (use_learned) {
     if ((st = ensure(h->b_feat, nq * feature_dim(h->d) * sizeof(float))) != TOPK_OK) return st;
@@ -1017,8 +1017,7 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
       CK(launch_batch_active(dq, dst, nqq, h->d, dabf, static_cast<uint8_t *>(h->b_abf_act.p), amap, amap + nq,
                              logslot, s));
       CK(launch_bf16_filter(fp, static_cast<const uint8_t *>(h->xbf.p), static_cast<const uint8_t *>(h->b_abf_act.p),
-                            amap, amap + nq, r, e, dq, dst, dcand, static_cast<uint4 *>(h->b_log.p),
-                            static_cast<uint2 *>(h->b_logh.p), rec_cap, h->wait_limit, derr, s));
+                            amap, amap + nq, r, e, dq, dst, dcand, dlog, dlogh, rec_cap, h->wait_limit, derr, s));
       // this chunk for every moved query; the previous one again for those that discarded it
       CK(launch_batch_score_fp32_list(h->table, h->ld, h->d, r, e, dq, dst, dcand, dsw + 2, dsw, nullptr, dwork, qmax,
                                       true, h->num_sms, s));
@@ -1049,7 +1048,7 @@ int run_batch(topk_table_t h, uint64_t nq, const uint64_t *ks, const uint32_t *q
                                (uint64_t)h->num_sms, log_ctas, h->wait_limit, h->num_parts, h->batch_qt,
                                quadruple, rec_cap};
   const void *key_ptrs[] = {h->table, dq, dabf, dorder, dst, dbest, dcand, dids, dscores, dcount, dthr, dact, derr,
-                            dsw, h->xbf.p, h->b_log.p, h->b_logh.p, h->b_feat.p, h->b_pred.p, h->pstats, h->mlp,
+                            dsw, h->xbf.p, dlog, h->b_feat.p, h->b_pred.p, h->pstats, h->mlp,
                             h->b_abf_act.p, h->b_amap.p};
   for (const void *ptr : key_ptrs) key.push_back((uint64_t)(uintptr_t)ptr);
   {
