@@ -223,10 +223,10 @@ int topk_merge_lists(int device, const void *d_lists, uint32_t nlists, uint64_t 
  * it, held until the process exits): k is limited to 1024 (TOPK_ERR_UNSUPPORTED
  * above), and calls whose work overlaps on the GPU share that array and race, so
  * serialise them.  The first call on each device performs a one-time set-up on
- * that device; make it before capturing work on that device.  The scan behind this
- * entry has no device-side wait that can give up, so a call that returns TOPK_OK
- * has enqueued work that always writes all its outputs; a kernel failure shows as a
- * CUDA error on `stream`.  Errors: the usual status codes, message from
+ * that device; make it before capturing work on that device.  The waits inside
+ * the scan are bounded, and one that runs out only makes it answer another way, so a
+ * call that returns TOPK_OK has enqueued work that always writes all its outputs; a
+ * kernel failure shows as a CUDA error on `stream`.  Errors: the usual status codes, message from
  * topk_last_error(). */
 int topk_query_noalloc(const float *d_table, uint64_t n, uint64_t ld, uint32_t d, uint64_t k, uint32_t qq,
                        const float *weights, const uint8_t *attr, uint64_t *d_ids, float *d_scores,
@@ -318,7 +318,8 @@ int topk_partition_info(topk_table_t h, uint32_t *num_parts, uint32_t *part_rows
  * scan runs again without it.  Results identical to topk_query.
  * stats (may be NULL): [0] partitions scanned, [1] partitions, [2] 1 if the cut
  * was accepted, [3] rounds: one for a scan from a cut, two for a scan that finds
- * its threshold on the way. */
+ * its threshold on the way (a count of how thresholds were found, not of launches: either
+ * is one). */
 int topk_query_pruned(topk_table_t h, uint64_t k, uint32_t qq, const float *weights, const uint8_t *attr, float cut,
                       uint64_t *ids, float *scores, uint64_t *count, float *threshold, uint64_t *stats);
 
@@ -479,7 +480,8 @@ int topk_last_batch_retired(topk_table_t h, uint64_t *retired);
 
 /* The tensor-core work the last topk_query_batch ran under the BF16 filter: for every
  * chunk, its served query tiles (128 queries each) times its object tiles (256 rows),
- * three BF16 MMA passes of 2 * 16 flops per (query, object).  0 for the other methods.
+ * three BF16 MMA passes of 2 * 16 flops per (query, object) and 16 attributes of the
+ * table's width.  0 for the other methods.
  * No reference counterpart (a measurement of this engine). */
 int topk_last_batch_filter_flops(topk_table_t h, double *flops);
 

@@ -69,19 +69,6 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t *bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Polling step with a suspend-time hint in nanoseconds.
-__device__ __forceinline__ bool mbar_try_wait_hint(uint64_t *bar, uint32_t parity, uint32_t ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n"
-      " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(ns)
-      : "memory");
-  return ok != 0;
-}
-
 // Bounded wait: returns false if the phase did not complete within `limit` polls.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, uint64_t limit) {
   for (uint64_t it = 0; it < limit; ++it)
@@ -101,27 +88,6 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
 
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// Named barrier `id` over `n` threads (whole warps); the warp reconverges first.
-__device__ __forceinline__ void named_sync(uint32_t id, uint32_t n) {
-  __syncwarp();
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
-}
-
-// Named barrier with an OR reduction of `pred` over its `n` threads.
-__device__ __forceinline__ bool named_or(uint32_t id, uint32_t n, bool pred) {
-  __syncwarp();
-  uint32_t r;
-  asm volatile(
-      "{\n .reg .pred p, q;\n"
-      " setp.ne.u32 p, %1, 0;\n"
-      " bar.red.or.pred q, %2, %3, p;\n"
-      " selp.u32 %0, 1, 0, q;\n}\n"
-      : "=r"(r)
-      : "r"((uint32_t)pred), "r"(id), "r"(n)
-      : "memory");
-  return r != 0;
 }
 
 __device__ __forceinline__ uint32_t ld_volatile_u32(const uint32_t *p) {

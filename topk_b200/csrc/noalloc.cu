@@ -163,10 +163,10 @@ extern "C" int topk_query_noalloc(const float *d_table, uint64_t n, uint64_t ld,
   if (tree_slots > kNoAllocMaxSlots || tree_groups > kNoAllocMaxGroups || p.nslots[p.levels] != 1 ||
       (uint64_t)tree_slots * kk > kNoAllocSlotEntries)
     return fail(TOPK_ERR_UNSUPPORTED, "merge tree of %d CTAs does not fit the fixed scratch", pl.grid);
-  // No wait hook: with fault_mode 0 the scan has no device-side wait that can give
-  // up (its only bounded wait is the fault-injection barrier of the handle-based
-  // path), so a launch that succeeds always runs to the root and writes ids, scores
-  // and the threshold; a failure shows as a CUDA error on the stream.
+  // With fault_mode 0 no wait that gives up ends the scan: its blocks' waits on each
+  // other (for a threshold, for the answer) are bounded, and one that runs out leads
+  // through the merge tree, so a launch that succeeds always writes ids, scores and the
+  // threshold; a failure shows as a CUDA error on the stream.
   p.wait_limit = 1ull << 26;
   p.fault_mode = 0;
   const uint32_t epochs = scan_epochs(tiles, (uint32_t)pl.grid, kEpochShift);

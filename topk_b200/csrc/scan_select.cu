@@ -214,8 +214,10 @@ __host__ __device__ constexpr uint32_t scan_vote_tiles(int qq, bool part) {
 }
 
 // CTAs per SM the register budget is sized for: one queried column needs little data
-// in flight and gains from more CTAs (6: 42 registers); more columns need their loads
-// in flight without spills (5: 51 registers up to 8 columns, 4: 64 above).
+// in flight and gains from more CTAs (6: 40 registers); more columns need their loads
+// in flight (5: 48 registers up to 8 columns, 4: 64 above; 8 to 32 bytes spill at q = 1, 4
+// and 13 to 16, and 4 to 28 in partition mode.  Without those of 14 to 16 and half of q =
+// 4's, by a loop over the CTA's tiles without segments, no time changed).
 // Partition mode runs at most 4 CTAs per SM, so it has their registers.  Two attributes in
 // id order take 48 registers at 5 CTAs; at 6 the loop spilled (2^28 rows, independent, us
 // at k = 16 / 1024 / 4096: 430 / 534 / 1110 with 6, 400 / 448 / 819 with 5; only k = 1 is

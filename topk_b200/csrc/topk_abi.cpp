@@ -518,7 +518,7 @@ constexpr uint32_t kPrunedCtasPerSm = 4;
 // seed, so every object of the true top-k was scanned); otherwise the scan runs again
 // without it.  stats: partitions scanned (tiles scanned / tiles per partition, over
 // every scan), partitions, seed accepted (1/0), rounds: one for a scan with a seed, two
-// for a scan that finds its threshold on the way.
+// for a scan that finds its threshold on the way (each is one launch of the scan).
 int run_pruned(topk_table_t h, uint64_t k, uint32_t qq, const float *weights, const uint8_t *attr, float cut,
                bool learned, uint64_t *ids, float *scores, uint64_t *count, float *threshold, uint64_t *stats,
                float *cut_out) {
@@ -594,7 +594,7 @@ int run_pruned(topk_table_t h, uint64_t k, uint32_t qq, const float *weights, co
   const uint32_t seed_host = std::isfinite(cut) ? host_f2key(cut) : 0u;
   const bool seeded = learned || seed_host != 0u;
   const uint64_t tiles_per_part = (1ull << h->part_log2) / 1024u;
-  uint64_t tiles = 0, scans = 0, accepted = 0;
+  uint64_t tiles = 0, rounds = 0, accepted = 0;
   float cut_seen = cut;
   // the seeded attempt (if any), then the scan without a seed
   for (int attempt = seeded ? 0 : 1; attempt < 2; attempt++) {
@@ -603,7 +603,7 @@ int run_pruned(topk_table_t h, uint64_t k, uint32_t qq, const float *weights, co
                       kPrunedCtasPerSm};
     st = enqueue_scan(h, c, s, 0, h->n, k, qq, weights, attr, d_ids, d_scores, &dho->threshold, &dho->count,
                       dho->stats, &ps);
-    scans += attempt == 0 ? 1u : 2u;
+    rounds += attempt == 0 ? 1u : 2u;  // (see above: not launches)
     if (st != TOPK_OK) return st;
     CK(cudaStreamSynchronize(s));
     if (hh->count > kk) {
@@ -632,7 +632,7 @@ int run_pruned(topk_table_t h, uint64_t k, uint32_t qq, const float *weights, co
     stats[0] = (tiles + tiles_per_part - 1) / tiles_per_part;
     stats[1] = P;
     stats[2] = accepted;
-    stats[3] = scans;
+    stats[3] = rounds;
   }
   g_last_cands = hh->stats[0];
   g_last_reductions = hh->stats[1];

@@ -57,14 +57,8 @@ static_assert(sizeof(ScanScratch) == 512, "four 128-byte lines");
 
 // TOPK_BOUNDS_CHECK codes
 enum : uint32_t {
-  kDiagCopyShape = 1,   // bulk copy size/alignment/destination out of range
-  kDiagCopySource = 2,  // bulk copy source outside the table
-  kDiagPhase = 3,       // stage barrier re-armed before its previous phase completed
-  kDiagAppend = 4,      // candidate append past capacity
-  kDiagCompact = 5,     // compaction write past capacity
-  kDiagWait = 6,        // a stage wait gave up
-  kDiagOutput = 7,      // output index out of range
-  kDiagMerge = 8,       // merge load past capacity
+  kDiagAppend = 4,  // candidate append past capacity
+  kDiagMerge = 8,   // merge load past capacity
 };
 
 struct ScanParams {

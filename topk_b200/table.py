@@ -325,7 +325,8 @@ class Table:
     def query_pruned(self, k, weights, attr, cut=float("nan")):
         """Exact top-k scanning only partitions that can reach the threshold;
         returns (ids, scores, threshold, stats) with stats = (partitions scanned,
-        partitions, cut accepted, scans)."""
+        partitions, cut accepted, rounds: 1 for a scan from a cut, 2 for one that finds
+        its threshold on the way, whatever the launches)."""
         w, a = _weights(weights, self.d), _attr(attr)
         cap = max(1, min(int(k), self.n))
         b = _call_block()
