@@ -215,9 +215,9 @@ __host__ __device__ constexpr uint32_t scan_vote_tiles(int qq, bool part) {
 
 // CTAs per SM the register budget is sized for: one queried column needs little data
 // in flight and gains from more CTAs (6: 40 registers); more columns need their loads
-// in flight (5: 48 registers up to 8 columns, 4: 64 above; 8 to 32 bytes spill at q = 1, 4
-// and 13 to 16, and 4 to 28 in partition mode.  Without those of 14 to 16 and half of q =
-// 4's, by a loop over the CTA's tiles without segments, no time changed).
+// in flight (5: 48 registers up to 8 columns; 4: 64 above and with a run-time count, which
+// took 4 % longer with 48.  8 to 32 bytes spill at q = 1, 4 and 14 to 16, 4 in partition
+// mode).
 // Partition mode runs at most 4 CTAs per SM, so it has their registers.  Two attributes in
 // id order take 48 registers at 5 CTAs; at 6 the loop spilled (2^28 rows, independent, us
 // at k = 16 / 1024 / 4096: 430 / 534 / 1110 with 6, 400 / 448 / 819 with 5; only k = 1 is
@@ -765,12 +765,17 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ, PART>())
         load_next(xn);
       }
     }
-    uint32_t i = 0;  // tiles of the segment so far
+    // i: the tile of the segment (base + i the CTA's), above eight columns the CTA's: one
+    // value less beside the loads (2^28 rows, q = 14: 2183 us with base, 2150 without; at
+    // q = 1, where the loop is unrolled, 426 with, 458 without)
+    constexpr bool kAbs = !PART && QQ > 8;
+    const uint32_t base = kAbs ? 0u : seg, end = kAbs ? seg + seg_len : seg_len;
+    uint32_t i = kAbs ? seg : 0u;
     // two tiles per vote: after every odd one, and in the second segment, which starts at
     // tile 1, after every even one -- no more than two tiles ever meet an unvoted buffer
     const uint32_t vote_at = seg == 1u ? 0u : 1u;
 #pragma unroll(kUnroll)
-    for (; i < seg_len; ++i) {
+    for (; i < end; ++i) {
       // every thread reads the same thresholds in tile i (see SmemCtl::thr_g); in id
       // order they are read after the scores, so they hold no register across the loads
       uint32_t thr = 0;
@@ -782,7 +787,7 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ, PART>())
           break;
         }
       }
-      const uint64_t tile0 = (prefetch && !PART) ? next_row : tile_row(seg + i, part_cur);
+      const uint64_t tile0 = (prefetch && !PART) ? next_row : tile_row(base + i, part_cur);
       const uint64_t row0 = tile0 + (uint64_t)t * kVec;
       const bool interior = (prefetch && !PART) ? next_tix - p.int_lo < p.int_n
                                                 : tile0 >= p.row_begin && tile0 + kTile <= p.row_end;  // uniform
@@ -792,8 +797,8 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ, PART>())
 #pragma unroll
         for (int m = 0; m < kPQ; ++m) x[m] = xn[m];
         if constexpr (PART) {
-          if (seg + i + 1 < ctl->my_tiles) load_rows(tile_row(seg + i + 1, part_nx), xn);
-        } else if (i + 1 < seg_len) {
+          if (base + i + 1 < ctl->my_tiles) load_rows(tile_row(base + i + 1, part_nx), xn);
+        } else if (i + 1 < end) {
           next_row += p.grid_rows;
           next_tix += ncta;
           load_next(xn);
@@ -805,7 +810,7 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ, PART>())
       if constexpr (PART) {
         part_cur = part_nx;
         key_cur = key_nx;
-        if (seg + i + 2 < ctl->my_tiles) part_of(seg + i + 2, part_nx, key_nx);
+        if (base + i + 2 < ctl->my_tiles) part_of(base + i + 2, part_nx, key_nx);
       }
 
       if constexpr (!PART) thr = max(ctl->thr_local, ctl->thr_g[i & 1u]);
@@ -848,23 +853,25 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ, PART>())
           }
       }
       // thread 0 hands the CTA its copy of the global threshold (see SmemCtl::thr_g): it
-      // loads the global word every 4 tiles and applies it 3 tiles later, so the L2 round
-      // trip is never waited on (every 2 and 1 later in partition mode, where it ends the
-      // scan).  The new value goes to the slot the next tile reads, and on the tile after
-      // into the other slot too; between updates both slots agree.
-      constexpr uint32_t kPoll = PART ? 1u : 3u;
+      // loads the global word every 4 tiles (8 where a tile is more than eight columns) and
+      // applies it on the last of them, so the L2 round trip is never waited on (every 2 and
+      // on the next in partition mode, where it ends the scan).  The new value goes to the
+      // slot the next tile reads, and on the tile after into the other slot too; between
+      // updates both slots agree.  One word: the larger of two would be waited for here, and
+      // every warp with it at the vote (2^28 rows, q = 14, k = 16: 2183 us so, 2135 now).
+      constexpr uint32_t kPoll = PART ? 1u : (QQ == 0 || QQ > 8) ? 7u : 3u;
       if (t == 0) {
         if ((i & kPoll) == kPoll) ctl->thr_g[(i + 1u) & 1u] = max(ctl->thr_g[i & 1u], g_pending);
         if ((i & kPoll) == 0u) {
           ctl->thr_g[(i + 1u) & 1u] = ctl->thr_g[i & 1u];
-          g_pending = max(ld_volatile_u32(&p.scratch->g_thr), ld_volatile_u32(&p.scratch->g_app));
+          g_pending = ld_volatile_u32(&p.scratch->g_app);
         }
       }
       // (uniform: every thread takes the same votes; the scan's end needs no room)
       if (kVoteTiles > 1 && (i & 1u) != vote_at) continue;
       const bool full = __syncthreads_or(after > cap - kVoteTiles * kTile);
       after = 0;
-      if (full && seg + i + 1 < ctl->my_tiles) {
+      if (full && base + i + 1 < ctl->my_tiles) {
         if (t == 0) {
           // the first fill may come before any bound: epoch 0's is on its way, and dropping
           // what lies below it costs one pass over the buffer instead of a select
@@ -891,12 +898,13 @@ __global__ void __launch_bounds__(kScanThreads, scan_min_blocks<QQ, PART>())
             // reordered copy) may win the tie: the threshold stays inclusive.
             ctl->thr_local = ctl->sel.kept_min + (p.row_ids ? 0u : 1u);
             atomicMax(&p.scratch->g_thr, ctl->sel.kept_min);
+            atomicMax(&p.scratch->g_app, ctl->sel.kept_min);
           }
         }
         bsync();
       }
     }
-    seg += i;
+    seg = base + i;
     // (a CTA that a seed stopped before epoch 0 arrives there all the same: others wait for it)
     if (ctl->epoch >= p.epochs || (stopped && ctl->epoch != 0u)) break;
     epoch_publish(p, cand0, ctl, hist);

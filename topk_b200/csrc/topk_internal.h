@@ -25,7 +25,8 @@ constexpr uint32_t kEpochShift = 2, kPartEpochShift = 1;
 // `gen`): the kernel puts every counter back before it ends.
 struct ScanScratch {
   uint32_t g_thr;           // running global threshold key (objects below it cannot win)
-  uint32_t g_app;           // the same for rows still to be scanned (ScanParams::epub)
+  uint32_t g_app;           // the same for rows still to be scanned (ScanParams::epub): at least
+                            // g_thr while the scan runs
   unsigned long long g_keep;  // the last epoch's bound: objects below this (key, ~id) cannot win
   uint32_t error;           // nonzero after a device wait gave up (bit 0: stage wait)
   uint32_t acc_reductions;  // CTA block-selects during this scan
