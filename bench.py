@@ -114,7 +114,7 @@ def measured_peaks():
 # DRAM bytes (read + write) per query of the fused scan at n = 2^28, by q: dram__bytes of
 # the launch of one query on a 2^26-row table (every object is read once, so traffic grows
 # with the rows scanned) scaled x4, the mean over k in {16, 64, 256, 1024}.
-TRAFFIC_PER_LAUNCH = {2: 2.1617e9, 4: 4.3117e9, 8: 8.5913e9, 16: 1.7193e10}
+TRAFFIC_PER_LAUNCH = {2: 2.1525e9, 4: 4.3125e9, 8: 8.5921e9, 16: 1.7193e10}
 TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the launch of each query on a "
                   "2^26-row table, mean over the four k, scaled x4 to "
                   "2^28 rows")

@@ -40,11 +40,11 @@
 //     last CTA of each group of G slots (per-group arrival counter) merges them to k
 //     entries in shared memory and moves up; the root sorts (bitonic) and writes the
 //     result.  Counters are put back to zero for the next query.
-//   Measured (us a query on a stream, independent rows, before -> after): 2^20 rows q = 4
-//   k = 16 35.4 -> 23.6, k = 256 64 -> 28; 2^24 rows q = 2 k = 16 70 -> 57, k = 1024 205 ->
-//   79 (two launches before: a threshold pass over every 64th tile first), q = 8 k = 1024
-//   201 -> 116; 2^27 rows q = 4 k = 1024 397 -> 351; q = 2 k = 16 230 -> 230.  Correlated
-//   rows, many equal: 2^24 rows q = 2 k = 1024 272 -> 91.
+//   Measured (us a query on a stream, independent rows, without epochs and coordinator ->
+//   with): 2^20 rows q = 4 k = 16 39.0 -> 25.0, k = 256 67 -> 31; 2^24 rows q = 2 k = 16 73
+//   -> 52, k = 1024 272 -> 83, q = 8 k = 1024 199 -> 127; 2^27 rows q = 4 k = 1024 482 -> 359
+//   (two launches before: a threshold pass over every 64th tile first), q = 2 k = 16 238 ->
+//   218.  Correlated rows, many equal: 2^24 rows q = 2 k = 1024 203 -> 71.
 //   A launch's fixed cost is what is left: the first tiles' latency (~5 us), the first
 //   epoch (~8 us, hidden from q = 8 on), the end (~10 us).
 #include <cstdint>
@@ -220,8 +220,7 @@ __host__ __device__ constexpr uint32_t scan_vote_tiles(int qq, bool part) {
 // mode).
 // Partition mode runs at most 4 CTAs per SM, so it has their registers.  Two attributes in
 // id order take 48 registers at 5 CTAs; at 6 the loop spilled (2^28 rows, independent, us
-// at k = 16 / 1024 / 4096: 430 / 534 / 1110 with 6, 400 / 448 / 819 with 5; only k = 1 is
-// slower than with 6 CTAs and no epochs, 395 against 383).
+// at k = 16 / 1024 / 4096: 430 / 534 / 1110 with 6, 400 / 448 / 819 with 5).
 template <int QQ, bool PART>
 constexpr int scan_min_blocks() {
   return PART ? 4 : QQ == 1 ? 6 : (QQ >= 2 && QQ <= 8) ? 5 : 4;

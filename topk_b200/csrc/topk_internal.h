@@ -88,7 +88,7 @@ struct ScanParams {
   // May be null (then the merge tree answers).  Else block 0 of the launch coordinates and
   // scans nothing (launch_scan adds it to the plan's grid).  At its end each scanning CTA
   // publishes its best entries here (at most kPubMaxEntries per CTA, about pub_m when it
-  // holds more); the coordinator answers the query from the published entries when none
+  // holds more, in partition mode its best k where pub_exact allows); the coordinator answers the query from the published entries when none
   // of the unpublished ones can belong to the result, else raises the global threshold
   // to the k-th largest published key and starts the merge tree.  The CTAs wait for that
   // decision, at most pub_wait polls; one whose wait runs out takes the decision for
