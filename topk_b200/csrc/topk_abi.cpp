@@ -137,6 +137,7 @@ struct topk_table_s {
   std::mutex mu;
   std::condition_variable cv;
   std::vector<Ctx *> ctxs;
+  uint32_t in_flight = 0;  // contexts taken
   Ctx *primary = nullptr;
   // batched path: one batch at a time per handle, device buffers grow and are kept
   std::mutex batch_mu;
@@ -273,20 +274,25 @@ void ctx_free(Ctx *c) {
   delete c;
 }
 
-// Take a free context (creating one up to kMaxContexts, else wait for one).
-int ctx_acquire(topk_table_t h, Ctx **out) {
+// Take a free context (creating one up to kMaxContexts, else wait for one); *in_flight: how
+// many are taken by now.
+int ctx_acquire(topk_table_t h, Ctx **out, uint32_t *in_flight) {
   std::unique_lock<std::mutex> lk(h->mu);
+  auto take = [&](Ctx *c) {
+    c->busy = true;
+    *in_flight = ++h->in_flight;
+    *out = c;
+    return TOPK_OK;
+  };
   for (;;) {
     for (Ctx *c : h->ctxs)
-      if (!c->busy) { c->busy = true; *out = c; return TOPK_OK; }
+      if (!c->busy) return take(c);
     if (h->ctxs.size() < kMaxContexts) {
       Ctx *c = nullptr;
       int st = ctx_create(h, &c);
       if (st != TOPK_OK) return st;
-      c->busy = true;
       h->ctxs.push_back(c);
-      *out = c;
-      return TOPK_OK;
+      return take(c);
     }
     h->cv.wait(lk);
   }
@@ -296,6 +302,7 @@ void ctx_release(topk_table_t h, Ctx *c) {
   {
     std::lock_guard<std::mutex> lk(h->mu);
     c->busy = false;
+    --h->in_flight;
   }
   h->cv.notify_one();
 }
@@ -303,8 +310,9 @@ void ctx_release(topk_table_t h, Ctx *c) {
 struct CtxLease {
   topk_table_t h;
   Ctx *c = nullptr;
+  uint32_t in_flight = 0;
   int status;
-  explicit CtxLease(topk_table_t hh) : h(hh) { status = ctx_acquire(h, &c); }
+  explicit CtxLease(topk_table_t hh) : h(hh) { status = ctx_acquire(h, &c, &in_flight); }
   ~CtxLease() { if (c) ctx_release(h, c); }
 };
 
@@ -321,6 +329,23 @@ int check_query(topk_table_t h, uint64_t k, uint32_t qq, const float *weights, c
   return TOPK_OK;
 }
 
+// Whether a scan of a call among `in_flight` on the handle is answered by the merge tree
+// alone, without epochs and coordinator: with them its CTAs keep their places until the last
+// one has published and the answer is decided, places that the other calls' CTAs wait for.
+// The tree's cost grows with k, a CTA's wait matters less the longer it scans.  us a query,
+// q = 4, with the coordinator / by the tree alone, from 2, 3, 4 and 8 threads: 2^20 rows (1.4
+// tiles a CTA) k = 16 23.7 23.9 23.8 24.2 / 28.4 20.3 16.7 16.7, k = 100 24.7 24.8 24.9 25.1 /
+// 44.7 31.4 25.0 17.7, k = 400 33 / 66 46 35 22; 2^24 rows (22 tiles) k = 16 59.7 60.2 60.2
+// 59.1 / 58.8 53.2 53.0 52.1, k = 100 67 / 84 65 63 61, k = 400 79 / 101 78 74 72; 2^27 rows
+// k = 16 320-327 / 302, k = 200 346 / 335 331 328 325.  Grids that do not fill the GPU leave
+// the others their places (2^17 rows, k = 16 to 400: 12-20 with, 13-41 without).
+bool crowded_scan(uint32_t in_flight, uint64_t k, uint64_t tiles_per_cta) {
+  if (k >= 512 || tiles_per_cta < 1) return false;
+  if (in_flight >= 5) return true;
+  if (in_flight >= 3) return k <= 64 || tiles_per_cta >= 8;
+  return in_flight == 2 && (tiles_per_cta >= 64 || (k <= 32 && tiles_per_cta >= 8));
+}
+
 // A scan over a list of partitions of the partitioned copy, with a threshold seed.
 struct PartScan {
   const uint32_t *d_list;  // partition numbers (device), by bound descending
@@ -335,7 +360,7 @@ struct PartScan {
 // writing into the given outputs.
 int enqueue_scan(topk_table_t h, Ctx *c, cudaStream_t stream, uint64_t r0, uint64_t r1, uint64_t k, uint32_t qq,
                  const float *weights, const uint8_t *attr, uint64_t *d_ids, float *d_scores, float *d_thr,
-                 uint32_t *d_count, uint32_t *d_stats = nullptr, const PartScan *ps = nullptr) {
+                 uint32_t *d_count, uint32_t *d_stats = nullptr, const PartScan *ps = nullptr, uint32_t in_flight = 1) {
   const uint64_t rows = ps ? ((uint64_t)ps->count << h->part_log2) : r1 - r0;
   ScanPlan pl = plan_scan(qq, (uint32_t)k, rows, h->num_sms, h->smem_optin, h->max_ctas_per_sm, ps != nullptr);
   if (pl.stages < 1) return fail(TOPK_ERR_UNSUPPORTED, "qq=%u, k=%llu do not fit in shared memory", qq, (unsigned long long)k);
@@ -397,7 +422,8 @@ int enqueue_scan(topk_table_t h, Ctx *c, cudaStream_t stream, uint64_t r0, uint6
   p.fault_mode = (uint32_t)h->fault_mode;
   const uint32_t shift = ps ? kPartEpochShift : kEpochShift;
   const uint32_t epochs = scan_epochs(tiles, (uint32_t)pl.grid, shift);
-  if (const uint32_t m = pub_entries((uint32_t)k, (uint32_t)pl.grid, epochs)) {
+  const bool alone = ps || !epochs || !crowded_scan(in_flight, k, tiles / (uint64_t)pl.grid);
+  if (const uint32_t m = alone ? pub_entries((uint32_t)k, (uint32_t)pl.grid, epochs) : 0u) {
     p.pub = c->pub;
     p.pub_m = m;
     p.pub_wait = (uint32_t)std::min<uint64_t>(kPubWaitPolls, h->wait_limit);
@@ -455,7 +481,7 @@ int run_query_sync(topk_table_t h, uint64_t r0, uint64_t r1, uint64_t k, uint32_
   // a sentinel count tells a completed scan from one that left early
   hh->count = 0xFFFFFFFFu;
   st = enqueue_scan(h, c, c->stream, r0, r1, k, qq, weights, attr, d_ids, d_scores, &dh->threshold, &dh->count,
-                    dh->stats);
+                    dh->stats, nullptr, lease.in_flight);
   if (st != TOPK_OK) return st;
   CK(cudaStreamSynchronize(c->stream));
   if (hh->count != (uint32_t)kk) {
