@@ -1,4 +1,4 @@
-"""Concurrent queries on one handle, whose scans are answered by the coordinator or, when
+"""Concurrent queries, plain and pruned, on one handle, whose scans are answered by the coordinator or, when
 several are in flight, by the merge tree alone: every thread's results against the oracle,
 bit for bit, over table sizes and k on both sides of that choice."""
 import threading
@@ -29,12 +29,14 @@ def test_threads_on_one_handle(n, threads):
     errors = []
     with T.Table(n, d) as t:
         t.upload(x)
+        t.build_partitions(1024, T.ORDER_KD)
 
         def work(i):
             try:
                 for j in range(3 * len(queries)):
                     k, w, a, want = queries[(i + j) % len(queries)]
                     H.assert_same_result(t.query(k, w, a), want)
+                    H.assert_same_result(t.query_pruned(k, w, a)[:3], want)
             except Exception as e:  # reported below
                 errors.append(e)
 

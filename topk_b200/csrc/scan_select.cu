@@ -378,6 +378,10 @@ __device__ __forceinline__ bool publish_entries(const ScanParams &p, uint2 *cand
   const int t = threadIdx.x;
   const int lane = t & 31, warp = t >> 5;
   ScanScratch *sc = p.scratch;
+  if (p.tree_end) {
+    if (t == 0) atomicAdd(&sc->pub_arrived, 1u);
+    return true;
+  }
   const uint32_t n = ctl->count;
   uint32_t *keys = hist;                               // 4 per warp, before the list
   uint2 *list = reinterpret_cast<uint2 *>(hist + 64);  // kPubMaxEntries entries
@@ -529,6 +533,7 @@ __device__ __noinline__ void coordinate(const ScanParams &p, SmemCtl *ctl, uint2
       ++epoch;
       continue;
     }
+    if (p.tree_end) break;  // (nothing is decided: every CTA is on its way through the tree)
     const uint32_t np = ld_volatile_u32(&sc->pub_n);
     const uint64_t hid = ld_volatile_u64(&sc->g_hid);
     unsigned long long *comp = reinterpret_cast<unsigned long long *>(buf);

@@ -96,6 +96,7 @@ struct ScanParams {
   uint2 *pub;
   uint32_t pub_m;
   uint32_t pub_wait;
+  uint32_t tree_end;   // nothing is published at the end: the tree answers and no CTA waits
   uint32_t pub_exact;  // partition mode: most entries that every CTA can publish at once
   // Threshold epochs (needs pub): after its tile 1, then 2^epoch_shift times as many,
   // and so on (`epochs` of them) each CTA publishes the best entries it holds (epoch_keys
